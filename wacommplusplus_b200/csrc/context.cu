@@ -517,7 +517,7 @@ PackedArgs packed_args(wacomm_b200_context *ctx) {
 
 // Histogram, offsets and scan scratch of the cell sort of `count` records.
 int reserve_sort(wacomm_b200_context *ctx, size_t count) {
-    size_t bins = (size_t)ctx->eta * ctx->xi + 1;
+    size_t bins = sort_bins(ctx->eta, ctx->xi, ctx->sRho, count).count();
     if (ctx->binsCap < bins + 2 || !ctx->dHist || !ctx->dOffsets) {
         cudaFree(ctx->dHist);
         cudaFree(ctx->dOffsets);
@@ -530,19 +530,20 @@ int reserve_sort(wacomm_b200_context *ctx, size_t count) {
     return reserve_scan(ctx, std::max(bins, count));
 }
 
-// Orders `count` records by cell into order[]. A sort of the whole resident set walks the records
-// in the previous full sort's order (when that is still a permutation of the slots) and keeps its
-// own result for the next one; a sort of a slab walks its slots in order.
-// Cell sort of `count` records: walks them in seqIn (a permutation of [0, count), or null: slot
-// order) and copies the resulting order to seqOut (or not, if null).
-int sort_work(wacomm_b200_context *ctx, const ParticleSoA &S, size_t count, uint32_t *keys,
-              uint32_t *order, const uint32_t *seqIn, uint32_t *seqOut, int &launches) {
-    size_t bins = (size_t)ctx->eta * ctx->xi + 1;
+// Cell sort of `count` records for interval P: walks them in seqIn (a permutation of [0, count),
+// or null: slot order) and copies the resulting order to seqOut (or not, if null). A sort of the
+// whole resident set walks the previous full sort's order (when that is still a permutation of
+// the slots); a sort of a slab walks its own previous one or its slots.
+int sort_work(wacomm_b200_context *ctx, const IntervalParams &P, const ParticleSoA &S, size_t count,
+              uint32_t *keys, uint32_t *order, const uint32_t *seqIn, uint32_t *seqOut,
+              int &launches) {
+    SortBins bins = sort_bins(ctx->eta, ctx->xi, ctx->sRho, count);
+    if (P.direction > 0) bins.idleTime = P.start + P.length;  // backward tracking releases all
     int rc;
     if ((rc = reserve_sort(ctx, count))) return rc;
-    CUDA_TRY(ctx, sort_by_cell(S.j, S.i, (int)count, ctx->eta, ctx->xi, seqIn, keys, ctx->dHist,
-                               ctx->dOffsets, ctx->dScanTemp, order, ctx->stream));
-    size_t blocks = (bins + 8191) / 8192;
+    CUDA_TRY(ctx, sort_by_cell(S, (int)count, bins, seqIn, keys, ctx->dHist, ctx->dOffsets,
+                               ctx->dScanTemp, order, ctx->stream));
+    size_t blocks = (bins.count() + 8191) / 8192;
     launches += 3 + (blocks > 1 ? 2 : 0);
     if (seqOut)
         CUDA_TRY(ctx, cudaMemcpyAsync(seqOut, order, count * sizeof(uint32_t),
@@ -587,7 +588,7 @@ int run_interval(wacomm_b200_context *ctx, const IntervalParams &base, size_t of
             L.order = seqIn;
             ctx->sortedAgo++;
         } else if (ctx->opt.sort_by_cell) {
-            int rc = sort_work(ctx, S, count, keys, order, c == 0 ? seqIn : seqOut, seqOut,
+            int rc = sort_work(ctx, P, S, count, keys, order, c == 0 ? seqIn : seqOut, seqOut,
                                launches);
             if (rc) return rc;
             L.order = order;
@@ -777,7 +778,7 @@ int run_surrogate(wacomm_b200_context *ctx, const IntervalParams &P, int &launch
             st.walkOrder = seqIn;
         } else {
             ctx->seqBounds.clear();
-            if ((rc = sort_work(ctx, ctx->S.s, count, ctx->dKeys, ctx->dOrder, seqIn, ctx->dSeq,
+            if ((rc = sort_work(ctx, P, ctx->S.s, count, ctx->dKeys, ctx->dOrder, seqIn, ctx->dSeq,
                                 launches)))
                 return rc;
             ctx->seqBounds = whole;

@@ -75,12 +75,23 @@ size_t scan_temp_words(size_t n);
 cudaError_t exclusive_scan(const uint32_t *in, uint32_t *out, size_t n, uint32_t *total,
                            uint32_t *temp, cudaStream_t stream);
 
-// Counting sort of particles by forcing cell: order[] receives particle slots grouped by cell.
+// Bins of the counting sort by forcing cell: one per cell and, with levels > 1, per vertical level
+// of a cell, then one last bin for the records that take no step in the interval (off the grid, or
+// released at or after idleTime).
+struct SortBins {
+    int eta, xi, levels;
+    double idleTime;
+    size_t count() const { return (size_t)eta * xi * levels + 1; }
+};
+// The bins `count` records are sorted into on a grid of sRho levels.
+SortBins sort_bins(int eta, int xi, int sRho, size_t count);
+
+// Counting sort of particles by forcing cell: order[] receives particle slots grouped by bin.
 // The records are visited in the sequence seq[n] (a permutation of the slots; null: slot order).
-// keys/hist/offsets/temp are scratch: keys[n], hist[eta*xi+1], offsets[eta*xi+2].
-cudaError_t sort_by_cell(const double *j, const double *i, int n, int eta, int xi,
-                         const uint32_t *seq, uint32_t *keys, uint32_t *hist, uint32_t *offsets,
-                         uint32_t *temp, uint32_t *order, cudaStream_t stream);
+// keys/hist/offsets/temp are scratch: keys[n], hist[bins.count()], offsets[bins.count() + 1].
+cudaError_t sort_by_cell(const ParticleSoA &S, int n, const SortBins &bins, const uint32_t *seq,
+                         uint32_t *keys, uint32_t *hist, uint32_t *offsets, uint32_t *temp,
+                         uint32_t *order, cudaStream_t stream);
 
 cudaError_t aos_to_soa(const wacomm_b200_particle *aos, int n, const ParticleSoA &S,
                        cudaStream_t stream);
