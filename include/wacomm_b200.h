@@ -120,8 +120,8 @@ typedef struct wacomm_b200_source {
 #define WACOMM_B200_RNG_PHILOX 1       /* Philox4x32-10 keyed on (particle id, interval, step time) */
 
 #define WACOMM_B200_LAUNCH_SHAPE_AUTO (-1) /* launch_shape by compiled form: 3 for the deterministic
-                                              form without drift (96 registers, no spills), 2 for
-                                              the others; the default */
+                                              form without drift (96 registers), 1 for the form
+                                              with every branch, 2 for the others; the default */
 
 typedef struct wacomm_b200_options {
     int semantics;            /* WACOMM_B200_SEMANTICS_* */
@@ -138,7 +138,7 @@ typedef struct wacomm_b200_options {
     int launch_shape;         /* FP32 step: 0 = 256 threads, registers unbounded; 1 = 128 threads,
                                  3 blocks/SM; 2 = 256 threads, 2 blocks/SM; 3 = 128 threads,
                                  5 blocks/SM (fewer registers, more resident warps);
-                                 WACOMM_B200_LAUNCH_SHAPE_AUTO (default): 3 or 2 by form */
+                                 WACOMM_B200_LAUNCH_SHAPE_AUTO (default): 3, 2 or 1 by form */
     int surrogate;            /* 1: forward intervals by the learned surrogate
                                  (wacomm_b200_set_surrogate), with the plain stochastic operator
                                  per substep when the random walk is on; the rest by the FP32 step */

@@ -51,16 +51,17 @@ inline int fast_variant(const wacomm_b200_config &cfg, int direction) {
     return diffuse ? VAR_DIFFUSE : VAR_LEAN;
 }
 
-// Shapes 1, 2 and 3 carry every form; shape 0 the full one. A negative shape picks by form: the
-// lean form fits shape 3's 96 registers without spills and runs 4 % faster there (20 resident
-// warps per SM instead of 16); the others spill at shape 3 and run at shape 2.
+// Shapes 1, 2 and 3 carry every form; shape 0 the full one. A negative shape picks by form, the
+// register needs deciding (move kernel, shapes 1 / 2 / 3): lean, 4.2 M records 11.37 / 10.23 /
+// 9.94 ms; random walk (Philox), 1.05 M 4.09 / 3.64 / 3.77 ms; leeway drift, 400,000 2.51 / 2.27 /
+// 2.94 ms; full 5.33 / 5.97 / 7.25 ms (568 bytes of spills at shape 2, 188 at shape 1).
 template <int SEM, int STORE>
 cudaError_t move_f32_unit(int shape, const wacomm_b200_config &cfg, const IntervalParams &P,
                           const PackedArgs &A, const ParticleSoA &S, const MoveLaunch &L,
                           cudaStream_t stream) {
     FastView<STORE> F = fast_view<STORE>(A);
     const int variant = fast_variant(cfg, P.direction);
-    if (shape < 0) shape = variant == VAR_LEAN ? 3 : 2;
+    if (shape < 0) shape = variant == VAR_LEAN ? 3 : variant == VAR_FULL ? 1 : 2;
     switch (shape) {
         case 0: return launch_move_fast<SEM, STORE, 0, VAR_FULL>(cfg, P, F, S, L, stream);
         case 3:

@@ -181,19 +181,6 @@ struct QuadPair {  // a field at 4 corners for the two bracketing records
 
 __device__ __forceinline__ Quad quad_of(float4 v) { return Quad{v.x, v.y, v.z, v.w}; }
 
-template <int STORE>
-__device__ __forceinline__ void load_quad(const CellQuad<STORE> *p, QuadPair &a, QuadPair &b);
-
-template <>
-__device__ __forceinline__ void load_quad<STORE_F32>(const CellQuad<STORE_F32> *p, QuadPair &a,
-                                                     QuadPair &b) {
-    const float4 *q = reinterpret_cast<const float4 *>(p);
-    a.t0 = quad_of(__ldg(q));
-    a.t1 = quad_of(__ldg(q + 1));
-    b.t0 = quad_of(__ldg(q + 2));
-    b.t1 = quad_of(__ldg(q + 3));
-}
-
 __device__ __forceinline__ Quad quad_h(uint32_t x, uint32_t y) {
     float2 lo = __half22float2(*reinterpret_cast<__half2 *>(&x));
     float2 hi = __half22float2(*reinterpret_cast<__half2 *>(&y));
@@ -205,29 +192,12 @@ __device__ __forceinline__ Quad quad_bf(uint32_t x, uint32_t y) {
     return Quad{lo.x, lo.y, hi.x, hi.y};
 }
 
-template <>
-__device__ __forceinline__ void load_quad<STORE_F16>(const CellQuad<STORE_F16> *p, QuadPair &a,
-                                                     QuadPair &b) {
-    const uint4 *q = reinterpret_cast<const uint4 *>(p);
-    uint4 x = __ldg(q), y = __ldg(q + 1);
-    a.t0 = quad_h(x.x, x.y);
-    a.t1 = quad_h(x.z, x.w);
-    b.t0 = quad_h(y.x, y.y);
-    b.t1 = quad_h(y.z, y.w);
-}
+// The velocity stencil of one cell and level: u, v and the two w levels at the bracketing records.
+struct Stencil {
+    QuadPair u, v, wUp, wLo;
+};
 
-template <>
-__device__ __forceinline__ void load_quad<STORE_BF16>(const CellQuad<STORE_BF16> *p, QuadPair &a,
-                                                      QuadPair &b) {
-    const uint4 *q = reinterpret_cast<const uint4 *>(p);
-    uint4 x = __ldg(q), y = __ldg(q + 1);
-    a.t0 = quad_bf(x.x, x.y);
-    a.t1 = quad_bf(x.z, x.w);
-    b.t0 = quad_bf(y.x, y.y);
-    b.t1 = quad_bf(y.z, y.w);
-}
-
-// The first field of a CellQuad only (w of a B record, without akt).
+// The first field of a CellQuad only (u of an A record, w of a B record).
 template <int STORE>
 __device__ __forceinline__ void load_first(const CellQuad<STORE> *p, QuadPair &a);
 
@@ -252,7 +222,7 @@ __device__ __forceinline__ void load_first<STORE_BF16>(const CellQuad<STORE_BF16
     a.t1 = quad_bf(x.z, x.w);
 }
 
-// The second field of a CellQuad only (akt of a B record, without w).
+// The second field of a CellQuad only (v of an A record, akt of a B record).
 template <int STORE>
 __device__ __forceinline__ void load_second(const CellQuad<STORE> *p, QuadPair &b);
 
@@ -287,28 +257,25 @@ struct CellView {
     const CellQuad<STORE> *columns;   // [cell][sW][2] (A, B)
     const CellSurface *surface;       // [cell]
 
-    // Velocity stencil of level kI (valid memory level) in cell (j, i): u, v at rho level kI;
-    // w, akt at W levels kI (up) and kI-1 (lo).
-    __device__ __forceinline__ void stencil(int kI, int j, int i, QuadPair &u, QuadPair &v,
-                                            QuadPair &wUp, QuadPair &aUp, QuadPair &wLo,
-                                            QuadPair &aLo) const {
-        size_t L = (size_t)(kI + sW - 1);
-        const CellQuad<STORE> *col = columns + (((size_t)j * xi + i) * sW + L) * 2;
-        load_quad<STORE>(col - 1, wLo, aLo);  // B(L-1)
-        load_quad<STORE>(col, u, v);          // A(L)
-        load_quad<STORE>(col + 1, wUp, aUp);  // B(L)
+    // Columns are numbered cell * sW + L (L = kI + sW - 1, kI a valid memory level, cell =
+    // j xi + i); 32 bits number more columns than the device's memory holds.
+
+    // Velocity stencil of a column: u, v at rho level kI; w at W levels kI (up) and kI-1 (lo).
+    __device__ __forceinline__ void stencil(uint32_t column, Stencil &s) const {
+        const CellQuad<STORE> *col = columns + 2 * (size_t)column;
+        load_first<STORE>(col - 1, s.wLo);  // B(L-1)
+        load_first<STORE>(col, s.u);        // A(L)
+        load_second<STORE>(col, s.v);
+        load_first<STORE>(col + 1, s.wUp);  // B(L)
     }
-    // The same without the diffusivity (deterministic steps).
-    __device__ __forceinline__ void stencil_w(int kI, int j, int i, QuadPair &u, QuadPair &v,
-                                              QuadPair &wUp, QuadPair &wLo) const {
-        size_t L = (size_t)(kI + sW - 1);
-        const CellQuad<STORE> *col = columns + (((size_t)j * xi + i) * sW + L) * 2;
-        load_first<STORE>(col - 1, wLo);  // B(L-1)
-        load_quad<STORE>(col, u, v);      // A(L)
-        load_first<STORE>(col + 1, wUp);  // B(L)
+    // Diffusivity at W levels kI (up) and kI-1 (lo) of a column.
+    __device__ __forceinline__ void akt(uint32_t column, QuadPair &up, QuadPair &lo) const {
+        const CellQuad<STORE> *col = columns + 2 * (size_t)column;
+        load_second<STORE>(col - 1, lo);
+        load_second<STORE>(col + 1, up);
     }
-    __device__ __forceinline__ CellSurface surf(int j, int i) const {
-        const float4 *q = reinterpret_cast<const float4 *>(surface + ((size_t)j * xi + i));
+    __device__ __forceinline__ CellSurface surf(uint32_t cell) const {
+        const float4 *q = reinterpret_cast<const float4 *>(surface + cell);
         return CellSurface{__ldg(q), __ldg(q + 1)};
     }
 };
