@@ -44,3 +44,21 @@ def test_records_do_not_depend_on_the_sort(cuda_device, n, arithmetic, direction
             counts.append(engine.concentration())
     assert got[0].tobytes() == got[1].tobytes()
     assert np.array_equal(counts[0], counts[1])
+
+
+# around one, two and all lanes per warp (592 warps), and in and out of the partly filled launches
+@pytest.mark.parametrize("n", [1, 592, 593, 1185, 18944, 18945])
+@pytest.mark.parametrize("arithmetic", ["fp32", "reference"])
+def test_records_do_not_depend_on_how_a_launch_is_spread(cuda_device, n, arithmetic):
+    win = syn.config1_window(n_frames=2, eta=16, xi=17, s_rho=6)
+    few, many = mixed_records(n, win, 5), mixed_records(40000, win, 6)
+    many["id"] += 50000
+    got = []
+    for p in (few, np.concatenate([few, many])):  # the larger launch fills its warps
+        with Engine(0, arithmetic=arithmetic, sort_by_cell=0) as engine:
+            engine.load_window(win)
+            engine.set_config(default_config(random=True))
+            engine.set_particles(p)
+            engine.move_interval(0)
+            got.append(engine.get_particles()[:n])
+    assert got[0].tobytes() == got[1].tobytes()

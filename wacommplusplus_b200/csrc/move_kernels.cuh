@@ -28,7 +28,34 @@ struct MoveLaunch {
     // FP32 step: work items per thread; the grid is that many times smaller and each block
     // strides over it (results do not depend on it).
     int perThread = 1;
+    // Work items per warp (1 to 32): a small launch leaves the other lanes of its warps idle and
+    // spreads over the SMs instead (spread_launch; results do not depend on it).
+    int lanes = 32;
 };
+
+// The work item of this thread in a block that starts at item `base`; `count` (none) on the lanes
+// left idle.
+__device__ __forceinline__ unsigned launch_item(const MoveLaunch &L, unsigned base, unsigned count) {
+    if (L.lanes >= 32) return base + threadIdx.x;
+    const unsigned lane = threadIdx.x & 31;
+    return lane < (unsigned)L.lanes ? base + (threadIdx.x >> 5) * L.lanes + lane : count;
+}
+
+// Lanes per warp and threads per block (at most maxThreads) of a launch over `count` items: one warp
+// per scheduler of the chip before a warp is filled, as blocks of one size on every SM. Such a launch
+// is bound by the latency of its substep chain; fewer lanes per warp meet fewer cell changes and
+// lines per load. 1,021 records (random walk) per host interval 0.473 -> 0.428 ms, 16,384 in
+// reference arithmetic 0.640 -> 0.564 ms; two warps per scheduler: 0.459 and 0.628 ms. From 18,945
+// items on the warps are full.
+inline void spread_launch(int count, int maxThreads, int &lanes, int &threads) {
+    constexpr int SMS = 148, WARPS = 4 * SMS;
+    lanes = (count + WARPS - 1) / WARPS;
+    if (lanes > 32) lanes = 32;
+    if (lanes < 1) lanes = 1;
+    const int warps = (count + lanes - 1) / lanes;
+    threads = 32 * ((warps + SMS - 1) / SMS);
+    if (threads > maxThreads) threads = maxThreads;
+}
 
 // Work items of a launch: count, or the device-side length of its list.
 __device__ __forceinline__ int launch_count(const MoveLaunch &L) {
@@ -69,10 +96,10 @@ __global__ void __launch_bounds__(256) move_soa_kernel(const wacomm_b200_config 
                                                        const IntervalParams P,
                                                        const PackedView<STORE> V, ParticleSoA S,
                                                        const MoveLaunch L) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = launch_item(L, blockIdx.x * (blockDim.x >> 5) * L.lanes, L.count);
     long long cell = -1;
     int steps = 0;
-    if (t < L.count) {
+    if (t < (unsigned)L.count) {
         uint32_t slot = L.order ? L.order[t] : (uint32_t)t;
         ParticleState p;
         p.id = S.id[slot];
@@ -129,12 +156,13 @@ __global__ void __launch_bounds__(LaunchShape<SHAPE>::threads, LaunchShape<SHAPE
                                                         const MoveLaunch L) {
     const int count = launch_count(L);
     // block-uniform stride loop (blocks past a device-side list take no turn)
-    for (long long base = (long long)blockIdx.x * blockDim.x; base < count;
-         base += (long long)gridDim.x * blockDim.x) {
-        const int t = (int)base + threadIdx.x;
+    const int items = (int)(blockDim.x >> 5) * L.lanes;
+    for (long long base = (long long)blockIdx.x * items; base < count;
+         base += (long long)gridDim.x * items) {
+        const unsigned t = launch_item(L, (unsigned)base, (unsigned)count);
         long long cell = -1;
         int steps = 0;
-        if (t < count) {
+        if (t < (unsigned)count) {
             uint32_t slot = L.order ? L.order[t] : (uint32_t)t;
             ParticleState p;
             p.id = S.id[slot];
@@ -168,10 +196,12 @@ cudaError_t launch_move_fast(const wacomm_b200_config &cfg, const IntervalParams
                              const FastView<STORE> &F, const ParticleSoA &S, const MoveLaunch &L,
                              cudaStream_t stream) {
     if (L.count <= 0) return cudaSuccess;
-    constexpr int threads = LaunchShape<SHAPE>::threads;
-    const int per = L.perThread > 1 ? L.perThread : 1;
-    int blocks = (L.count + threads * per - 1) / (threads * per);
-    move_fast_kernel<SEM, STORE, SHAPE, VARIANT><<<blocks, threads, 0, stream>>>(cfg, P, F, S, L);
+    MoveLaunch M = L;
+    int threads;
+    spread_launch(L.count, LaunchShape<SHAPE>::threads, M.lanes, threads);
+    const long long items = (long long)(threads / 32) * M.lanes * (L.perThread > 1 ? L.perThread : 1);
+    const int blocks = (int)((L.count + items - 1) / items);
+    move_fast_kernel<SEM, STORE, SHAPE, VARIANT><<<blocks, threads, 0, stream>>>(cfg, P, F, S, M);
     return cudaGetLastError();
 }
 
@@ -181,8 +211,12 @@ cudaError_t launch_move_soa(const wacomm_b200_config &cfg, const IntervalParams 
                             const PackedView<STORE> &V, const ParticleSoA &S, const MoveLaunch &L,
                             int blockSize, cudaStream_t stream) {
     if (L.count <= 0) return cudaSuccess;
-    int blocks = (L.count + blockSize - 1) / blockSize;
-    move_soa_kernel<SEM, ARITH, STORE><<<blocks, blockSize, 0, stream>>>(cfg, P, V, S, L);
+    MoveLaunch M = L;
+    int threads;
+    spread_launch(L.count, blockSize, M.lanes, threads);
+    const int items = threads / 32 * M.lanes;
+    const int blocks = (L.count + items - 1) / items;
+    move_soa_kernel<SEM, ARITH, STORE><<<blocks, threads, 0, stream>>>(cfg, P, V, S, M);
     return cudaGetLastError();
 }
 
