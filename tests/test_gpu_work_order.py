@@ -62,3 +62,24 @@ def test_records_do_not_depend_on_how_a_launch_is_spread(cuda_device, n, arithme
             engine.move_interval(0)
             got.append(engine.get_particles()[:n])
     assert got[0].tobytes() == got[1].tobytes()
+
+
+# 39,999 and 40,000 records have their normals drawn ahead of the step, 40,001 do not; with 601
+# substeps the draws of 27,869 records fit their buffer and those of 27,893 do not
+@pytest.mark.parametrize("n,dti", [(1, 30.0), (777, 0.1), (39999, 60.0), (40001, 60.0),
+                                   (27869, 6.0), (27893, 6.0), (3001, 7.3)])
+@pytest.mark.parametrize("chunk", [0, 7])
+def test_normals_drawn_ahead_are_the_steps_own(cuda_device, n, dti, chunk):
+    win = syn.config1_window(n_frames=2, eta=16, xi=17, s_rho=6)
+    if dti < 1:
+        win.times[1] = win.times[0] + 60.0  # 0.1 does not sum to whole substeps
+    p = mixed_records(40001, win, 9)
+    got = []
+    for count in (n, 40001):
+        with Engine(0, sort_by_cell=0, substeps_per_launch=chunk) as engine:
+            engine.load_window(win)
+            engine.set_config(default_config(random=True, dti=dti))
+            engine.set_particles(p[:count])
+            engine.move_interval(0)
+            got.append(engine.get_particles()[:n])
+    assert got[0].tobytes() == got[1].tobytes()

@@ -24,6 +24,7 @@ constexpr int VAR_DIFFUSE = 1;  // random walk; no drifting objects, no jibing
 constexpr int VAR_DRIFT = 2;    // leeway drift without wind-error fields, calibration regions or
                                 // coefficient ensemble, with or without the random walk; no jibing
 constexpr int VAR_FULL = 3;     // every branch
+constexpr int VAR_DRAWN = 4;    // VAR_DIFFUSE with the reference keys' normals drawn ahead
 
 constexpr int CLOSURE_CONSTRAINT = 1;  // Config.hpp:201-203
 constexpr int CLOSURE_KILL = 2;

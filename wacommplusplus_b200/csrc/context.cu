@@ -100,6 +100,8 @@ struct wacomm_b200_context {
     uint32_t *dHist2 = nullptr, *dOffsets2 = nullptr, *dScanTemp2 = nullptr;
     size_t binsCap2 = 0, scanTempCap2 = 0;
     cudaEvent_t evLaneStart = nullptr, evLaneDone = nullptr;
+    float4 *dDraws = nullptr;  // normals drawn ahead of a small interval (draw_normals)
+    size_t drawsCap = 0;
     uint32_t *dCount = nullptr;  // scratch word (compaction result)
 
     wacomm_b200_particle *dAos = nullptr;
@@ -575,6 +577,19 @@ int run_interval(wacomm_b200_context *ctx, const IntervalParams &base, size_t of
     L.concTimes = ctx->concTimes;
     L.steps = ctx->dSteps;
     L.err = ctx->dErr;
+    // whole populations only: the slabs of two compute lanes would share the buffer
+    const unsigned steps =
+        count == ctx->n ? draw_steps(ctx->opt, ctx->cfg, base.length, count) : 0;
+    if (steps) {
+        int rc = grow(ctx, ctx->dDraws, ctx->drawsCap, steps * count);
+        if (rc) return rc;
+        CUDA_TRY(ctx, draw_normals(S.id, (int)count, ctx->cfg.randomSeed, base.intervalKey, steps,
+                                   ctx->dDraws, ctx->stream));
+        launches++;
+        L.draws = ctx->dDraws;
+        L.drawSteps = steps;
+        L.drawStride = (unsigned)count;
+    }
     double chunk = ctx->opt.substeps_per_launch > 0 ? ctx->opt.substeps_per_launch * ctx->cfg.dti : 0;
     int nChunks = 1;
     if (chunk > 0 && base.length > 0) nChunks = (int)std::ceil(base.length / chunk);
@@ -940,6 +955,7 @@ int wacomm_b200_context_destroy(wacomm_b200_context *ctx) {
     cudaFree(ctx->dHist2);
     cudaFree(ctx->dOffsets2);
     cudaFree(ctx->dScanTemp2);
+    cudaFree(ctx->dDraws);
     cudaFree(ctx->dCount);
     cudaFree(ctx->dAos);
     cudaFree(ctx->dConc);
@@ -2136,7 +2152,8 @@ std::vector<uint64_t> layout_of(const wacomm_b200_context *ctx) {
     for (const void *p : {(const void *)ctx->dKeys, (const void *)ctx->dOrder,
                           (const void *)ctx->dSeq,
                           (const void *)ctx->dHist, (const void *)ctx->dOffsets,
-                          (const void *)ctx->dScanTemp, (const void *)ctx->dNodes,
+                          (const void *)ctx->dScanTemp, (const void *)ctx->dDraws,
+                          (const void *)ctx->dNodes,
                           (const void *)ctx->dCells, (const void *)ctx->dCellSurface,
                           (const void *)ctx->dSurf, (const void *)ctx->dEnv,
                           (const void *)ctx->dConc, (const void *)ctx->dMetric,
@@ -2210,6 +2227,9 @@ int wacomm_b200_graph_capture(wacomm_b200_context *ctx, int first_time_index, in
         const FrameDevice a = frame_of(ctx, P.t0), b = frame_of(ctx, P.t1);
         bool env = a.windU || a.windV || a.stokesU || b.windU || b.windV || b.stokesU;
         if ((rc = reserve_pair_buffers(ctx, env, cells))) return rc;
+        if (!ctx->opt.surrogate)
+            if (const size_t steps = draw_steps(ctx->opt, ctx->cfg, P.length, ctx->n))
+                if ((rc = grow(ctx, ctx->dDraws, ctx->drawsCap, steps * ctx->n))) return rc;
     }
     if ((rc = ensure_metric(ctx))) return rc;
     if (ctx->n) {

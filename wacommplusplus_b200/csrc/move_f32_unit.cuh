@@ -61,6 +61,9 @@ cudaError_t move_f32_unit(int shape, const wacomm_b200_config &cfg, const Interv
                           cudaStream_t stream) {
     FastView<STORE> F = fast_view<STORE>(A);
     const int variant = fast_variant(cfg, P.direction);
+    // small launches, bound by latency: one block size serves every shape
+    if (variant == VAR_DIFFUSE && L.draws)
+        return launch_move_fast<SEM, STORE, 1, VAR_DRAWN>(cfg, P, F, S, L, stream);
     if (shape < 0) shape = variant == VAR_LEAN ? 3 : variant == VAR_FULL ? 1 : 2;
     switch (shape) {
         case 0: return launch_move_fast<SEM, STORE, 0, VAR_FULL>(cfg, P, F, S, L, stream);

@@ -31,6 +31,10 @@ struct MoveLaunch {
     // Work items per warp (1 to 32): a small launch leaves the other lanes of its warps idle and
     // spreads over the SMs instead (spread_launch; results do not depend on it).
     int lanes = 32;
+    // FP32 step with the reference's random keys: the three normals of every substep of every slot,
+    // drawn ahead ([drawSteps][drawStride], draw_normals; VAR_DRAWN), or null: drawn in the step.
+    const float4 *draws = nullptr;
+    unsigned drawSteps = 0, drawStride = 0;
 };
 
 // The work item of this thread in a block that starts at item `base`; `count` (none) on the lanes
@@ -175,7 +179,9 @@ __global__ void __launch_bounds__(LaunchShape<SHAPE>::threads, LaunchShape<SHAPE
             p.type = S.type[slot];
             p.side = S.side[slot];
             double elapsed = P.firstChunk ? P.elapsed0 : S.elapsed[slot];
-            steps = move_particle_fast<SEM, STORE, VARIANT>(cfg, P, F, p, elapsed, L.err);
+            steps = move_particle_fast<SEM, STORE, VARIANT>(
+                cfg, P, F, Draws{L.draws + slot, L.drawSteps, L.drawStride}, p,
+                elapsed, L.err);
             S.k[slot] = p.k;
             S.j[slot] = p.j;
             S.i[slot] = p.i;

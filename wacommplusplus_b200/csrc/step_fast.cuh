@@ -247,6 +247,12 @@ __device__ __forceinline__ float signf_of(float a, float b) {
     return fabsf(a) * (float)((b > 0.f) - (b < 0.f));
 }
 
+// The normals of a record drawn ahead (VAR_DRAWN): those of substep s at at[s * stride].
+struct Draws {
+    const float4 *at;
+    unsigned steps, stride;
+};
+
 // VARIANT (VAR_*): the branches the run parameters can reach are compiled in, the rest out --
 // fewer registers and a smaller instruction footprint for the common runs.
 //
@@ -261,8 +267,8 @@ __device__ __forceinline__ float signf_of(float a, float b) {
 // by instruction issue.
 template <int SEM, int STORE, int VARIANT>
 __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalParams &P,
-                                  const FastView<STORE> &F, ParticleState &p, double &elapsed,
-                                  int *err) {
+                                  const FastView<STORE> &F, const Draws draws, ParticleState &p,
+                                  double &elapsed, int *err) {
     const PackedView<STORE> &V = F.V;
     const CellView<STORE> &C = F.C;
     const int eta = V.g.eta, xi = V.g.xi, sW = V.g.sW;
@@ -272,8 +278,8 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
     const float dirf = (float)direction, dtiF = (float)cfg.dti;
     const float sv = (float)cfg.sv, shore = (float)cfg.shoreLimit;
     const bool midpoint = cfg.integrator == INTEGRATOR_MIDPOINT;
-    constexpr bool canDiffuse = VARIANT != VAR_LEAN, canDrift = VARIANT >= VAR_DRIFT;
-    constexpr bool full = VARIANT == VAR_FULL;
+    constexpr bool canDiffuse = VARIANT != VAR_LEAN, full = VARIANT == VAR_FULL;
+    constexpr bool canDrift = VARIANT == VAR_DRIFT || full, drawn = VARIANT == VAR_DRAWN;
     const bool diffuse = canDiffuse && cfg.random && (direction > 0 || cfg.backwardDiffusion);
     const bool drift = canDrift && cfg.driftModel == 1 && p.type != 0;
     const bool jibe = full && cfg.leewayJibeProbabilityHourly > 0 && p.type != 0;
@@ -365,6 +371,18 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
             break;
         }
         steps++;
+        // the substep index keys the reference draws and the jibe draw; Philox streams are keyed
+        // on the step's elapsed time instead (unique per step, no division)
+        uint64_t stepKey = 0;
+        const bool philox = P.rng == WACOMM_B200_RNG_PHILOX;
+        float4 normals;
+        if (drawn) {
+            const unsigned substep = (unsigned)floor(elapsed / cfg.dti);
+            const unsigned last = draws.steps - 1;
+            normals = __ldg(draws.at + (size_t)(substep < last ? substep : last) * draws.stride);
+        } else if ((diffuse && !philox) || jibe) {
+            stepKey = fold(prefix, (uint64_t)floor(elapsed / cfg.dti));
+        }
         const float alpha = (float)((elapsed + 0.5 * stepDt) * invLength);
         const float hc = here.height(alpha);
         if (hc <= shore && cfg.horizontalClosure == CLOSURE_KILL) {
@@ -391,18 +409,17 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
             uu += du;
             vv += dv;
         }
-        // the substep index keys the reference draws and the jibe draw; Philox streams are keyed
-        // on the step's elapsed time instead (unique per step, no division)
-        uint64_t stepKey = 0;
-        const bool philox = P.rng == WACOMM_B200_RNG_PHILOX;
-        if ((diffuse && !philox) || jibe) stepKey = fold(prefix, (uint64_t)floor(elapsed / cfg.dti));
         float rx = 0.f, ry = 0.f, rz = 0.f;
         if (diffuse) {
             const float aa = akt_at_cell(C, startColumn, alpha, kF, jF, iF);
             float sigmaDepth = (float)(cfg.sigma * (1 - p.k * P.invKLower));
             float scale = sqrtf(dt / dtiF);
             float n0, n1, n2;
-            if (philox) {
+            if (drawn) {
+                n0 = normals.x;
+                n1 = normals.y;
+                n2 = normals.z;
+            } else if (philox) {
                 philox_normals3(philoxKey, P.intervalKey, (uint64_t)__double_as_longlong(elapsed),
                                 n0, n1, n2);
             } else {

@@ -468,6 +468,57 @@ cudaError_t sort_by_cell(const ParticleSoA &S, int n, const SortBins &bins, cons
     return cudaGetLastError();
 }
 
+// ------------------------------------------------------------------ random draws ahead of the step
+
+// The draws of the reference keys depend on the record, the interval and the substep alone, not on
+// the path: a small launch, whose time is the latency of its substep chain, has them drawn here by
+// one thread per (substep, record) instead of one after the other inside the chain. Bound by FP64
+// issue (log, square root and cosine of three normals): 20,011 records x 121 substeps in about
+// 0.05 ms; the move kernel they feed takes 0.26 ms instead of 0.48 ms (1,021 records: 0.18 instead of
+// 0.40 ms).
+__global__ void __launch_bounds__(256) draw_normals_kernel(const uint64_t *id, unsigned count,
+                                                          uint64_t seed, long long interval,
+                                                          unsigned steps, float4 *out) {
+    const size_t total = (size_t)steps * count;
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
+         e += (size_t)gridDim.x * blockDim.x) {
+        const unsigned s = (unsigned)(e / count), slot = (unsigned)(e - (size_t)s * count);
+        const uint64_t key = key_prefix(seed, id[slot], interval, s);
+        out[e] = make_float4((float)prefix_normal(key, 0), (float)prefix_normal(key, 1),
+                             (float)prefix_normal(key, 2), 0.f);
+    }
+}
+
+// Up to here the move with the draws ahead is the faster one (whole interval of 120 substeps, with /
+// without): 1,021 records 0.26 / 0.43 ms, 20,011 0.40 / 0.51 ms, 30,000 0.45 / 0.52 ms, 45,000 0.54 /
+// 0.56 ms, 59,000 0.59 / 0.56 ms: beyond, the chip is busy with substeps and the draws cost the same
+// either way. The draws stay in L2 (77 MB at the limit).
+constexpr size_t DRAW_AHEAD_RECORDS = 40000;
+constexpr double DRAW_AHEAD_BYTES = 256.0 * (1 << 20);
+
+unsigned draw_steps(const wacomm_b200_options &opt, const wacomm_b200_config &cfg, double length,
+                    size_t count) {
+    const bool diffuse = cfg.random && (cfg.trackingDirection > 0 || cfg.backwardDiffusion);
+    const bool plain = cfg.driftModel != 1 && !(cfg.leewayJibeProbabilityHourly > 0);
+    if (!diffuse || !plain || opt.rng != WACOMM_B200_RNG_REFERENCE || opt.arithmetic != WACOMM_B200_ARITH_FP32)
+        return 0;
+    // floor(elapsed / dti) of a substep that starts before the end; the quotient may round up to the
+    // next whole number there
+    const double steps = ceil(length / cfg.dti) + 1;
+    if (!(steps >= 2 && steps <= 1e6) || count > DRAW_AHEAD_RECORDS ||
+        steps * count * sizeof(float4) > DRAW_AHEAD_BYTES)
+        return 0;
+    return (unsigned)steps;
+}
+
+cudaError_t draw_normals(const uint64_t *id, int count, uint64_t seed, long long interval,
+                         unsigned steps, float4 *out, cudaStream_t stream) {
+    if (count <= 0 || !steps) return cudaSuccess;
+    draw_normals_kernel<<<grid_for((size_t)steps * count, 256), 256, 0, stream>>>(
+        id, (unsigned)count, seed, interval, steps, out);
+    return cudaGetLastError();
+}
+
 // ------------------------------------------------------------------ record layout
 
 __global__ void aos_to_soa_kernel(const wacomm_b200_particle *aos, int n, ParticleSoA S) {
