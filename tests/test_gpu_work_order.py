@@ -3,6 +3,7 @@ that take no step last) changes no result: every record moves on its own."""
 import numpy as np
 import pytest
 
+from oracle import bindings as ob
 from wacommplusplus_b200 import synthetic as syn
 from wacommplusplus_b200.engine import Engine
 from wacommplusplus_b200.types import default_config
@@ -83,3 +84,45 @@ def test_normals_drawn_ahead_are_the_steps_own(cuda_device, n, dti, chunk):
             engine.move_interval(0)
             got.append(engine.get_particles()[:n])
     assert got[0].tobytes() == got[1].tobytes()
+
+
+# the reference arithmetic keeps its velocity stencil up to 37,888 records
+@pytest.mark.parametrize("drift", [0, 1])
+def test_reference_arithmetic_with_and_without_the_kept_stencil(cuda_device, drift):
+    win = syn.RealisticForcing(eta=40, xi=44, s_rho=6, n_frames=2, seed=4, dlon=0.002, dlat=0.002,
+                               land_fraction=0.1, water_border=2).window()
+    win.windU10, win.windV10 = syn.vector_series((40, 44), 2, 8.0, 3, 8.0)
+    p = mixed_records(37889, win, 12)
+    p["driftObjectType"], p["driftSide"] = np.arange(len(p)) % 23, 1
+    cfg = default_config(random=True, driftModel=drift, hasWind=bool(drift))
+    got = []
+    for n in (37888, 37889):
+        with Engine(0, arithmetic="reference") as engine:
+            engine.load_window(win)
+            engine.set_config(cfg)
+            engine.set_particles(p[:n])
+            engine.move_interval(0)
+            got.append(engine.get_particles()[:37888])
+    assert got[0].tobytes() == got[1].tobytes()
+
+
+def test_reference_arithmetic_on_subnormal_and_fill_values(cuda_device):
+    """Time blends round to float precision on the subnormal grid too: a vertical velocity of a few
+    subnormal steps decides at the surface closure, and the fill value stays finite."""
+    win = syn.config1_window(n_frames=2, eta=16, xi=17, s_rho=6)
+    rng = np.random.default_rng(5)
+    win.w[:] = (rng.integers(-3, 4, win.w.shape) * 1.401298464324817e-45).astype(np.float32)
+    win.u[:, :, 12:, :] = 1e37
+    p = mixed_records(3000, win, 14)
+    p["k"][::2] = 0.0
+    cfg = default_config(random=False, upperClosure=2)
+    want = ob.oracle_move(cfg, p.copy(), win, 0, ob.SEMANTICS_HOST, threads=1)
+    with Engine(0, arithmetic="reference") as engine:
+        engine.load_window(win)
+        engine.set_config(cfg)
+        engine.set_particles(p)
+        engine.move_interval(0)
+        got = engine.get_particles()
+    assert np.array_equal(got["health"] > 0, want["health"] > 0)
+    for name in ("k", "j", "i"):
+        assert np.array_equal(got[name], want[name], equal_nan=True), name

@@ -12,8 +12,6 @@ namespace wb {
 
 constexpr int SEM_HOST = WACOMM_B200_SEMANTICS_HOST;
 constexpr int SEM_DEVICE = WACOMM_B200_SEMANTICS_DEVICE;
-constexpr int ARITH_REF = WACOMM_B200_ARITH_REFERENCE;
-constexpr int ARITH_F32 = WACOMM_B200_ARITH_FP32;
 constexpr int STORE_F32 = WACOMM_B200_STORAGE_FP32;
 constexpr int STORE_F16 = WACOMM_B200_STORAGE_FP16;
 constexpr int STORE_BF16 = WACOMM_B200_STORAGE_BF16;

@@ -56,7 +56,7 @@ struct wacomm_b200_context {
     bool hasGrid = false;
     double *dMask = nullptr, *dLon = nullptr, *dLat = nullptr, *dH = nullptr, *dDepth = nullptr;
     bool hasMask = false;
-    double2 *dMetric = nullptr;
+    CellMetric *dMetric = nullptr;
     float2 *dInvMetric = nullptr;
     float *dDepthF = nullptr;
     int metricSemantics = -1;
@@ -64,12 +64,12 @@ struct wacomm_b200_context {
     std::vector<double> times;
     std::vector<FrameSlot> slots;
 
-    void *dNodes = nullptr;
-    size_t nodesBytes = 0;
+    NodeRecord *dNodes = nullptr;
+    size_t nodesCap = 0, surfCap = 0;
     void *dCells = nullptr, *dCellSurface = nullptr;
     size_t cellsBytes = 0, cellSurfaceBytes = 0;
-    bool pairCells = false;
-    SurfPair *dSurf = nullptr;
+    bool pairCells = false, pairNodes = false;
+    SurfRecord *dSurf = nullptr;
     EnvPair *dEnv = nullptr;
     int pairT0 = -1, pairT1 = -1, pairStorage = -1;
     bool pairEnv = false;
@@ -433,16 +433,14 @@ void release_environment(wacomm_b200_context *ctx) {
     }
 }
 
-// Device buffers of the packed forcing pair (node records, environment pair, cell-column records).
+// Device buffers of the packed forcing pair: the environment pair, the cell-column records of the
+// FP32 step or the node and surface records of the reference arithmetic.
 int reserve_pair_buffers(wacomm_b200_context *ctx, bool env, bool cells) {
     size_t plane = (size_t)ctx->eta * ctx->xi;
-    size_t need = plane * ctx->sW * node_record_bytes(ctx->opt.storage);
-    if (need > ctx->nodesBytes) {
-        cudaFree(ctx->dNodes);
-        ctx->dNodes = nullptr;
-        ctx->nodesBytes = 0;
-        CUDA_TRY(ctx, cudaMalloc(&ctx->dNodes, need));
-        ctx->nodesBytes = need;
+    int rc;
+    if (!cells) {
+        if ((rc = grow(ctx, ctx->dNodes, ctx->nodesCap, plane * ctx->sW))) return rc;
+        if ((rc = grow(ctx, ctx->dSurf, ctx->surfCap, plane))) return rc;
     }
     if (env && !ctx->dEnv) CUDA_TRY(ctx, cudaMalloc(&ctx->dEnv, plane * sizeof(EnvPair)));
     if (cells) {
@@ -471,24 +469,28 @@ int ensure_pair(wacomm_b200_context *ctx, int t0, int t1, int &launches) {
     bool env = a.windU || a.windV || a.stokesU || b.windU || b.windV || b.stokesU;
     bool cells = ctx->opt.arithmetic == WACOMM_B200_ARITH_FP32;
     if (ctx->pairT0 == t0 && ctx->pairT1 == t1 && ctx->pairStorage == ctx->opt.storage &&
-        ctx->pairEnv == env && (!cells || ctx->pairCells))
+        ctx->pairEnv == env && (cells ? ctx->pairCells : ctx->pairNodes))
         return WACOMM_B200_OK;
     int rc = reserve_pair_buffers(ctx, env, cells);
     if (rc) return rc;
-    CUDA_TRY(ctx, pack_pair(ctx->opt.storage, ctx->eta, ctx->xi, ctx->sW, a, b,
-                            ctx->dH, ctx->dNodes, ctx->dSurf, env ? ctx->dEnv : nullptr,
-                            ctx->stream));
-    launches += 2;
+    if (env) {
+        CUDA_TRY(ctx, pack_environment(ctx->eta, ctx->xi, a, b, ctx->dEnv, ctx->stream));
+        launches++;
+    }
     if (cells) {
         CUDA_TRY(ctx, pack_cells(ctx->opt.storage, ctx->eta, ctx->xi, ctx->sW, a, b, ctx->dH,
                                  ctx->dCells, ctx->dCellSurface, ctx->stream));
-        launches += 2;
+    } else {
+        CUDA_TRY(ctx, pack_pair(ctx->eta, ctx->xi, ctx->sW, a, b, ctx->dH, ctx->dNodes, ctx->dSurf,
+                                ctx->stream));
     }
+    launches += 2;
     ctx->pairT0 = t0;
     ctx->pairT1 = t1;
     ctx->pairStorage = ctx->opt.storage;
     ctx->pairEnv = env;
     ctx->pairCells = cells;
+    ctx->pairNodes = !cells;
     return WACOMM_B200_OK;
 }
 
@@ -1065,6 +1067,7 @@ int wacomm_b200_set_grid(wacomm_b200_context *ctx, int eta, int xi, int s_rho, i
     ctx->dInvMetric = nullptr;
     ctx->dDepthF = nullptr;
     ctx->dSurf = nullptr;
+    ctx->surfCap = 0;
     cudaFree(ctx->dEnv);
     ctx->dEnv = nullptr;
     ctx->hasGrid = false;
@@ -1079,10 +1082,9 @@ int wacomm_b200_set_grid(wacomm_b200_context *ctx, int eta, int xi, int s_rho, i
     CUDA_TRY(ctx, cudaMalloc(&ctx->dLat, plane * sizeof(double)));
     CUDA_TRY(ctx, cudaMalloc(&ctx->dH, plane * sizeof(double)));
     CUDA_TRY(ctx, cudaMalloc(&ctx->dDepth, (size_t)(s_w - 1) * sizeof(double)));
-    CUDA_TRY(ctx, cudaMalloc(&ctx->dMetric, plane * sizeof(double2)));
+    CUDA_TRY(ctx, cudaMalloc(&ctx->dMetric, plane * sizeof(CellMetric)));
     CUDA_TRY(ctx, cudaMalloc(&ctx->dInvMetric, plane * sizeof(float2)));
     CUDA_TRY(ctx, cudaMalloc(&ctx->dDepthF, (size_t)(s_w - 1) * sizeof(float)));
-    CUDA_TRY(ctx, cudaMalloc(&ctx->dSurf, plane * sizeof(SurfPair)));
     CUDA_TRY(ctx, cudaMemcpy(ctx->dLon, lon_rad, plane * sizeof(double), cudaMemcpyHostToDevice));
     CUDA_TRY(ctx, cudaMemcpy(ctx->dLat, lat_rad, plane * sizeof(double), cudaMemcpyHostToDevice));
     CUDA_TRY(ctx, cudaMemcpy(ctx->dH, h, plane * sizeof(double), cudaMemcpyHostToDevice));

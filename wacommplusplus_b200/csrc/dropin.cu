@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(256) dropin_move_kernel(
     p.type = rec.driftObjectType;
     p.side = rec.driftSide;
     double elapsed = P.elapsed0;
-    move_particle<SEM_DEVICE, ARITH_REF>(cfg, P, view, p, elapsed, nullptr);
+    move_particle<SEM_DEVICE, true, false>(cfg, P, view, p, elapsed, nullptr);
     rec.k = p.k;
     rec.j = p.j;
     rec.i = p.i;
@@ -94,7 +94,7 @@ int dropin_move(const wacomm_b200_config *config, wacomm_b200_particle *particle
     V.u = u;
     V.v = v;
     V.w = w;
-    V.akt = akt;
+    V.aktField = akt;
     V.windU = windU;
     V.windV = windV;
     V.stokesU = stokesU;

@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(256) noalloc_move_kernel(
     p.type = rec.driftObjectType;
     p.side = rec.driftSide;
     double elapsed = P.elapsed0;
-    move_particle<SEM_DEVICE, ARITH_REF>(cfg, P, view, p, elapsed, nullptr);
+    move_particle<SEM_DEVICE, true, false>(cfg, P, view, p, elapsed, nullptr);
     rec.k = p.k;
     rec.j = p.j;
     rec.i = p.i;
@@ -215,7 +215,7 @@ extern "C" int wacomm_b200_cuda_move_particle_noalloc(
     V.u = u;
     V.v = v;
     V.w = w;
-    V.akt = akt;
+    V.aktField = akt;
     V.windU = wind_u10;
     V.windV = wind_v10;
     V.stokesU = stokes_u;

@@ -16,17 +16,19 @@ namespace wb {
 struct IntervalParams;
 struct ParticleSoA;
 struct MoveLaunch;
-struct SurfPair;
+struct NodeRecord;
+struct SurfRecord;
+struct CellMetric;
 struct EnvPair;
 
 struct PackedArgs {
     int eta, xi, sW, sRho;
-    const void *nodes;  // NodeRecord<storage>[sW][eta][xi]
-    const SurfPair *surf;
+    const NodeRecord *nodes;  // [sW][eta][xi] (reference arithmetic)
+    const SurfRecord *surf;   // [eta][xi] (reference arithmetic)
     const EnvPair *env;
     bool hasWindU, hasWindV, hasStokes;
     const double *lonRad, *latRad, *depthIntervals;
-    const double2 *metric;
+    const CellMetric *metric;
     const float2 *invMetric;           // {1/xdist, 1/ydist} per cell (FP32 step)
     const float *depthIntervalsF;      // FP32 copy of depthIntervals (FP32 step)
     const wacomm_b200_config *cfgDevice;  // device copy of the run parameters (FP32 step, drift)
@@ -45,17 +47,19 @@ cudaError_t move_f32_dispatch(int semantics, int storage, int shape, const wacom
 
 // support.cu ----------------------------------------------------------------------------
 
-// Size in bytes of one node record of the packed pair.
-size_t node_record_bytes(int storage);
-
 struct FrameDevice {  // one forcing record in the reference layout (device)
     const float *zeta, *u, *v, *w, *akt;
     const float *windU, *windV, *stokesU, *stokesV;
 };
 
-cudaError_t pack_pair(int storage, int eta, int xi, int sW, const FrameDevice &f0,
-                      const FrameDevice &f1, const double *h, void *nodes, SurfPair *surf,
-                      EnvPair *env, cudaStream_t stream);
+// Node and surface records of the pair for the reference arithmetic (views.cuh).
+size_t node_record_bytes();
+size_t surf_record_bytes();
+cudaError_t pack_pair(int eta, int xi, int sW, const FrameDevice &f0, const FrameDevice &f1,
+                      const double *h, NodeRecord *nodes, SurfRecord *surf, cudaStream_t stream);
+// Wind and Stokes records of the pair (fields a record lacks are zero).
+cudaError_t pack_environment(int eta, int xi, const FrameDevice &f0, const FrameDevice &f1,
+                             EnvPair *env, cudaStream_t stream);
 
 // Cell-column layout of the pair for the FP32 step (views.cuh): bytes per (cell, level) and per
 // cell surface, and the packing kernel.
@@ -66,7 +70,7 @@ cudaError_t pack_cells(int storage, int eta, int xi, int sW, const FrameDevice &
                        cudaStream_t stream);
 
 cudaError_t build_metric(int semantics, int eta, int xi, const double *lonRad,
-                         const double *latRad, double2 *metric, float2 *invMetric,
+                         const double *latRad, CellMetric *metric, float2 *invMetric,
                          cudaStream_t stream);
 
 // Exclusive scan of n uint32 values; `temp` must hold scan_temp_words(n) words. The total is
@@ -258,7 +262,7 @@ void surrogate_pack(const float *flat, uint8_t *out);
 long long surrogate_cell_levels(int eta, int xi, int sW);
 cudaError_t surrogate_cells(int eta, int xi, int sW, int sRho, const FrameDevice &f0,
                             const FrameDevice &f1, const double *h, const double *depthIntervals,
-                            const double2 *metric, const uint8_t *weights, __half *z, void *corners,
+                            const CellMetric *metric, const uint8_t *weights, __half *z, void *corners,
                             int *err, int smCount, cudaStream_t stream);
 // The step kernel (layers 1-4 of every work item into s.rows) and the post kernel (displacement,
 // closures, state, concentration, fallback list) or, for diffusive intervals, the walk kernel

@@ -9,26 +9,9 @@
 namespace wb {
 
 template <int STORE>
-inline PackedView<STORE> typed_view(const PackedArgs &A) {
-    PackedView<STORE> V;
-    V.g = GridShape{A.eta, A.xi, A.sW, A.sRho};
-    V.nodes = static_cast<const NodeRecord<STORE> *>(A.nodes);
-    V.surf = A.surf;
-    V.env = A.env;
-    V.hasWindU = A.hasWindU;
-    V.hasWindV = A.hasWindV;
-    V.hasStokes = A.hasStokes;
-    V.lonRad = A.lonRad;
-    V.latRad = A.latRad;
-    V.depthIntervals = A.depthIntervals;
-    V.metric = A.metric;
-    return V;
-}
-
-template <int STORE>
 inline FastView<STORE> fast_view(const PackedArgs &A) {
     FastView<STORE> F;
-    F.V = typed_view<STORE>(A);
+    F.V = packed_view(A);
     F.X.invMetric = A.invMetric;
     F.X.depthIntervals = A.depthIntervalsF;
     F.X.cfgDevice = A.cfgDevice;

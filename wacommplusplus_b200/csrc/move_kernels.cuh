@@ -1,6 +1,7 @@
 // Move kernels: one thread per particle, the whole interval (or one chunk of it) in registers.
 #pragma once
 
+#include "engine.h"
 #include "step.cuh"
 #include "step_fast.cuh"
 
@@ -14,6 +15,22 @@ struct ParticleSoA {
     int8_t *side;
     double *elapsed;  // resume point between chunks
 };
+
+inline PackedView packed_view(const PackedArgs &A) {
+    PackedView V;
+    V.g = GridShape{A.eta, A.xi, A.sW, A.sRho};
+    V.nodes = A.nodes;
+    V.surf = A.surf;
+    V.env = A.env;
+    V.hasWindU = A.hasWindU;
+    V.hasWindV = A.hasWindV;
+    V.hasStokes = A.hasStokes;
+    V.lonRad = A.lonRad;
+    V.latRad = A.latRad;
+    V.depthIntervals = A.depthIntervals;
+    V.metric = A.metric;
+    return V;
+}
 
 struct MoveLaunch {
     int count;                    // work items
@@ -95,11 +112,18 @@ __device__ __forceinline__ void warp_sum_steps(unsigned long long *counter, int 
     if ((threadIdx.x & 31) == 0 && counter && steps) atomicAdd(counter, (unsigned long long)steps);
 }
 
-template <int SEM, int ARITH, int STORE>
-__global__ void __launch_bounds__(256) move_soa_kernel(const wacomm_b200_config cfg,
-                                                       const IntervalParams P,
-                                                       const PackedView<STORE> V, ParticleSoA S,
-                                                       const MoveLaunch L) {
+// Reference arithmetic. The latency of FP64 chains and the conversions to float and back bound it;
+// 128 registers allow 16 warps per SM. Where one or two warps per scheduler hold all records (KEEP)
+// the registers go to the velocity stencil instead, out of the substep's chain of loads. Move kernel,
+// KEEP / not: 16,384 records 0.366 / 0.449 ms, 65,536 0.751 / 0.802 ms, 131,072 1.37 / 1.36 ms,
+// 500,009 4.73 / 3.71 ms (with the random walk 0.609 / 0.687, 1.28 / 1.15, 2.44 / 1.96, 8.14 / 6.30);
+// 242 registers and float operands before: 500,009 with the random walk 10.2 ms, XU pipe 54 -> 22 %,
+// FP64 24 -> 44 %, issue 36 -> 57 %.
+template <int SEM, bool DRIFT, bool KEEP>
+__global__ void __launch_bounds__(256, KEEP ? 1 : 2) move_soa_kernel(const wacomm_b200_config cfg,
+                                                          const IntervalParams P,
+                                                          const PackedView V, ParticleSoA S,
+                                                          const MoveLaunch L) {
     const unsigned t = launch_item(L, blockIdx.x * (blockDim.x >> 5) * L.lanes, L.count);
     long long cell = -1;
     int steps = 0;
@@ -116,7 +140,7 @@ __global__ void __launch_bounds__(256) move_soa_kernel(const wacomm_b200_config 
         p.type = S.type[slot];
         p.side = S.side[slot];
         double elapsed = P.firstChunk ? P.elapsed0 : S.elapsed[slot];
-        steps = move_particle<SEM, ARITH>(cfg, P, V, p, elapsed, L.err);
+        steps = move_particle<SEM, DRIFT, KEEP>(cfg, P, V, p, elapsed, L.err);
         S.k[slot] = p.k;
         S.j[slot] = p.j;
         S.i[slot] = p.i;
@@ -211,10 +235,12 @@ cudaError_t launch_move_fast(const wacomm_b200_config &cfg, const IntervalParams
     return cudaGetLastError();
 }
 
+constexpr int KEEP_RECORDS = 2 * 4 * 148 * 32;  // two full warps per scheduler
+
 // Host launchers (one per template instance, defined in the instantiation units).
-template <int SEM, int ARITH, int STORE>
+template <int SEM>
 cudaError_t launch_move_soa(const wacomm_b200_config &cfg, const IntervalParams &P,
-                            const PackedView<STORE> &V, const ParticleSoA &S, const MoveLaunch &L,
+                            const PackedView &V, const ParticleSoA &S, const MoveLaunch &L,
                             int blockSize, cudaStream_t stream) {
     if (L.count <= 0) return cudaSuccess;
     MoveLaunch M = L;
@@ -222,7 +248,14 @@ cudaError_t launch_move_soa(const wacomm_b200_config &cfg, const IntervalParams 
     spread_launch(L.count, blockSize, M.lanes, threads);
     const int items = threads / 32 * M.lanes;
     const int blocks = (L.count + items - 1) / items;
-    move_soa_kernel<SEM, ARITH, STORE><<<blocks, threads, 0, stream>>>(cfg, P, V, S, M);
+    const bool keep = L.count <= KEEP_RECORDS;
+    if (cfg.driftModel == 1) {
+        if (keep) move_soa_kernel<SEM, true, true><<<blocks, threads, 0, stream>>>(cfg, P, V, S, M);
+        else move_soa_kernel<SEM, true, false><<<blocks, threads, 0, stream>>>(cfg, P, V, S, M);
+    } else {
+        if (keep) move_soa_kernel<SEM, false, true><<<blocks, threads, 0, stream>>>(cfg, P, V, S, M);
+        else move_soa_kernel<SEM, false, false><<<blocks, threads, 0, stream>>>(cfg, P, V, S, M);
+    }
     return cudaGetLastError();
 }
 

@@ -3,10 +3,9 @@
 //
 // SEM selects the rules of the reference path being replaced: SEM_HOST follows
 // Particle::move (Particle.cpp:71-824), SEM_DEVICE follows the reference kernel
-// (kernel.cu:153-368); the few places where they differ are marked. ARITH_REF reproduces the
-// reference arithmetic (FP64 with float-rounded corner terms; compiled with -fmad=false so that
-// no product is fused), ARITH_F32 interpolates in FP32 and keeps FP64 for positions, time
-// weights and metric ratios.
+// (kernel.cu:153-368); the few places where they differ are marked. The arithmetic is the
+// reference's (FP64 with float-rounded corner terms; compiled with -fmad=false so that no product is
+// fused except where it is written so).
 #pragma once
 
 #include "common.cuh"
@@ -110,79 +109,120 @@ struct ParticleState {
 
 // ------------------------------------------------------------------ interpolation pieces
 
-// (float)interpolateTime(v0, v1, alpha) (NumericalHelpers.hpp:37-39, kernel.cu:71-74).
-__device__ __forceinline__ float at_ref(float v0, float v1, double a) {
-    return (float)((1.0 - a) * (double)v0 + a * (double)v1);
+// x rounded to float precision and range grid (the value of (float)x for every |x| below the float
+// overflow bound): adding and subtracting 1.5 2^29 times the power of two of x (of 2^-126 for smaller
+// x, the grid of the subnormal floats) rounds to nearest, ties to even, at the float's last place.
+// Two FP64 adds and four integer instructions in place of a conversion to float and one back, both
+// on the quarter-rate unit that bounds the reference arithmetic.
+__device__ __forceinline__ double rounded_to_float(double x) {
+    const int power = max(__double2hiint(x) & 0x7ff00000, (1023 - 126) << 20);
+    const double shift = __hiloint2double(power + (29 << 20) + (1 << 19), 0);
+    return __dadd_rn(__dadd_rn(x, shift), -shift);
 }
+
+// (float)interpolateTime(v0, v1, alpha) (NumericalHelpers.hpp:37-39, kernel.cu:71-74) as a double;
+// v0 and v1 hold float values, as floats or as doubles.
+template <class T>
+__device__ __forceinline__ double at_ref(T v0, T v1, double a) {
+    return rounded_to_float((1.0 - a) * (double)v0 + a * (double)v1);
+}
+__device__ __forceinline__ double at_ref(double2 v, double a) { return at_ref(v.x, v.y, a); }
 __device__ __forceinline__ float at_f32(float v0, float v1, float a) { return fmaf(a, v1 - v0, v0); }
 
-// Bilinear corner weights in reference order: (j,i), (j+1,i), (j+1,i+1), (j,i+1).
-struct Weights32 {
-    float w1, w2, w3, w4;
-};
-__device__ __forceinline__ Weights32 weights32(double jF, double iF) {
-    float fj = (float)jF, fi = (float)iF;
-    return Weights32{(1.f - fi) * (1.f - fj), (1.f - fi) * fj, fi * fj, fi * (1.f - fj)};
+// a / b correctly rounded from r = 1 / b correctly rounded: the product with r, then two
+// residual corrections (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990: a quotient within one unit in the last place, corrected once more
+// with the correctly rounded reciprocal, is the rounded quotient). 5 FP64 instructions instead of a
+// division's reciprocal iteration and range tests.
+__device__ __forceinline__ double quotient(double a, double b, double r) {
+    double q = a * r;
+    if (!(fabs(q) <= DBL_MAX)) return a / b;
+    q = __fma_rn(__fma_rn(-b, q, a), r, q);
+    return __fma_rn(__fma_rn(-b, q, a), r, q);
+}
+
+// Adding 1.5 2^52 rounds |x| < 2^31 to an integer in the direction of the add and leaves it in the
+// sum's low word: floor and ceil with their index in two FP64 adds, no conversion on the
+// quarter-rate unit.
+constexpr double INTEGER_SHIFT = 6755399441055744.0;
+
+// floor(x) as to_index gives it, and x - floor(x) as x - index.
+template <int SEM>
+__device__ __forceinline__ int floor_index(double x, double &fraction) {
+    if (fabs(x) < 2147483648.0) {
+        const double shifted = __dadd_rd(x, INTEGER_SHIFT);
+        fraction = x - (shifted - INTEGER_SHIFT);
+        return __double2loint(shifted);
+    }
+    const int index = to_index<SEM>(floor(x));
+    fraction = x - index;
+    return index;
+}
+
+// ceil(k) as to_index gives it, and ceil(k) - k.
+template <int SEM>
+__device__ __forceinline__ int ceil_index(double k, double &fraction) {
+    if (fabs(k) < 2147483648.0) {
+        const double shifted = __dadd_ru(k, INTEGER_SHIFT);
+        fraction = (shifted - INTEGER_SHIFT) - k;
+        return __double2loint(shifted);
+    }
+    const double up = ceil(k);
+    fraction = up - k;
+    return to_index<SEM>(up);
 }
 
 // Float sum of four float-rounded corner terms c*(1-iF)*(1-jF) ... (Particle.cpp:271-277).
-__device__ __forceinline__ float bilinear_ref(float c1, float c2, float c3, float c4, double jF,
+__device__ __forceinline__ float bilinear_ref(double c1, double c2, double c3, double c4, double jF,
                                               double iF) {
-    float f1 = (float)((double)c1 * (1.0 - iF) * (1.0 - jF));
-    float f2 = (float)((double)c2 * (1.0 - iF) * jF);
-    float f3 = (float)((double)c3 * iF * jF);
-    float f4 = (float)((double)c4 * iF * (1.0 - jF));
+    float f1 = (float)(c1 * (1.0 - iF) * (1.0 - jF));
+    float f2 = (float)(c2 * (1.0 - iF) * jF);
+    float f3 = (float)(c3 * iF * jF);
+    float f4 = (float)(c4 * iF * (1.0 - jF));
     return f1 + f2 + f3 + f4;
 }
 
 // Surface at a position: bilinear h (double) and zeta (float) (Particle.cpp:271-290;
 // kernel.cu:197-198).
-template <int ARITH, class View>
+template <class View>
 __device__ __forceinline__ void surface_at(const View &V, int jI, int iI, double jF, double iF,
                                            double alpha, double &hh, float &zz) {
-    SurfPair s1 = V.surface(jI, iI), s2 = V.surface(jI + 1, iI);
-    SurfPair s3 = V.surface(jI + 1, iI + 1), s4 = V.surface(jI, iI + 1);
+    const auto s1 = V.surface(jI, iI), s2 = V.surface(jI + 1, iI);
+    const auto s3 = V.surface(jI + 1, iI + 1), s4 = V.surface(jI, iI + 1);
     hh = s1.h * (1.0 - iF) * (1.0 - jF) + s2.h * (1.0 - iF) * jF + s3.h * iF * jF +
          s4.h * iF * (1.0 - jF);
-    if (ARITH == ARITH_REF) {
-        zz = bilinear_ref(at_ref(s1.z0, s1.z1, alpha), at_ref(s2.z0, s2.z1, alpha),
-                          at_ref(s3.z0, s3.z1, alpha), at_ref(s4.z0, s4.z1, alpha), jF, iF);
-    } else {
-        float a = (float)alpha;
-        Weights32 w = weights32(jF, iF);
-        zz = at_f32(s1.z0, s1.z1, a) * w.w1 + at_f32(s2.z0, s2.z1, a) * w.w2 +
-             at_f32(s3.z0, s3.z1, a) * w.w3 + at_f32(s4.z0, s4.z1, a) * w.w4;
-    }
+    zz = bilinear_ref(at_ref(s1.z0, s1.z1, alpha), at_ref(s2.z0, s2.z1, alpha),
+                      at_ref(s3.z0, s3.z1, alpha), at_ref(s4.z0, s4.z1, alpha), jF, iF);
 }
 
 // hcMid of the host rules: one double chain of four h and four zeta terms (Particle.cpp:601-604).
 template <class View>
 __device__ __forceinline__ double hc_mid_host(const View &V, int jI, int iI, double jF, double iF,
                                               double alpha) {
-    SurfPair s1 = V.surface(jI, iI), s2 = V.surface(jI + 1, iI);
-    SurfPair s3 = V.surface(jI + 1, iI + 1), s4 = V.surface(jI, iI + 1);
+    const auto s1 = V.surface(jI, iI), s2 = V.surface(jI + 1, iI);
+    const auto s3 = V.surface(jI + 1, iI + 1), s4 = V.surface(jI, iI + 1);
     return s1.h * (1.0 - iF) * (1.0 - jF) + s2.h * (1.0 - iF) * jF + s3.h * iF * jF +
-           s4.h * iF * (1.0 - jF) + (double)at_ref(s1.z0, s1.z1, alpha) * (1.0 - iF) * (1.0 - jF) +
-           (double)at_ref(s2.z0, s2.z1, alpha) * (1.0 - iF) * jF +
-           (double)at_ref(s3.z0, s3.z1, alpha) * iF * jF +
-           (double)at_ref(s4.z0, s4.z1, alpha) * iF * (1.0 - jF);
+           s4.h * iF * (1.0 - jF) + at_ref(s1.z0, s1.z1, alpha) * (1.0 - iF) * (1.0 - jF) +
+           at_ref(s2.z0, s2.z1, alpha) * (1.0 - iF) * jF +
+           at_ref(s3.z0, s3.z1, alpha) * iF * jF +
+           at_ref(s4.z0, s4.z1, alpha) * iF * (1.0 - jF);
 }
 
 // Vertical field blend: host rules sum eight float terms (Particle.cpp:464-474, 490-500);
 // device rules blend two float bilinears in double (kernel.cu:258-259, 265-266).
 template <int SEM>
-__device__ __forceinline__ double trilinear_ref(float u1, float u2, float u3, float u4, float l1,
-                                                float l2, float l3, float l4, double kF,
+__device__ __forceinline__ double trilinear_ref(double u1, double u2, double u3, double u4,
+                                                double l1, double l2, double l3, double l4, double kF,
                                                 double jF, double iF) {
     if (SEM == SEM_HOST) {
-        float w1 = (float)((double)u1 * (1.0 - iF) * (1.0 - jF) * (1.0 - kF));
-        float w2 = (float)((double)u2 * (1.0 - iF) * jF * (1.0 - kF));
-        float w3 = (float)((double)u3 * iF * jF * (1.0 - kF));
-        float w4 = (float)((double)u4 * iF * (1.0 - jF) * (1.0 - kF));
-        float w5 = (float)((double)l1 * (1.0 - iF) * (1.0 - jF) * kF);
-        float w6 = (float)((double)l2 * (1.0 - iF) * jF * kF);
-        float w7 = (float)((double)l3 * iF * jF * kF);
-        float w8 = (float)((double)l4 * iF * (1.0 - jF) * kF);
+        float w1 = (float)(u1 * (1.0 - iF) * (1.0 - jF) * (1.0 - kF));
+        float w2 = (float)(u2 * (1.0 - iF) * jF * (1.0 - kF));
+        float w3 = (float)(u3 * iF * jF * (1.0 - kF));
+        float w4 = (float)(u4 * iF * (1.0 - jF) * (1.0 - kF));
+        float w5 = (float)(l1 * (1.0 - iF) * (1.0 - jF) * kF);
+        float w6 = (float)(l2 * (1.0 - iF) * jF * kF);
+        float w7 = (float)(l3 * iF * jF * kF);
+        float w8 = (float)(l4 * iF * (1.0 - jF) * kF);
         return (double)(w1 + w2 + w3 + w4 + w5 + w6 + w7 + w8);
     } else {
         return (double)bilinear_ref(u1, u2, u3, u4, jF, iF) * (1.0 - kF) +
@@ -205,33 +245,19 @@ struct DrawKeys {
 
 // Ocean current plus leeway and Stokes at a fractional position and forcing weight
 // (Particle.cpp:352-475; kernel.cu:206-260). kI must already be a valid memory level.
-template <int SEM, int ARITH, class View>
+template <int SEM, bool DRIFT, class View>
 __device__ __forceinline__ void advective_velocity(const wacomm_b200_config &cfg,
                                                    const IntervalParams &P, const View &V,
-                                                   const ParticleState &p, int kI, double kF,
-                                                   int jI, double jF, int iI, double iF,
+                                                   const RefStencil &s, const ParticleState &p,
+                                                   double kF, int jI, double jF, int iI, double iF,
                                                    double sa, double elapsed,
                                                    double physicalTime, double stepDt,
-                                                   const DrawKeys &keys, float &uu, float &vv,
-                                                   double &ww, int *err) {
-    NodeUp c1 = V.up(kI, jI, iI), c2 = V.up(kI, jI + 1, iI);
-    NodeUp c3 = V.up(kI, jI + 1, iI + 1), c4 = V.up(kI, jI, iI + 1);
-    NodeLo l1 = V.lo(kI, jI, iI), l2 = V.lo(kI, jI + 1, iI);
-    NodeLo l3 = V.lo(kI, jI + 1, iI + 1), l4 = V.lo(kI, jI, iI + 1);
-    if (ARITH == ARITH_REF) {
-        uu = bilinear_ref(at_ref(c1.u0, c1.u1, sa), at_ref(c2.u0, c2.u1, sa),
-                          at_ref(c3.u0, c3.u1, sa), at_ref(c4.u0, c4.u1, sa), jF, iF);
-        vv = bilinear_ref(at_ref(c1.v0, c1.v1, sa), at_ref(c2.v0, c2.v1, sa),
-                          at_ref(c3.v0, c3.v1, sa), at_ref(c4.v0, c4.v1, sa), jF, iF);
-    } else {
-        float a = (float)sa;
-        Weights32 w = weights32(jF, iF);
-        uu = at_f32(c1.u0, c1.u1, a) * w.w1 + at_f32(c2.u0, c2.u1, a) * w.w2 +
-             at_f32(c3.u0, c3.u1, a) * w.w3 + at_f32(c4.u0, c4.u1, a) * w.w4;
-        vv = at_f32(c1.v0, c1.v1, a) * w.w1 + at_f32(c2.v0, c2.v1, a) * w.w2 +
-             at_f32(c3.v0, c3.v1, a) * w.w3 + at_f32(c4.v0, c4.v1, a) * w.w4;
-    }
-    if (cfg.driftModel == 1 && p.type != 0) {
+                                                   float &uu, float &vv, double &ww, int *err) {
+    uu = bilinear_ref(at_ref(s.u[0], sa), at_ref(s.u[1], sa), at_ref(s.u[2], sa), at_ref(s.u[3], sa),
+                      jF, iF);
+    vv = bilinear_ref(at_ref(s.v[0], sa), at_ref(s.v[1], sa), at_ref(s.v[2], sa), at_ref(s.v[3], sa),
+                      jF, iF);
+    if (DRIFT && cfg.driftModel == 1 && p.type != 0) {
         if (SEM == SEM_HOST && (p.type < 0 || p.type > 22)) atomicOr(err, ERR_DRIFT_OBJECT);
         double windU = cfg.windU10, windV = cfg.windV10;
         EnvPair e1{}, e2{}, e3{}, e4{};
@@ -309,45 +335,21 @@ __device__ __forceinline__ void advective_velocity(const wacomm_b200_config &cfg
             vv += (float)((1.0 - sa) * fv + sa * nv);
         }
     }
-    if (ARITH == ARITH_REF) {
-        ww = trilinear_ref<SEM>(at_ref(c1.w0, c1.w1, sa), at_ref(c2.w0, c2.w1, sa),
-                                at_ref(c3.w0, c3.w1, sa), at_ref(c4.w0, c4.w1, sa),
-                                at_ref(l1.w0, l1.w1, sa), at_ref(l2.w0, l2.w1, sa),
-                                at_ref(l3.w0, l3.w1, sa), at_ref(l4.w0, l4.w1, sa), kF, jF, iF);
-    } else {
-        float a = (float)sa, fk = (float)kF;
-        Weights32 w = weights32(jF, iF);
-        float up = at_f32(c1.w0, c1.w1, a) * w.w1 + at_f32(c2.w0, c2.w1, a) * w.w2 +
-                   at_f32(c3.w0, c3.w1, a) * w.w3 + at_f32(c4.w0, c4.w1, a) * w.w4;
-        float lo = at_f32(l1.w0, l1.w1, a) * w.w1 + at_f32(l2.w0, l2.w1, a) * w.w2 +
-                   at_f32(l3.w0, l3.w1, a) * w.w3 + at_f32(l4.w0, l4.w1, a) * w.w4;
-        ww = (double)(up * (1.f - fk) + lo * fk);
-    }
+    ww = trilinear_ref<SEM>(at_ref(s.wUp[0], sa), at_ref(s.wUp[1], sa), at_ref(s.wUp[2], sa),
+                            at_ref(s.wUp[3], sa), at_ref(s.wLo[0], sa), at_ref(s.wLo[1], sa),
+                            at_ref(s.wLo[2], sa), at_ref(s.wLo[3], sa), kF, jF, iF);
 }
 
 // Vertical diffusivity at the particle (Particle.cpp:490-500; kernel.cu:265-266).
-template <int SEM, int ARITH, class View>
+template <int SEM, class View>
 __device__ __forceinline__ double akt_at(const View &V, int kI, double kF, int jI, double jF,
                                          int iI, double iF, double alpha) {
-    NodeUp c1 = V.up(kI, jI, iI), c2 = V.up(kI, jI + 1, iI);
-    NodeUp c3 = V.up(kI, jI + 1, iI + 1), c4 = V.up(kI, jI, iI + 1);
-    NodeLo l1 = V.lo(kI, jI, iI), l2 = V.lo(kI, jI + 1, iI);
-    NodeLo l3 = V.lo(kI, jI + 1, iI + 1), l4 = V.lo(kI, jI, iI + 1);
-    if (ARITH == ARITH_REF) {
-        return trilinear_ref<SEM>(at_ref(c1.a0, c1.a1, alpha), at_ref(c2.a0, c2.a1, alpha),
-                                  at_ref(c3.a0, c3.a1, alpha), at_ref(c4.a0, c4.a1, alpha),
-                                  at_ref(l1.a0, l1.a1, alpha), at_ref(l2.a0, l2.a1, alpha),
-                                  at_ref(l3.a0, l3.a1, alpha), at_ref(l4.a0, l4.a1, alpha), kF,
-                                  jF, iF);
-    } else {
-        float a = (float)alpha, fk = (float)kF;
-        Weights32 w = weights32(jF, iF);
-        float up = at_f32(c1.a0, c1.a1, a) * w.w1 + at_f32(c2.a0, c2.a1, a) * w.w2 +
-                   at_f32(c3.a0, c3.a1, a) * w.w3 + at_f32(c4.a0, c4.a1, a) * w.w4;
-        float lo = at_f32(l1.a0, l1.a1, a) * w.w1 + at_f32(l2.a0, l2.a1, a) * w.w2 +
-                   at_f32(l3.a0, l3.a1, a) * w.w3 + at_f32(l4.a0, l4.a1, a) * w.w4;
-        return (double)(up * (1.f - fk) + lo * fk);
-    }
+    return trilinear_ref<SEM>(
+        at_ref(V.akt(kI, jI, iI), alpha), at_ref(V.akt(kI, jI + 1, iI), alpha),
+        at_ref(V.akt(kI, jI + 1, iI + 1), alpha), at_ref(V.akt(kI, jI, iI + 1), alpha),
+        at_ref(V.akt(kI - 1, jI, iI), alpha), at_ref(V.akt(kI - 1, jI + 1, iI), alpha),
+        at_ref(V.akt(kI - 1, jI + 1, iI + 1), alpha), at_ref(V.akt(kI - 1, jI, iI + 1), alpha), kF,
+        jF, iF);
 }
 
 __device__ __forceinline__ void close_upper(const wacomm_b200_config &cfg, double &k, double &health,
@@ -368,8 +370,10 @@ __device__ __forceinline__ void close_lower(const wacomm_b200_config &cfg, doubl
 
 // Integrates particle p from `elapsed` while substeps start before min(length, chunkEnd).
 // On return `elapsed` is where the next chunk resumes (>= length when the particle is done).
-// Returns the number of substeps taken (particle-steps of this launch).
-template <int SEM, int ARITH, class View>
+// Returns the number of substeps taken (particle-steps of this launch). DRIFT false leaves the
+// drifting objects' branch out, for runs without a drift model; KEEP holds the velocity stencil (64
+// registers) from substep to substep, for launches with registers to spare.
+template <int SEM, bool DRIFT, bool KEEP, class View>
 __device__ int move_particle(const wacomm_b200_config &cfg, const IntervalParams &P,
                              const View &V, ParticleState &p, double &elapsed, int *err) {
     const int eta = V.g.eta, xi = V.g.xi, sW = V.g.sW;
@@ -390,6 +394,18 @@ __device__ int move_particle(const wacomm_b200_config &cfg, const IntervalParams
     keys.prefix = fold(fold(mix64(cfg.randomSeed), p.id), (uint64_t)P.intervalKey);
     keys.philoxKey = p.id ^ mix64(cfg.randomSeed);
     const double stop = P.chunkEnd < length ? P.chunkEnd : length;
+    const double rLength = 1.0 / length;
+    // The velocity stencil of the particle's cell and level; KEEP: read again only when either
+    // changes.
+    RefStencil kept;
+    long long keptColumn = -1;
+    auto keep_column = [&](int kI, int jI, int iI) {
+        const long long column = ((long long)(kI + sW - 1) * eta + jI) * xi + iI;
+        if (!KEEP || column != keptColumn) {
+            V.stencil(kI, jI, iI, kept);
+            keptColumn = column;
+        }
+    };
 
     while (elapsed < stop) {
         double stepDt = SEM == SEM_HOST ? smin(cfg.dti, length - elapsed)
@@ -413,10 +429,9 @@ __device__ int move_particle(const wacomm_b200_config &cfg, const IntervalParams
             elapsed = length;
             break;
         }
-        double kc = ceil(p.k);
-        int kI = to_index<SEM>(kc);
-        int jI = to_index<SEM>(floor(p.j)), iI = to_index<SEM>(floor(p.i));
-        double kF = kc - p.k, jF = p.j - jI, iF = p.i - iI;
+        double kF, jF, iF;
+        const int kI = ceil_index<SEM>(p.k, kF);
+        const int jI = floor_index<SEM>(p.j, jF), iI = floor_index<SEM>(p.i, iF);
         if (!valid_cell(jI, iI, eta, xi)) {
             p.health = -1;
             lazy = false;
@@ -430,11 +445,11 @@ __device__ int move_particle(const wacomm_b200_config &cfg, const IntervalParams
             break;
         }
         steps++;
-        double alpha = length == 0 ? 0 : (elapsed + 0.5 * stepDt) / length;
-        double alphaStart = length == 0 ? 0 : elapsed / length;
+        double alpha = length == 0 ? 0 : quotient(elapsed + 0.5 * stepDt, length, rLength);
+        double alphaStart = length == 0 ? 0 : quotient(elapsed, length, rLength);
         double hh;
         float zz;
-        surface_at<ARITH>(V, jI, iI, jF, iF, alpha, hh, zz);
+        surface_at(V, jI, iI, jF, iF, alpha, hh, zz);
         double hc = hh + zz;
         if (hc <= cfg.shoreLimit && cfg.horizontalClosure == CLOSURE_KILL) {
             p.health = -1;
@@ -447,9 +462,10 @@ __device__ int move_particle(const wacomm_b200_config &cfg, const IntervalParams
         const int kM = mem_level(kI, sW);
         float uu, vv;
         double ww;
-        advective_velocity<SEM, ARITH>(cfg, P, V, p, kM, kF, jI, jF, iI, iF,
+        keep_column(kM, jI, iI);
+        advective_velocity<SEM, DRIFT>(cfg, P, V, kept, p, kF, jI, jF, iI, iF,
                                        midpoint ? alphaStart : alpha, elapsed, physicalTime,
-                                       stepDt, keys, uu, vv, ww, err);
+                                       stepDt, uu, vv, ww, err);
         double dxleap = dir * uu * stepDt, dyleap = dir * vv * stepDt;
         double dzleap = dir * (cfg.sv + ww) * stepDt;
         double rx = 0, ry = 0, rz = 0;
@@ -462,9 +478,9 @@ __device__ int move_particle(const wacomm_b200_config &cfg, const IntervalParams
         }
         if (diffuse) {
             // Stochastic leap (Particle.cpp:518-533; kernel.cu:269-276)
-            double aa = akt_at<SEM, ARITH>(V, kM, kF, jI, jF, iI, iF, alpha);
-            double sigmaDepth = cfg.sigma * (1 - p.k / kLower);
-            double scale = sqrt(stepDt / cfg.dti);
+            double aa = akt_at<SEM>(V, kM, kF, jI, jF, iI, iF, alpha);
+            double sigmaDepth = cfg.sigma * (1 - quotient(p.k, kLower, P.invKLower));
+            double scale = stepDt == cfg.dti ? 1.0 : sqrt(stepDt / cfg.dti);
             double n0, n1, n2;
             if (P.rng == WACOMM_B200_RNG_PHILOX) {
                 float f0, f1, f2;
@@ -484,57 +500,55 @@ __device__ int move_particle(const wacomm_b200_config &cfg, const IntervalParams
         }
         double xleap = dxleap + rx, yleap = dyleap + ry, zleap = dzleap + rz;
 
-        double2 md = V.cell_metric(jI, iI);
-        double xdist = md.x, ydist = md.y;
+        const CellMetric md = V.cell_metric(jI, iI);
+        const double xdist = md.x, ydist = md.y;
         double zdist = hc * V.depth_interval(kM);
 
         if (midpoint) {
             // Explicit midpoint (Particle.cpp:585-641; kernel.cu:281-317)
             double kHalf = dir * (cfg.sv + ww) * 0.5 * stepDt;
             if (fabs(kHalf) > zdist) kHalf = sign_of(zdist, kHalf);
-            double iMid = p.i + dir * uu * 0.5 * stepDt / xdist;
-            double jMid = p.j + dir * vv * 0.5 * stepDt / ydist;
+            double iMid = p.i + quotient(dir * uu * 0.5 * stepDt, xdist, md.rx);
+            double jMid = p.j + quotient(dir * vv * 0.5 * stepDt, ydist, md.ry);
             double kMid = SEM == SEM_HOST ? smin(0.0, smax(kLower, p.k + kHalf / zdist))
                                           : fmin(0.0, fmax(kLower, p.k + kHalf / zdist));
-            int iMI = to_index<SEM>(floor(iMid)), jMI = to_index<SEM>(floor(jMid));
+            // the midpoint, or the start where the midpoint has no water: one evaluation for both
+            double iMF, jMF, kMF = kF;
+            int iMI = floor_index<SEM>(iMid, iMF), jMI = floor_index<SEM>(jMid, jMF), kMI = kM;
             bool midValid = valid_cell(jMI, iMI, eta, xi);
-            double hcMid = 0, iMF = 0, jMF = 0;
+            double hcMid = 0;
             if (midValid) {
-                iMF = iMid - iMI;
-                jMF = jMid - jMI;
-                if (SEM == SEM_HOST && ARITH == ARITH_REF) {
+                if (SEM == SEM_HOST) {
                     hcMid = hc_mid_host(V, jMI, iMI, jMF, iMF, alpha);
                 } else {
                     double hm;
                     float zm;
-                    surface_at<ARITH>(V, jMI, iMI, jMF, iMF, alpha, hm, zm);
+                    surface_at(V, jMI, iMI, jMF, iMF, alpha, hm, zm);
                     hcMid = hm + zm;
                 }
                 midValid = hcMid > cfg.shoreLimit && hcMid > 0;
             }
-            double detX, detY, detZ;
             if (midValid) {
-                double kmc = ceil(kMid);
-                int kMI = mem_level(to_index<SEM>(kmc), sW);
-                double kMF = kmc - kMid;
-                float um, vm;
-                double wm;
-                advective_velocity<SEM, ARITH>(cfg, P, V, p, kMI, kMF, jMI, jMF, iMI, iMF, alpha,
-                                               elapsed, physicalTime, stepDt, keys, um, vm, wm,
-                                               err);
-                double2 mm = V.cell_metric(jMI, iMI);
-                double zdistMid = hcMid * V.depth_interval(kMI);
-                detX = dir * um * stepDt * xdist / mm.x;
-                detY = dir * vm * stepDt * ydist / mm.y;
-                detZ = dir * (cfg.sv + wm) * stepDt * zdist / zdistMid;
+                kMI = mem_level(ceil_index<SEM>(kMid, kMF), sW);
             } else {
-                float ue, ve;
-                double we;
-                advective_velocity<SEM, ARITH>(cfg, P, V, p, kM, kF, jI, jF, iI, iF, alpha, elapsed,
-                                               physicalTime, stepDt, keys, ue, ve, we, err);
-                detX = dir * ue * stepDt;
-                detY = dir * ve * stepDt;
-                detZ = dir * (cfg.sv + we) * stepDt;
+                iMI = iI;
+                jMI = jI;
+                iMF = iF;
+                jMF = jF;
+            }
+            float um, vm;
+            double wm;
+            keep_column(kMI, jMI, iMI);
+            advective_velocity<SEM, DRIFT>(cfg, P, V, kept, p, kMF, jMI, jMF, iMI, iMF, alpha,
+                                           elapsed, physicalTime, stepDt, um, vm, wm, err);
+            double detX = dir * um * stepDt, detY = dir * vm * stepDt;
+            double detZ = dir * (cfg.sv + wm) * stepDt;
+            if (midValid) {
+                const CellMetric mm = V.cell_metric(jMI, iMI);
+                double zdistMid = hcMid * V.depth_interval(kMI);
+                detX = quotient(detX * xdist, mm.x, mm.rx);
+                detY = quotient(detY * ydist, mm.y, mm.ry);
+                detZ = detZ * zdist / zdistMid;
             }
             if (SEM == SEM_HOST) {
                 xleap = detX + rx;
@@ -549,19 +563,19 @@ __device__ int move_particle(const wacomm_b200_config &cfg, const IntervalParams
 
         // Vertical cap, candidate position and vertical closures (Particle.cpp:644-704)
         if (fabs(zleap) > zdist) zleap = sign_of(zdist, zleap);
-        double jdet = p.j + yleap / ydist;
-        double idet = p.i + xleap / xdist;
+        double jdet = p.j + quotient(yleap, ydist, md.ry);
+        double idet = p.i + quotient(xleap, xdist, md.rx);
         double kdet = p.k + zleap / zdist;
         if (kdet > 0.) close_upper(cfg, kdet, p.health, lazy);
         if (kdet < kLower) close_lower(cfg, kLower, kdet, p.health, lazy);
 
         // Horizontal landing and closures (Particle.cpp:706-791; kernel.cu:331-353)
-        int jdetI = to_index<SEM>(floor(jdet)), idetI = to_index<SEM>(floor(idet));
+        double jdetF, idetF;
+        const int jdetI = floor_index<SEM>(jdet, jdetF), idetI = floor_index<SEM>(idet, idetF);
         if (valid_cell(jdetI, idetI, eta, xi)) {
-            double idetF = idet - idetI, jdetF = jdet - jdetI;
             double hd;
             float zd;
-            surface_at<ARITH>(V, jdetI, idetI, jdetF, idetF, alpha, hd, zd);
+            surface_at(V, jdetI, idetI, jdetF, idetF, alpha, hd, zd);
             double hcdet = hd + zd;
             if (hcdet <= cfg.shoreLimit) {
                 if (cfg.horizontalClosure == CLOSURE_CONSTRAINT) {

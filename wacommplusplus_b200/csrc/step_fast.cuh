@@ -24,7 +24,7 @@ struct FastExtras {
 
 template <int STORE>
 struct FastView {
-    PackedView<STORE> V;   // node layout: wind/Stokes pair, lon/lat (drift model)
+    PackedView V;          // grid, wind/Stokes pair, lon/lat (drift model)
     CellView<STORE> C;     // cell-column layout: velocity stencil and surface
     FastExtras X;
 };
@@ -132,11 +132,6 @@ template <int SEM>
 __device__ __forceinline__ bool on_axis(double x, double nodes) {
     return SEM == SEM_HOST ? (x >= 0.0 && x < nodes - 1.0) : !(x < 0.0) && !(x >= nodes - 1.0);
 }
-
-// Adding 1.5 2^52 rounds |x| < 2^31 to an integer in the direction of the add and leaves it in the
-// sum's low word: floor and ceil with their index in two FP64 adds, no conversion on the
-// quarter-rate unit.
-constexpr double INTEGER_SHIFT = 6755399441055744.0;
 
 // Cell index and fraction of a position on the axis (on_axis).
 template <int SEM>
@@ -269,7 +264,7 @@ template <int SEM, int STORE, int VARIANT>
 __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalParams &P,
                                   const FastView<STORE> &F, const Draws draws, ParticleState &p,
                                   double &elapsed, int *err) {
-    const PackedView<STORE> &V = F.V;
+    const PackedView &V = F.V;
     const CellView<STORE> &C = F.C;
     const int eta = V.g.eta, xi = V.g.xi, sW = V.g.sW;
     const double kLower = P.kLower, length = P.length;

@@ -11,107 +11,67 @@ static inline int grid_for(size_t n, int block, int maxBlocks = 148 * 16) {
     return blocks < 1 ? 1 : (int)blocks;
 }
 
-size_t node_record_bytes(int storage) {
-    return storage == STORE_F32 ? sizeof(NodeRecord<STORE_F32>) : sizeof(NodeRecord<STORE_F16>);
-}
+size_t node_record_bytes() { return sizeof(NodeRecord); }
+size_t surf_record_bytes() { return sizeof(SurfRecord); }
 
 // ------------------------------------------------------------------ forcing pair packing
 
-template <int STORE>
-__device__ __forceinline__ void store_node(NodeRecord<STORE> *dst, float w0, float a0, float u0,
-                                           float v0, float w1, float a1, float u1, float v1);
-template <>
-__device__ __forceinline__ void store_node<STORE_F32>(NodeRecord<STORE_F32> *dst, float w0,
-                                                      float a0, float u0, float v0, float w1,
-                                                      float a1, float u1, float v1) {
-    dst->t0 = make_float4(w0, a0, u0, v0);
-    dst->t1 = make_float4(w1, a1, u1, v1);
-}
-template <>
-__device__ __forceinline__ void store_node<STORE_F16>(NodeRecord<STORE_F16> *dst, float w0,
-                                                      float a0, float u0, float v0, float w1,
-                                                      float a1, float u1, float v1) {
-    NodeRecord<STORE_F16> r;
-    r.wa0 = __floats2half2_rn(w0, a0);
-    r.uv0 = __floats2half2_rn(u0, v0);
-    r.wa1 = __floats2half2_rn(w1, a1);
-    r.uv1 = __floats2half2_rn(u1, v1);
-    *dst = r;
-}
-template <>
-__device__ __forceinline__ void store_node<STORE_BF16>(NodeRecord<STORE_BF16> *dst, float w0,
-                                                       float a0, float u0, float v0, float w1,
-                                                       float a1, float u1, float v1) {
-    NodeRecord<STORE_BF16> r;
-    r.wa0 = __floats2bfloat162_rn(w0, a0);
-    r.uv0 = __floats2bfloat162_rn(u0, v0);
-    r.wa1 = __floats2bfloat162_rn(w1, a1);
-    r.uv1 = __floats2bfloat162_rn(u1, v1);
-    *dst = r;
-}
-
-// Interleaves records t0 and t1 into node records {w(L), akt(L), u(L-1), v(L-1)} x 2.
-template <int STORE>
+// Interleaves records t0 and t1 into the node records of the reference arithmetic.
 __global__ void pack_nodes_kernel(int eta, int xi, int sW, FrameDevice f0, FrameDevice f1,
-                                  NodeRecord<STORE> *nodes) {
+                                  NodeRecord *nodes) {
     size_t plane = (size_t)eta * xi, total = plane * sW;
     for (size_t n = blockIdx.x * (size_t)blockDim.x + threadIdx.x; n < total;
          n += (size_t)gridDim.x * blockDim.x) {
-        size_t L = n / plane, cell = n - L * plane;
-        float w0 = f0.w[n], a0 = f0.akt[n], w1 = f1.w[n], a1 = f1.akt[n];
-        float u0 = 0, v0 = 0, u1 = 0, v1 = 0;
-        if (L > 0) {
-            size_t r = (L - 1) * plane + cell;
-            u0 = f0.u[r];
-            v0 = f0.v[r];
-            u1 = f1.u[r];
-            v1 = f1.v[r];
+        NodeRecord r;
+        r.w = make_double2(f0.w[n], f1.w[n]);
+        r.akt = make_double2(f0.akt[n], f1.akt[n]);
+        r.u = r.v = make_double2(0.0, 0.0);
+        if (n >= plane) {  // W level 0 has no rho level below it
+            r.u = make_double2(f0.u[n - plane], f1.u[n - plane]);
+            r.v = make_double2(f0.v[n - plane], f1.v[n - plane]);
         }
-        store_node<STORE>(nodes + n, w0, a0, u0, v0, w1, a1, u1, v1);
+        nodes[n] = r;
     }
 }
 
 __global__ void pack_surface_kernel(int eta, int xi, FrameDevice f0, FrameDevice f1,
-                                    const double *h, SurfPair *surf, EnvPair *env) {
+                                    const double *h, SurfRecord *surf) {
+    size_t plane = (size_t)eta * xi;
+    for (size_t n = blockIdx.x * (size_t)blockDim.x + threadIdx.x; n < plane;
+         n += (size_t)gridDim.x * blockDim.x)
+        surf[n] = SurfRecord{h[n], f0.zeta[n], f1.zeta[n], 0.0};
+}
+
+__global__ void pack_environment_kernel(int eta, int xi, FrameDevice f0, FrameDevice f1,
+                                        EnvPair *env) {
     size_t plane = (size_t)eta * xi;
     for (size_t n = blockIdx.x * (size_t)blockDim.x + threadIdx.x; n < plane;
          n += (size_t)gridDim.x * blockDim.x) {
-        surf[n] = SurfPair{h[n], f0.zeta[n], f1.zeta[n]};
-        if (env) {
-            EnvPair e;
-            e.wu0 = f0.windU ? f0.windU[n] : 0.f;
-            e.wv0 = f0.windV ? f0.windV[n] : 0.f;
-            e.su0 = f0.stokesU ? f0.stokesU[n] : 0.f;
-            e.sv0 = f0.stokesV ? f0.stokesV[n] : 0.f;
-            e.wu1 = f1.windU ? f1.windU[n] : 0.f;
-            e.wv1 = f1.windV ? f1.windV[n] : 0.f;
-            e.su1 = f1.stokesU ? f1.stokesU[n] : 0.f;
-            e.sv1 = f1.stokesV ? f1.stokesV[n] : 0.f;
-            env[n] = e;
-        }
+        EnvPair e;
+        e.wu0 = f0.windU ? f0.windU[n] : 0.f;
+        e.wv0 = f0.windV ? f0.windV[n] : 0.f;
+        e.su0 = f0.stokesU ? f0.stokesU[n] : 0.f;
+        e.sv0 = f0.stokesV ? f0.stokesV[n] : 0.f;
+        e.wu1 = f1.windU ? f1.windU[n] : 0.f;
+        e.wv1 = f1.windV ? f1.windV[n] : 0.f;
+        e.su1 = f1.stokesU ? f1.stokesU[n] : 0.f;
+        e.sv1 = f1.stokesV ? f1.stokesV[n] : 0.f;
+        env[n] = e;
     }
 }
 
-cudaError_t pack_pair(int storage, int eta, int xi, int sW, const FrameDevice &f0,
-                      const FrameDevice &f1, const double *h, void *nodes, SurfPair *surf,
-                      EnvPair *env, cudaStream_t stream) {
-    size_t total = (size_t)eta * xi * sW;
-    int blocks = grid_for(total, 256);
-    switch (storage) {
-        case STORE_F16:
-            pack_nodes_kernel<STORE_F16><<<blocks, 256, 0, stream>>>(
-                eta, xi, sW, f0, f1, static_cast<NodeRecord<STORE_F16> *>(nodes));
-            break;
-        case STORE_BF16:
-            pack_nodes_kernel<STORE_BF16><<<blocks, 256, 0, stream>>>(
-                eta, xi, sW, f0, f1, static_cast<NodeRecord<STORE_BF16> *>(nodes));
-            break;
-        default:
-            pack_nodes_kernel<STORE_F32><<<blocks, 256, 0, stream>>>(
-                eta, xi, sW, f0, f1, static_cast<NodeRecord<STORE_F32> *>(nodes));
-    }
-    pack_surface_kernel<<<grid_for((size_t)eta * xi, 256), 256, 0, stream>>>(eta, xi, f0, f1, h,
-                                                                           surf, env);
+cudaError_t pack_pair(int eta, int xi, int sW, const FrameDevice &f0, const FrameDevice &f1,
+                      const double *h, NodeRecord *nodes, SurfRecord *surf, cudaStream_t stream) {
+    const size_t plane = (size_t)eta * xi;
+    pack_nodes_kernel<<<grid_for(plane * sW, 256), 256, 0, stream>>>(eta, xi, sW, f0, f1, nodes);
+    pack_surface_kernel<<<grid_for(plane, 256), 256, 0, stream>>>(eta, xi, f0, f1, h, surf);
+    return cudaGetLastError();
+}
+
+cudaError_t pack_environment(int eta, int xi, const FrameDevice &f0, const FrameDevice &f1,
+                             EnvPair *env, cudaStream_t stream) {
+    pack_environment_kernel<<<grid_for((size_t)eta * xi, 256), 256, 0, stream>>>(eta, xi, f0, f1,
+                                                                               env);
     return cudaGetLastError();
 }
 
@@ -250,13 +210,13 @@ cudaError_t pack_cells(int storage, int eta, int xi, int sW, const FrameDevice &
 // with the cross difference dropped (Particle.cpp:548-574); device rules: full haversine between
 // the nodes (kernel.cu:145-149,278-279). Cells on the last row/column are never valid.
 __global__ void metric_kernel(int semantics, int eta, int xi, const double *lat,
-                              const double *lon, double2 *metric, float2 *invMetric) {
+                              const double *lon, CellMetric *metric, float2 *invMetric) {
     size_t plane = (size_t)eta * xi;
     for (size_t n = blockIdx.x * (size_t)blockDim.x + threadIdx.x; n < plane;
          n += (size_t)gridDim.x * blockDim.x) {
         int j = (int)(n / xi), i = (int)(n - (size_t)j * xi);
         if (j + 1 >= eta || i + 1 >= xi) {
-            metric[n] = make_double2(0.0, 0.0);
+            metric[n] = CellMetric{0.0, 0.0, 0.0, 0.0};
             invMetric[n] = make_float2(0.f, 0.f);
             continue;
         }
@@ -280,13 +240,13 @@ __global__ void metric_kernel(int semantics, int eta, int xi, const double *lat,
             value = sin(.5 * dLat) * sin(.5 * dLat) + sin(.5 * dLon) * sin(.5 * dLon) * cos(latE) * cos(lat0);
             xdist = 2.0 * atan2(sqrt(value), sqrt(1.0 - value)) * 6371000.0;
         }
-        metric[n] = make_double2(xdist, ydist);
+        metric[n] = CellMetric{xdist, ydist, 1.0 / xdist, 1.0 / ydist};
         invMetric[n] = make_float2((float)(1.0 / xdist), (float)(1.0 / ydist));
     }
 }
 
 cudaError_t build_metric(int semantics, int eta, int xi, const double *lonRad,
-                         const double *latRad, double2 *metric, float2 *invMetric,
+                         const double *latRad, CellMetric *metric, float2 *invMetric,
                          cudaStream_t stream) {
     metric_kernel<<<grid_for((size_t)eta * xi, 256), 256, 0, stream>>>(semantics, eta, xi, latRad,
                                                                       lonRad, metric, invMetric);

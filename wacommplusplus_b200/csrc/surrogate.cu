@@ -118,7 +118,7 @@ struct CellArgs {
     long long nCL;  // (eta-1) * (xi-1) * (sW-1) cell-levels, index ((j*(xi-1)) + i)*(sW-1) + kI+sW-2
     const float *u0, *v0, *w0, *u1, *v1, *w1, *z0, *z1;
     const double *h, *depthIntervals;
-    const double2 *metric;
+    const CellMetric *metric;
     const uint8_t *weights;
     __half *z;             // [nCL][256]
     CellCorners *corners;  // [nCL]
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(128, 1) surrogate_cell_kernel(const CellArgs a
                 c.zeta[1][q] = a.z1[corner[q]];
                 c.h[q] = (float)a.h[corner[q]];
             }
-            const double2 m = a.metric[c00];
+            const CellMetric m = a.metric[c00];
             c.invXdist = 1.0 / m.x;
             c.invYdist = 1.0 / m.y;
             c.depth = a.depthIntervals[kI + a.sW - 2];
@@ -1379,7 +1379,7 @@ long long surrogate_cell_levels(int eta, int xi, int sW) {
 
 cudaError_t surrogate_cells(int eta, int xi, int sW, int sRho, const FrameDevice &f0,
                             const FrameDevice &f1, const double *h, const double *depthIntervals,
-                            const double2 *metric, const uint8_t *weights, __half *z, void *corners,
+                            const CellMetric *metric, const uint8_t *weights, __half *z, void *corners,
                             int *err, int smCount, cudaStream_t stream) {
     CellArgs a;
     a.eta = eta;

@@ -1,12 +1,14 @@
 // Forcing views: how the step reads the bracketing forcing pair.
 //
-// PackedView is the engine layout. For each interval the two bracketing records are
-// interleaved into one node record per (W level L, j, i):
-//     {w(L), akt(L), u(L-1), v(L-1)} of record t0, then the same of record t1
-// so that one particle's trilinear stencil (4 corners x 2 levels) is 8 records, each one
-// 32-byte sector (16 bytes in half precision), instead of 48 scalar gathers from four fields
-// and two frames. Surface data sit in a 16-byte {h, zeta(t0), zeta(t1)} record per node, the
-// optional wind/Stokes pair in a 32-byte record, the cell metric in a per-cell table.
+// PackedView is the engine layout of the reference arithmetic. For each interval the two bracketing
+// records are interleaved into one node record per (W level L, j, i), as doubles:
+//     {w(L), akt(L), u(L-1), v(L-1)} of record t0 and t1
+// so that one particle's trilinear stencil (4 corners x 2 levels) is 8 records instead of 48 scalar
+// gathers from four fields and two frames, and the step's FP64 products read their operands without
+// a float-to-double conversion each (a quarter-rate instruction; there are more of them in a substep
+// than anything else on that unit). Surface data sit in a {h, zeta(t0), zeta(t1)} record per node,
+// the optional wind/Stokes pair in a 32-byte record, the cell metric in a per-cell table. The FP32
+// step shares the wind/Stokes pair and the grid.
 //
 // RawView reads the reference device layout directly (kernel.cu:63-80): it serves the drop-in
 // launcher, whose caller owns separate field arrays for the whole window.
@@ -20,119 +22,74 @@
 
 namespace wb {
 
-// Time pair of one node: upper record (u, v, w, akt) and lower record (w, akt).
-struct NodeUp {
-    float u0, u1, v0, v1, w0, w1, a0, a1;
-};
-struct NodeLo {
-    float w0, w1, a0, a1;
-};
+template <class T>
 struct SurfPair {
     double h;
-    float z0, z1;
+    T z0, z1;
 };
 struct EnvPair {
     float wu0, wv0, su0, sv0, wu1, wv1, su1, sv1;
 };
 
-// Record of the packed pair in each storage precision.
-template <int STORE>
-struct NodeRecord;
-template <>
-struct NodeRecord<STORE_F32> {
-    float4 t0, t1;  // (w, akt, u, v) of records t0 and t1
+// Records of the packed pair: {t0, t1} per field.
+struct alignas(16) NodeRecord {
+    double2 w, akt, u, v;
 };
-template <>
-struct alignas(16) NodeRecord<STORE_F16> {
-    __half2 wa0, uv0, wa1, uv1;
-};
-template <>
-struct alignas(16) NodeRecord<STORE_BF16> {
-    __nv_bfloat162 wa0, uv0, wa1, uv1;
+struct alignas(16) SurfRecord {
+    double h, z0, z1, unused;
 };
 
-template <int STORE>
-__device__ __forceinline__ void load_node(const NodeRecord<STORE> *p, float &w0, float &a0,
-                                          float &u0, float &v0, float &w1, float &a1, float &u1,
-                                          float &v1);
+// Cell sizes in metres along i and j and their correctly rounded reciprocals.
+struct CellMetric {
+    double x, y, rx, ry;
+};
 
-template <>
-__device__ __forceinline__ void load_node<STORE_F32>(const NodeRecord<STORE_F32> *p, float &w0,
-                                                     float &a0, float &u0, float &v0, float &w1,
-                                                     float &a1, float &u1, float &v1) {
-    float4 x = __ldg(&p->t0), y = __ldg(&p->t1);
-    w0 = x.x; a0 = x.y; u0 = x.z; v0 = x.w;
-    w1 = y.x; a1 = y.y; u1 = y.z; v1 = y.w;
-}
-
-template <>
-__device__ __forceinline__ void load_node<STORE_F16>(const NodeRecord<STORE_F16> *p, float &w0,
-                                                     float &a0, float &u0, float &v0, float &w1,
-                                                     float &a1, float &u1, float &v1) {
-    uint4 raw = __ldg(reinterpret_cast<const uint4 *>(p));
-    float2 wa0 = __half22float2(*reinterpret_cast<__half2 *>(&raw.x));
-    float2 uv0 = __half22float2(*reinterpret_cast<__half2 *>(&raw.y));
-    float2 wa1 = __half22float2(*reinterpret_cast<__half2 *>(&raw.z));
-    float2 uv1 = __half22float2(*reinterpret_cast<__half2 *>(&raw.w));
-    w0 = wa0.x; a0 = wa0.y; u0 = uv0.x; v0 = uv0.y;
-    w1 = wa1.x; a1 = wa1.y; u1 = uv1.x; v1 = uv1.y;
-}
-
-template <>
-__device__ __forceinline__ void load_node<STORE_BF16>(const NodeRecord<STORE_BF16> *p, float &w0,
-                                                      float &a0, float &u0, float &v0, float &w1,
-                                                      float &a1, float &u1, float &v1) {
-    uint4 raw = __ldg(reinterpret_cast<const uint4 *>(p));
-    float2 wa0 = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162 *>(&raw.x));
-    float2 uv0 = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162 *>(&raw.y));
-    float2 wa1 = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162 *>(&raw.z));
-    float2 uv1 = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162 *>(&raw.w));
-    w0 = wa0.x; a0 = wa0.y; u0 = uv0.x; v0 = uv0.y;
-    w1 = wa1.x; a1 = wa1.y; u1 = uv1.x; v1 = uv1.y;
-}
+// The velocity stencil of one cell and level: u, v (rho level kI) and w (W levels kI and kI-1) at the
+// corners (j,i), (j+1,i), (j+1,i+1), (j,i+1) of records t0 and t1.
+struct RefStencil {
+    double2 u[4], v[4], wUp[4], wLo[4];  // {t0, t1}
+};
 
 // Grid-level constants every view shares.
 struct GridShape {
     int eta, xi, sW, sRho;
 };
 
-template <int STORE>
 struct PackedView {
     GridShape g;
-    const NodeRecord<STORE> *nodes;  // [sW][eta][xi]
-    const SurfPair *surf;            // [eta][xi]
+    const NodeRecord *nodes;         // [sW][eta][xi]
+    const SurfRecord *surf;          // [eta][xi]
     const EnvPair *env;              // [eta][xi] or null
     bool hasWindU, hasWindV, hasStokes;
     const double *lonRad, *latRad;   // [eta][xi]
     const double *depthIntervals;    // [sW-1]
-    const double2 *metric;           // [eta][xi] {xdist, ydist} of cell (j, i)
+    const CellMetric *metric;        // [eta][xi]
 
     __device__ __forceinline__ size_t node_index(int L, int j, int i) const {
         return ((size_t)L * (size_t)g.eta + (size_t)j) * (size_t)g.xi + (size_t)i;
     }
-    // Upper node of logical level kI (W level kI with rho level kI), kI in [-sW+2, 0].
-    __device__ __forceinline__ NodeUp up(int kI, int j, int i) const {
-        NodeUp n;
-        load_node<STORE>(nodes + node_index(kI + g.sW - 1, j, i), n.w0, n.a0, n.u0, n.v0, n.w1,
-                         n.a1, n.u1, n.v1);
-        return n;
+    // Stencil of logical level kI, kI in [-sW+2, 0].
+    __device__ __forceinline__ void stencil(int kI, int j, int i, RefStencil &s) const {
+        const NodeRecord *up = nodes + node_index(kI + g.sW - 1, j, i);
+        const NodeRecord *lo = nodes + node_index(kI + g.sW - 2, j, i);
+        const int corner[4] = {0, g.xi, g.xi + 1, 1};
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            s.u[c] = __ldg(&up[corner[c]].u);
+            s.v[c] = __ldg(&up[corner[c]].v);
+            s.wUp[c] = __ldg(&up[corner[c]].w);
+            s.wLo[c] = __ldg(&lo[corner[c]].w);
+        }
     }
-    // Lower node (W level kI-1).
-    __device__ __forceinline__ NodeLo lo(int kI, int j, int i) const {
-        float w0, a0, u0, v0, w1, a1, u1, v1;
-        load_node<STORE>(nodes + node_index(kI + g.sW - 2, j, i), w0, a0, u0, v0, w1, a1, u1, v1);
-        return NodeLo{w0, w1, a0, a1};
+    // Diffusivity {t0, t1} at W level kI.
+    __device__ __forceinline__ double2 akt(int kI, int j, int i) const {
+        return __ldg(&nodes[node_index(kI + g.sW - 1, j, i)].akt);
     }
-    __device__ __forceinline__ SurfPair surface(int j, int i) const {
-        double2 raw = __ldg(reinterpret_cast<const double2 *>(surf) + (size_t)j * g.xi + i);
-        SurfPair s;
-        s.h = raw.x;
-        float2 z = *reinterpret_cast<float2 *>(&raw.y);
-        s.z0 = z.x;
-        s.z1 = z.y;
-        return s;
+    __device__ __forceinline__ SurfPair<double> surface(int j, int i) const {
+        const double2 *s = reinterpret_cast<const double2 *>(surf + ((size_t)j * g.xi + i));
+        const double2 hz = __ldg(s), z = __ldg(s + 1);
+        return SurfPair<double>{hz.x, hz.y, z.x};
     }
-    __device__ __forceinline__ double h(int j, int i) const { return surface(j, i).h; }
     __device__ __forceinline__ EnvPair environment(int j, int i) const {
         const float4 *p = reinterpret_cast<const float4 *>(env + (size_t)j * g.xi + i);
         float4 a = __ldg(p), b = __ldg(p + 1);
@@ -143,8 +100,10 @@ struct PackedView {
     __device__ __forceinline__ double depth_interval(int kI) const {
         return __ldg(depthIntervals + (kI + g.sW - 2));
     }
-    __device__ __forceinline__ double2 cell_metric(int j, int i) const {
-        return __ldg(metric + (size_t)j * g.xi + i);
+    __device__ __forceinline__ CellMetric cell_metric(int j, int i) const {
+        const double2 *m = reinterpret_cast<const double2 *>(metric + ((size_t)j * g.xi + i));
+        const double2 size = __ldg(m), reciprocal = __ldg(m + 1);
+        return CellMetric{size.x, size.y, reciprocal.x, reciprocal.y};
     }
 };
 
@@ -284,7 +243,7 @@ struct CellView {
 struct RawView {
     GridShape g;
     int t0, t1;
-    const float *zeta, *u, *v, *w, *akt;
+    const float *zeta, *u, *v, *w, *aktField;
     const float *windU, *windV, *stokesU, *stokesV;
     const double *hField, *lonRad, *latRad, *depthIntervals;
     bool hasWindU, hasWindV, hasStokes;
@@ -296,29 +255,29 @@ struct RawView {
     __device__ __forceinline__ size_t i4(int t, int storageLevel, int levels, int j, int i) const {
         return (((size_t)t * levels + storageLevel) * g.eta + j) * g.xi + i;
     }
-    __device__ __forceinline__ NodeUp up(int kI, int j, int i) const {
-        int Lw = kI + g.sW - 1, Lr = kI + g.sRho - 1;
-        NodeUp n;
-        n.u0 = __ldg(u + i4(t0, Lr, g.sRho, j, i));
-        n.u1 = __ldg(u + i4(t1, Lr, g.sRho, j, i));
-        n.v0 = __ldg(v + i4(t0, Lr, g.sRho, j, i));
-        n.v1 = __ldg(v + i4(t1, Lr, g.sRho, j, i));
-        n.w0 = __ldg(w + i4(t0, Lw, g.sW, j, i));
-        n.w1 = __ldg(w + i4(t1, Lw, g.sW, j, i));
-        n.a0 = __ldg(akt + i4(t0, Lw, g.sW, j, i));
-        n.a1 = __ldg(akt + i4(t1, Lw, g.sW, j, i));
-        return n;
+    __device__ __forceinline__ double2 pair(const float *field, int level, int levels, int j,
+                                            int i) const {
+        return make_double2(__ldg(field + i4(t0, level, levels, j, i)),
+                            __ldg(field + i4(t1, level, levels, j, i)));
     }
-    __device__ __forceinline__ NodeLo lo(int kI, int j, int i) const {
-        int Lw = kI + g.sW - 2;
-        return NodeLo{__ldg(w + i4(t0, Lw, g.sW, j, i)), __ldg(w + i4(t1, Lw, g.sW, j, i)),
-                      __ldg(akt + i4(t0, Lw, g.sW, j, i)), __ldg(akt + i4(t1, Lw, g.sW, j, i))};
+    __device__ __forceinline__ void stencil(int kI, int j, int i, RefStencil &s) const {
+        const int Lr = kI + g.sRho - 1, Lw = kI + g.sW - 1;
+        const int dj[4] = {0, 1, 1, 0}, di[4] = {0, 0, 1, 1};
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            s.u[c] = pair(u, Lr, g.sRho, j + dj[c], i + di[c]);
+            s.v[c] = pair(v, Lr, g.sRho, j + dj[c], i + di[c]);
+            s.wUp[c] = pair(w, Lw, g.sW, j + dj[c], i + di[c]);
+            s.wLo[c] = pair(w, Lw - 1, g.sW, j + dj[c], i + di[c]);
+        }
     }
-    __device__ __forceinline__ SurfPair surface(int j, int i) const {
-        return SurfPair{__ldg(hField + (size_t)j * g.xi + i), __ldg(zeta + i3(t0, j, i)),
+    __device__ __forceinline__ double2 akt(int kI, int j, int i) const {
+        return pair(aktField, kI + g.sW - 1, g.sW, j, i);
+    }
+    __device__ __forceinline__ SurfPair<float> surface(int j, int i) const {
+        return SurfPair<float>{__ldg(hField + (size_t)j * g.xi + i), __ldg(zeta + i3(t0, j, i)),
                         __ldg(zeta + i3(t1, j, i))};
     }
-    __device__ __forceinline__ double h(int j, int i) const { return __ldg(hField + (size_t)j * g.xi + i); }
     __device__ __forceinline__ EnvPair environment(int j, int i) const {
         EnvPair e{0, 0, 0, 0, 0, 0, 0, 0};
         if (hasWindU) { e.wu0 = __ldg(windU + i3(t0, j, i)); e.wu1 = __ldg(windU + i3(t1, j, i)); }
@@ -335,7 +294,7 @@ struct RawView {
         return __ldg(depthIntervals + (kI + g.sW - 2));
     }
     // Full haversine between the nodes of the cell's edges (kernel.cu:145-149,278-279).
-    __device__ __forceinline__ double2 cell_metric(int j, int i) const {
+    __device__ __forceinline__ CellMetric cell_metric(int j, int i) const {
         double lat0 = lat(j, i), lon0 = lon(j, i);
         double latN = lat(j + 1, i), lonN = lon(j + 1, i);
         double latE = lat(j, i + 1), lonE = lon(j, i + 1);
@@ -346,7 +305,7 @@ struct RawView {
         dLon = lonE - lon0;
         value = sin(.5 * dLat) * sin(.5 * dLat) + sin(.5 * dLon) * sin(.5 * dLon) * cos(latE) * cos(lat0);
         double xdist = 2.0 * atan2(sqrt(value), sqrt(1.0 - value)) * 6371000.0;
-        return make_double2(xdist, ydist);
+        return CellMetric{xdist, ydist, 1.0 / xdist, 1.0 / ydist};
     }
 };
 
