@@ -11,7 +11,7 @@ import os
 import numpy as np
 import pytest
 
-from helpers import DEG, load_move_cases, max_abs_diff
+from helpers import DEG, load_move_cases, max_abs_diff, records_equal
 from oracle import bindings as ob
 from wacommplusplus_b200 import _native, synthetic as syn
 from wacommplusplus_b200.types import PARTICLE_DTYPE, default_config, make_particles
@@ -197,3 +197,36 @@ def test_engine_abi_from_a_cpp_program(cuda_device, tmp_path):
     run = subprocess.run([exe], capture_output=True, text=True, timeout=300)
     assert run.returncode == 0, (run.returncode, run.stdout[-2000:], run.stderr[-2000:])
     assert "2000 records, 0 off" in run.stdout
+
+
+def same_records_packed_and_read(win, n, environment, direction):
+    """The allocation-free launcher always reads the window; the other packs the pair."""
+    if environment:
+        shape = (win.eta, win.xi)
+        win.windU10, win.windV10 = syn.vector_series(shape, win.T, 8.0, 3, 3.0)
+        win.stokesU, win.stokesV = syn.vector_series(shape, win.T, 0.1, 4, 3.0)
+    rng = np.random.default_rng(n)
+    p = syn.uniform_particles(n, win.eta, win.xi, seed=n, time=win.times[0])
+    p["k"] = rng.uniform(-3.5, 0.0, n)
+    p["driftObjectType"], p["driftSide"] = rng.integers(0, 23, n), 1
+    cfg = default_config(random=True, driftModel=int(environment), hasWind=environment,
+                         trackingDirection=direction, backwardDiffusion=1)
+    got = call_dropin(cfg, p, win, 1)
+    noalloc = call_dropin(cfg, p, win, 1, _native.lib().wacomm_b200_cuda_move_particle_noalloc)
+    assert records_equal(got, noalloc)
+
+
+# with and without the kept stencil (37,888 records)
+@pytest.mark.parametrize("n", [1, 593, 37888, 40000])
+@pytest.mark.parametrize("environment", [False, True])
+@pytest.mark.parametrize("direction", [1, -1])
+def test_packed_pair_and_window_reads_agree(cuda_device, n, environment, direction):
+    win = syn.RealisticForcing(eta=9, xi=8, s_rho=4, n_frames=3, seed=8, land_fraction=0.1,
+                               water_border=1).window()
+    same_records_packed_and_read(win, n, environment, direction)
+
+
+# 1,310,720 nodes: packed from 40,960 records on
+@pytest.mark.parametrize("n", [40959, 40960])
+def test_pair_packed_by_records_on_a_large_grid(cuda_device, n):
+    same_records_packed_and_read(syn.config1_window(n_frames=2, eta=512, xi=512, s_rho=4), n, False, 1)

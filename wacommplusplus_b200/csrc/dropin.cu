@@ -1,29 +1,66 @@
 // Drop-in replacement of the reference GPU launcher (kernel.cu:370-382): same arguments, same
 // in-place update of the caller's particle_data records, device rules and reference arithmetic.
-// The work is ordered by horizontal cell first (key per record, histogram, exclusive scan,
-// scatter into a work order), so that the threads of a warp gather the same forcing cells; each
-// record still moves independently, so the order changes no result. The ordering scratch is
-// stream-ordered (cudaMallocAsync/cudaFreeAsync on the caller's stream, served from the device's
-// memory pool without a device-wide synchronization); if it cannot be had, the records are moved
-// in caller order. Compiled with -fmad=false.
+// The work is ordered by horizontal cell (and level) first -- key per record, histogram, exclusive
+// scan, scatter into a work order -- so that the threads of a warp gather the same forcing cells, and
+// the forcing pair and the cell metric are packed once per call (views.cuh) instead of being gathered
+// from the window and recomputed by haversines in every substep; each record still moves
+// independently, so neither changes a result. The scratch is stream-ordered
+// (cudaMallocAsync/cudaFreeAsync on the caller's stream, served from the device's memory pool without
+// a device-wide synchronization); what cannot be had is done without: the records are moved in
+// caller order, or read the window directly. Compiled with -fmad=false.
 #include "engine.h"
 #include "move_kernels.cuh"
 #include "wacomm_b200_kernel.h"
 
 namespace wb {
 
-// Cell key of each record (last bin for records outside the interpolation cells) and the
-// warp-aggregated histogram of the keys.
+// Sort key of each record (its cell, and its level where `levels` > 1; the last bin for records
+// outside the interpolation cells) and the warp-aggregated histogram of the keys.
 __global__ void dropin_key_kernel(const wacomm_b200_particle *particles, int n, int eta, int xi,
-                                  uint32_t *keys, uint32_t *hist) {
+                                  int levels, uint32_t *keys, uint32_t *hist) {
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-        double fj = floor(particles[p].j), fi = floor(particles[p].i);
-        uint32_t key = (fj >= 0.0 && fi >= 0.0 && fj < (double)(eta - 1) && fi < (double)(xi - 1))
-                           ? (uint32_t)((int)fj * xi + (int)fi)
-                           : (uint32_t)((size_t)eta * xi);
+        const double fj = floor(particles[p].j), fi = floor(particles[p].i);
+        uint32_t key = (uint32_t)((size_t)eta * xi * levels);
+        if (fj >= 0.0 && fi >= 0.0 && fj < (double)(eta - 1) && fi < (double)(xi - 1)) {
+            const double down = fmin(fmax(-ceil(particles[p].k), 0.0), (double)(levels - 1));
+            key = (uint32_t)((int)fj * xi + (int)fi) * (uint32_t)levels + (uint32_t)down;
+        }
         keys[p] = key;
         unsigned peers = __match_any_sync(__activemask(), key);
         if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(hist + key, (uint32_t)__popc(peers));
+    }
+}
+
+// The call's forcing pair and cell metric in the engine's layout. Like the move, each thread reads
+// the tracking direction from the device copy of the config; one thread per (level, node).
+__global__ void dropin_pack_kernel(const wacomm_b200_config *__restrict__ config, int timeIndex,
+                                   int oceanTime, RawView V, NodeRecord *nodes, SurfRecord *surf,
+                                   CellMetric *metric, EnvPair *env) {
+    const int next = timeIndex + config->trackingDirection;
+    V.t0 = timeIndex;
+    V.t1 = next >= 0 && next < oceanTime ? next : timeIndex;
+    const int eta = V.g.eta, xi = V.g.xi;
+    const size_t plane = (size_t)eta * xi, total = plane * V.g.sW;
+    for (size_t n = blockIdx.x * (size_t)blockDim.x + threadIdx.x; n < total;
+         n += (size_t)gridDim.x * blockDim.x) {
+        const int L = (int)(n / plane);
+        const size_t c = n - (size_t)L * plane;
+        const int j = (int)(c / xi), i = (int)(c - (size_t)j * xi);
+        NodeRecord r;
+        r.w = V.pair(V.w, L, V.g.sW, j, i);
+        r.akt = V.pair(V.aktField, L, V.g.sW, j, i);
+        r.u = r.v = make_double2(0.0, 0.0);
+        if (L > 0) {
+            r.u = V.pair(V.u, L - 1, V.g.sRho, j, i);
+            r.v = V.pair(V.v, L - 1, V.g.sRho, j, i);
+        }
+        nodes[n] = r;
+        if (L == 0) {
+            const SurfPair<float> s = V.surface(j, i);
+            surf[c] = SurfRecord{s.h, s.z0, s.z1, 0.0};
+            if (j + 1 < eta && i + 1 < xi) metric[c] = V.cell_metric(j, i);
+            if (env) env[c] = V.environment(j, i);
+        }
     }
 }
 
@@ -41,24 +78,42 @@ __global__ void dropin_scatter_kernel(const uint32_t *keys, int n, uint32_t *cur
     }
 }
 
-// One thread per record, taken in the work order (null: caller order). Like the reference
+__device__ __forceinline__ RawView at_interval(RawView V, const IntervalParams &P) {
+    V.t0 = P.t0;
+    V.t1 = P.t1;
+    return V;
+}
+__device__ __forceinline__ const PackedView &at_interval(const PackedView &V, const IntervalParams &) {
+    return V;
+}
+
+// One work item per record, taken in the work order (null: caller order). Like the reference
 // kernel, each thread derives the interval from the device copies of config and times
 // (kernel.cu:158-171); the particle is read from and written back to the caller's AoS array.
-__global__ void __launch_bounds__(256) dropin_move_kernel(
+// 524,287 records on 128 x 128 x 10, 120 substeps: 13.7 ms with the window read and two haversines
+// per substep (244 registers), 3.9 ms with the packed pair (3.4 times faster per call); bound as move_soa_kernel is.
+template <bool KEEP, class View>
+__global__ void __launch_bounds__(128, KEEP ? 1 : 4) dropin_move_kernel(
     const wacomm_b200_config *__restrict__ config, wacomm_b200_particle *particles,
     const uint32_t *__restrict__ order, int timeIndex, int oceanTime,
-    const double *__restrict__ times, RawView V, int count) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count) return;
+    const double *__restrict__ times, const View V, const MoveLaunch L) {
+    const unsigned t = launch_item(L, blockIdx.x * (blockDim.x >> 5) * L.lanes, L.count);
+    if (t >= (unsigned)L.count) return;
     const wacomm_b200_config &cfg = *config;
     IntervalParams P;
     make_interval(cfg, times, oceanTime, timeIndex, V.g.sW, SEM_DEVICE, P);
     if (P.skip) return;
-    RawView view = V;
-    view.t0 = P.t0;
-    view.t1 = P.t1;
+    const View &view = at_interval(V, P);
     uint32_t idx = order ? order[t] : (uint32_t)t;
-    wacomm_b200_particle rec = particles[idx];
+    // the whole record as words, so that its padding bytes go back as they came
+    union {
+        unsigned long long words[8];
+        wacomm_b200_particle rec;
+    } held;
+    static_assert(sizeof(wacomm_b200_particle) == 64, "record layout");
+    unsigned long long *words = reinterpret_cast<unsigned long long *>(particles + idx);
+    for (int w = 0; w < 8; w++) held.words[w] = words[w];
+    wacomm_b200_particle &rec = held.rec;
     ParticleState p;
     p.id = rec.id;
     p.k = rec.k;
@@ -70,14 +125,80 @@ __global__ void __launch_bounds__(256) dropin_move_kernel(
     p.type = rec.driftObjectType;
     p.side = rec.driftSide;
     double elapsed = P.elapsed0;
-    move_particle<SEM_DEVICE, true, false>(cfg, P, view, p, elapsed, nullptr);
+    if (cfg.driftModel == 1)
+        move_particle<SEM_DEVICE, true, KEEP>(cfg, P, view, p, elapsed, nullptr);
+    else
+        move_particle<SEM_DEVICE, false, KEEP>(cfg, P, view, p, elapsed, nullptr);
     rec.k = p.k;
     rec.j = p.j;
     rec.i = p.i;
     rec.health = p.health;
     rec.age = p.age;
     rec.driftSide = (int8_t)p.side;
-    particles[idx] = rec;
+    for (int w = 1; w < 8; w++)
+        if (w != 6) words[w] = held.words[w];  // all but the id and the release time
+}
+
+template <class View>
+cudaError_t launch_dropin(const wacomm_b200_config *config, wacomm_b200_particle *particles,
+                          const uint32_t *order, int timeIndex, int oceanTime, const double *times,
+                          const View &V, int count, cudaStream_t stream) {
+    MoveLaunch L{};
+    L.count = count;
+    int threads;
+    spread_launch(count, 128, L.lanes, threads);
+    const int items = threads / 32 * L.lanes, blocks = (count + items - 1) / items;
+    if (count <= KEEP_RECORDS)
+        dropin_move_kernel<true><<<blocks, threads, 0, stream>>>(config, particles, order, timeIndex,
+                                                                 oceanTime, times, V, L);
+    else
+        dropin_move_kernel<false><<<blocks, threads, 0, stream>>>(config, particles, order, timeIndex,
+                                                                  oceanTime, times, V, L);
+    return cudaGetLastError();
+}
+
+// The pair is packed up to this many nodes, and beyond while there are at most so many per record:
+// packing a node costs about 0.02 ns, reading the window and evaluating haversines instead above 10 ns
+// per record and, in the latency of its substep chain, at least 0.4 ms per call (2,000 records on
+// 180,224 nodes: 1.1 ms). It bounds the scratch to 64 MB or 2 KB per record.
+constexpr size_t PACK_NODES = (size_t)1 << 20, PACK_NODES_PER_RECORD = 32;
+
+// The call's packed pair in `scratch` (null: no scratch, read the window), stream-ordered.
+cudaError_t pack_window(const wacomm_b200_config *config, int timeIndex, int oceanTime,
+                        const RawView &V, int count, PackedView &out, void **scratch,
+                        cudaStream_t stream) {
+    const size_t plane = (size_t)V.g.eta * V.g.xi, nodes = plane * V.g.sW;
+    const bool env = V.hasWindU || V.hasWindV || V.hasStokes;
+    *scratch = nullptr;
+    if (V.g.eta < 2 || V.g.xi < 2 ||
+        (nodes > PACK_NODES && nodes > PACK_NODES_PER_RECORD * (size_t)count))
+        return cudaSuccess;
+    const size_t bytes = nodes * sizeof(NodeRecord) +
+                         plane * (sizeof(SurfRecord) + sizeof(CellMetric) + (env ? sizeof(EnvPair) : 0));
+    if (cudaMallocAsync(scratch, bytes, stream) != cudaSuccess) {
+        *scratch = nullptr;
+        (void)cudaGetLastError();  // no pool memory: read the window
+        return cudaSuccess;
+    }
+    NodeRecord *n = static_cast<NodeRecord *>(*scratch);
+    SurfRecord *s = reinterpret_cast<SurfRecord *>(n + nodes);
+    CellMetric *m = reinterpret_cast<CellMetric *>(s + plane);
+    EnvPair *e = env ? reinterpret_cast<EnvPair *>(m + plane) : nullptr;
+    size_t blocks = (nodes + 255) / 256;
+    if (blocks > 148 * 16) blocks = 148 * 16;
+    dropin_pack_kernel<<<(unsigned)blocks, 256, 0, stream>>>(config, timeIndex, oceanTime, V, n, s, m, e);
+    out.g = V.g;
+    out.nodes = n;
+    out.surf = s;
+    out.env = e;
+    out.hasWindU = V.hasWindU;
+    out.hasWindV = V.hasWindV;
+    out.hasStokes = V.hasStokes;
+    out.lonRad = V.lonRad;
+    out.latRad = V.latRad;
+    out.depthIntervals = V.depthIntervals;
+    out.metric = m;
+    return cudaGetLastError();
 }
 
 int dropin_move(const wacomm_b200_config *config, wacomm_b200_particle *particles, int timeIndex,
@@ -109,7 +230,8 @@ int dropin_move(const wacomm_b200_config *config, wacomm_b200_particle *particle
     uint32_t *order = nullptr, *scratch = nullptr;
     if (eta >= 2 && xi >= 2) {
         // keys[count] | order[count] | histogram[bins] | offsets[bins + 1] | scan partials
-        size_t bins = (size_t)eta * xi + 1;
+        const int levels = sort_bins(eta, xi, sRho, (size_t)count).levels;
+        size_t bins = (size_t)eta * xi * levels + 1;
         size_t words = 2 * (size_t)count + 2 * bins + 1 + scan_temp_words(bins);
         if (cudaMallocAsync((void **)&scratch, words * sizeof(uint32_t), stream) == cudaSuccess) {
             uint32_t *keys = scratch, *hist = scratch + 2 * (size_t)count;
@@ -118,8 +240,8 @@ int dropin_move(const wacomm_b200_config *config, wacomm_b200_particle *particle
             if (blocks > 148 * 16) blocks = 148 * 16;
             cudaError_t e = cudaMemsetAsync(hist, 0, bins * sizeof(uint32_t), stream);
             if (e == cudaSuccess) {
-                dropin_key_kernel<<<blocks, 256, 0, stream>>>(particles, count, eta, xi, keys,
-                                                              hist);
+                dropin_key_kernel<<<blocks, 256, 0, stream>>>(particles, count, eta, xi, levels,
+                                                              keys, hist);
                 e = exclusive_scan(hist, offsets, bins, offsets + bins, partials, stream);
             }
             if (e == cudaSuccess) {
@@ -134,15 +256,19 @@ int dropin_move(const wacomm_b200_config *config, wacomm_b200_particle *particle
             (void)cudaGetLastError();  // no pool memory: caller order
         }
     }
-    const int threads = 128;
-    int blocks = count / threads + ((count % threads) == 0 ? 0 : 1);
-    dropin_move_kernel<<<blocks, threads, 0, stream>>>(config, particles, order, timeIndex,
-                                                       oceanTime, times, V, count);
-    cudaError_t e = cudaGetLastError();
-    if (scratch) {
-        cudaError_t f = cudaFreeAsync(scratch, stream);
-        if (e == cudaSuccess) e = f;
-    }
+    PackedView packed;
+    void *pair = nullptr;
+    cudaError_t e = pack_window(config, timeIndex, oceanTime, V, count, packed, &pair, stream);
+    if (e == cudaSuccess)
+        e = pair ? launch_dropin(config, particles, order, timeIndex, oceanTime, times, packed, count,
+                                 stream)
+                 : launch_dropin(config, particles, order, timeIndex, oceanTime, times, V, count,
+                                 stream);
+    for (void *held : {pair, (void *)scratch})
+        if (held) {
+            cudaError_t f = cudaFreeAsync(held, stream);
+            if (e == cudaSuccess) e = f;
+        }
     return (int)e;
 }
 
