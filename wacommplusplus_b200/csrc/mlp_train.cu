@@ -1,17 +1,24 @@
 // Training of the advection surrogate's MLP (388 -> 256 -> 256 -> 256 -> 3, GELU tanh form, the
 // outputs multiplied by the stencil's uniformity gate) with the library's own kernels: the forward
 // pass, the mean-squared loss against the targets, the backward pass through all four layers and
-// an Adam update. The GEMMs of layers 1-3 (forward, input gradients) and every weight gradient
-// run on the tcgen05 tensor cores with BF16 operands and FP32 accumulation; the three-output layer
-// 4 forward and input gradient, the loss, GELU derivatives, bias sums and Adam are FP32 on the
-// CUDA cores. The parameters use the flat layout of
+// an Adam update. The GEMMs of layers 1-3 (forward, input gradients) and their weight gradients run
+// on the tcgen05 tensor cores with BF16 operands and FP32 accumulation; the three-output layer 4, the
+// loss, GELU and its derivative, bias sums and Adam are FP32 on the CUDA cores (layer 4's weight
+// gradient from BF16-rounded operands). The parameters use the flat layout of
 // wacomm_b200_set_surrogate (w1 [256][388], b1, w2 [256][256], b2, w3, b3, w4 [3][256], b4), so
 // trained weights go to the inference kernels unchanged.
 //
-// The tensor-core GEMM covers the three products of a layer: the forward Z = X W^T (bias and GELU
-// fused into its epilogue), the input gradient dX = dZ W, and the weight gradient dW = dZ^T X (the
-// reduction over the batch, split over the SMs and summed in a fixed order). A tiled FP32 GEMM on
-// the CUDA cores serves layer 4, whose three outputs are too few for a tensor-core tile.
+// A step is four launches:
+//   pack_weights_kernel  W1, W2, W3 as BF16 in the tensor cores' shared-memory layout (umma.cuh);
+//   tile_kernel          128 rows of the batch through the forward pass, the loss and the input
+//                        gradients of every layer, with the activations in shared memory and the
+//                        accumulators in tensor memory; leaves the BF16 operands of the weight
+//                        gradients (X, H1, H2, dZ1, dZ2, dZ3) as shared-memory images and the
+//                        tile's bias, layer-4 and loss sums;
+//   weight_grad_kernel   dW = dZ^T X of layers 1-3 over a range of tiles: the images as they are,
+//                        read along the other index (MN-major operands);
+//   finish_kernel        the partial sums in a fixed order, the gradients, Adam.
+// Every sum runs in a fixed order: a step is reproducible bit for bit.
 #include <cmath>
 
 #include <cuda_bf16.h>
@@ -29,547 +36,694 @@ constexpr size_t OFF_TW1 = 0, OFF_TB1 = OFF_TW1 + (size_t)T_HID * T_IN, OFF_TW2 
                  OFF_TB3 = OFF_TW3 + (size_t)T_HID * T_HID, OFF_TW4 = OFF_TB3 + T_HID,
                  OFF_TB4 = OFF_TW4 + (size_t)T_OUT * T_HID, T_PARAMS = OFF_TB4 + T_OUT;
 
-__device__ __forceinline__ float gelu_exact_tanh(float x, float *derivative) {
-    const float c0 = 0.7978845608028654f, c1 = 0.044715f;
-    const float t = tanhf(c0 * (x + c1 * x * x * x));
-    if (derivative) *derivative = 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * c0 * (1.f + 3.f * c1 * x * x);
-    return 0.5f * x * (1.f + t);
+constexpr int TROWS = 128;                     // rows of a tile
+constexpr int X_KB = (T_IN + 63) / 64;         // 7 K-blocks of the input (388 -> 448, zero-padded)
+constexpr int H_KB = T_HID / 64;               // 4 K-blocks of a hidden layer
+constexpr uint32_t A_BLOCK = TROWS * 128;      // 16 KB: 128 rows x 64 BF16
+constexpr uint32_t W_BLOCK = T_HID * 128;      // 32 KB: 256 rows x 64 BF16
+constexpr uint32_t X_IMAGE = X_KB * A_BLOCK, H_IMAGE = H_KB * A_BLOCK;
+constexpr int W_BLOCKS = X_KB + 2 * H_KB;      // W1, W2, W3
+constexpr int W2_BLOCK = X_KB, W3_BLOCK = X_KB + H_KB;
+
+// Sums of a tile over its rows: db1, db2, db3, dW4 [3][256], db4 [3], loss.
+constexpr int SUM_DB = 0, SUM_DW4 = 3 * T_HID, SUM_DB4 = 6 * T_HID, SUM_LOSS = SUM_DB4 + T_OUT,
+              SUMS = SUM_LOSS + 1;
+
+// Weight-gradient units: 128 rows (hidden units of dZ) by up to 256 columns each: W3, W2 (two row
+// halves), W1 (two row halves by two column parts).
+constexpr int UNITS = 8;
+constexpr int X_TAIL = T_IN - T_HID;           // columns of W1's second part
+constexpr int X_TAIL_N = (X_TAIL + 15) / 16 * 16;
+constexpr int MAX_SPLITS = 148 / UNITS;        // ranges of tiles: about one block per SM
+
+// The work buffer: an error word (at its start), then, from the next 1024-byte boundary, the packed
+// weights, the images and sums per tile and the partial weight gradients.
+struct Work {
+    int *err;
+    uint8_t *weights;                    // [W_BLOCKS][W_BLOCK]
+    uint8_t *X, *H1, *H2, *dZ1, *dZ2, *dZ3;  // [tiles] images
+    float4 *slope1;                      // [tiles][T_HID / 4][TROWS]: GELU'(Z1)
+    float *sums;                         // [tiles][SUMS]
+    float4 *partial;                     // [UNITS][splits][T_HID / 4][TROWS]
+};
+
+size_t tiles_of(int batch) { return ((size_t)batch + TROWS - 1) / TROWS; }
+
+size_t work_bytes(size_t tiles, Work *w, uint8_t *base) {
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        uint8_t *p = base ? base + at : nullptr;
+        at += (bytes + 1023) / 1024 * 1024;
+        return p;
+    };
+    Work f{};
+    f.weights = take((size_t)W_BLOCKS * W_BLOCK);
+    f.X = take(tiles * X_IMAGE);
+    f.H1 = take(tiles * H_IMAGE);
+    f.H2 = take(tiles * H_IMAGE);
+    f.dZ1 = take(tiles * H_IMAGE);
+    f.dZ2 = take(tiles * H_IMAGE);
+    f.dZ3 = take(tiles * H_IMAGE);
+    f.slope1 = reinterpret_cast<float4 *>(take(tiles * TROWS * T_HID * sizeof(float)));
+    f.sums = reinterpret_cast<float *>(take(tiles * SUMS * sizeof(float)));
+    f.partial = reinterpret_cast<float4 *>(
+        take((size_t)UNITS * MAX_SPLITS * TROWS * T_HID * sizeof(float)));
+    if (w) *w = f;
+    return at;
 }
 
-// ------------------------------------------------------------------ tcgen05 GEMM (layers 1-3)
-//
-// C[M][N] = sum_k a(m, k) b(n, k), a(m, k) = A[m sam + k sak], b(n, k) = B[n sbn + k sbk]: BF16
-// operands, FP32 accumulation in tensor memory. A block owns a 128-row by up to 256-column tile
-// and a range of K; its 256 threads read the FP32 operands (coalesced along whichever index is
-// contiguous in memory, so transposed operands need no separate pass), round them to BF16 and
-// write them into shared memory in the K-major 128-byte-swizzle layout of umma.cuh, two K-blocks
-// of 64 in flight: while one thread issues the four MMAs of block kb, the others fill block kb+1.
-// Epilogues: 0 store; 1 add bias[n]; 2 add bias[n], store Z and GELU(Z); 3 store the block's
-// partial sum of its K range to partial[blockIdx.z] (reduced afterwards in a fixed order, so the
-// weight gradients are reproducible bit for bit).
-constexpr int UM = 128, UK = 64, UN = 256, UTHREADS = 256;
-constexpr uint32_t UA_BYTES = UM * 128, UB_BYTES = UN * 128;
-constexpr size_t USMEM = 2 * ((size_t)UA_BYTES + UB_BYTES) + 1024;
-
-struct UmmaGemm {
-    int M, N, K, kPerSplit;
-    const float *A;
-    long long sam, sak;
-    const float *B;
-    long long sbn, sbk;
-    const float *bias;
-    float *C, *H, *partial;
-    int ldc;
-    int *err;
-};
+__device__ __forceinline__ float gelu_exact_tanh(float x, float &derivative) {
+    const float c0 = 0.7978845608028654f, c1 = 0.044715f;
+    const float t = tanhf(c0 * (x + c1 * x * x * x));
+    derivative = 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * c0 * (1.f + 3.f * c1 * x * x);
+    return 0.5f * x * (1.f + t);
+}
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
     __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<uint32_t *>(&v);
 }
 
-__device__ __forceinline__ uint4 pack8(float4 a, float4 b) {
-    return make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y),
-                      pack_bf16x2(b.z, b.w));
+__device__ __forceinline__ uint4 pack8(const float *v) {
+    return make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
+                      pack_bf16x2(v[6], v[7]));
 }
 
-// One rows x 64 operand block, a(r, k) = src[r sRow + k sK], rounded to BF16 into its swizzled
-// shared-memory image; rows at or past `rows` and k at or past kEnd read as zero. Three ways to
-// read it, chosen per block: with k contiguous, each item is a row's 16-byte chunk of 8 k values
-// (two float4 loads); with rows contiguous, each item is 4 rows x 8 k values (eight float4 loads
-// along the rows, written as four chunks); otherwise scalar pairs. Every thread issues its loads
-// before its stores, so many loads are in flight.
-__device__ __forceinline__ void stage_block(uint8_t *dst, int rowsInBlock, const float *src,
-                                            long long sRow, long long sK, int row0, int rows,
-                                            int k0, int kEnd, int tid) {
-    const bool aligned = (((uintptr_t)src) & 15) == 0 && k0 + UK <= kEnd;
-    if (aligned && sK == 1 && (sRow & 3) == 0) {
-        const int items = rowsInBlock * 8;
-        for (int base = 0; base < items; base += 4 * UTHREADS) {
-            float4 v[4][2];
+__device__ __forceinline__ float bf16_rounded(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+
+// Sum over the warp's 32 lanes of each of v[0..31]: lane l returns the sum of v[l] (v is used up).
+// Each exchange halves the values a lane still carries: 31 shuffles for 32 sums.
+__device__ __forceinline__ float lane_sums(float (&v)[32], int lane) {
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int it = base + u * UTHREADS + tid, r = it >> 3, c = it & 7;
-                v[u][0] = v[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (it < items && row0 + r < rows) {
-                    const float4 *q =
-                        reinterpret_cast<const float4 *>(src + (long long)(row0 + r) * sRow + k0 + c * 8);
-                    v[u][0] = __ldg(q);
-                    v[u][1] = __ldg(q + 1);
-                }
-            }
+    for (int s = 16; s >= 1; s >>= 1) {
+        const bool upper = lane & s;
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int it = base + u * UTHREADS + tid;
-                if (it < items)
-                    *reinterpret_cast<uint4 *>(dst + umma::sw128_offset(it >> 3, (it & 7) * 8)) =
-                        pack8(v[u][0], v[u][1]);
-            }
+        for (int q = 0; q < s; q++) {
+            const float send = upper ? v[q] : v[q + s], keep = upper ? v[q + s] : v[q];
+            v[q] = keep + __shfl_xor_sync(0xffffffffu, send, s);
         }
-        return;
     }
-    if (aligned && sRow == 1 && (sK & 3) == 0 && (row0 & 3) == 0) {
-        const int groups = (rowsInBlock + 3) / 4, items = groups * 8;
-        for (int it = tid; it < items; it += UTHREADS) {
-            const int g = it % groups, c = it / groups, r0 = 4 * g, gr0 = row0 + r0;
-            float4 v[8];
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-                const float *col = src + (long long)(k0 + c * 8 + q) * sK;
-                if (gr0 + 3 < rows) {
-                    v[q] = __ldg(reinterpret_cast<const float4 *>(col + gr0));
-                } else {
-                    v[q].x = gr0 < rows ? __ldg(col + gr0) : 0.f;
-                    v[q].y = gr0 + 1 < rows ? __ldg(col + gr0 + 1) : 0.f;
-                    v[q].z = gr0 + 2 < rows ? __ldg(col + gr0 + 2) : 0.f;
-                    v[q].w = 0.f;
-                }
-            }
-            *reinterpret_cast<uint4 *>(dst + umma::sw128_offset(r0 + 0, c * 8)) =
-                pack8(make_float4(v[0].x, v[1].x, v[2].x, v[3].x), make_float4(v[4].x, v[5].x, v[6].x, v[7].x));
-            *reinterpret_cast<uint4 *>(dst + umma::sw128_offset(r0 + 1, c * 8)) =
-                pack8(make_float4(v[0].y, v[1].y, v[2].y, v[3].y), make_float4(v[4].y, v[5].y, v[6].y, v[7].y));
-            *reinterpret_cast<uint4 *>(dst + umma::sw128_offset(r0 + 2, c * 8)) =
-                pack8(make_float4(v[0].z, v[1].z, v[2].z, v[3].z), make_float4(v[4].z, v[5].z, v[6].z, v[7].z));
-            *reinterpret_cast<uint4 *>(dst + umma::sw128_offset(r0 + 3, c * 8)) =
-                pack8(make_float4(v[0].w, v[1].w, v[2].w, v[3].w), make_float4(v[4].w, v[5].w, v[6].w, v[7].w));
-        }
-        return;
-    }
-    const int pairs = rowsInBlock * (UK / 2);
-    for (int e = tid; e < pairs; e += UTHREADS) {
-        int r, kp;
-        if (sK == 1) {
-            r = e / (UK / 2);
-            kp = e % (UK / 2);
-        } else {
-            kp = e / rowsInBlock;
-            r = e % rowsInBlock;
-        }
-        const int gr = row0 + r, gk = k0 + 2 * kp;
-        float v0 = 0.f, v1 = 0.f;
-        if (gr < rows) {
-            const float *p = src + (long long)gr * sRow;
-            if (gk < kEnd) v0 = __ldg(p + (long long)gk * sK);
-            if (gk + 1 < kEnd) v1 = __ldg(p + (long long)(gk + 1) * sK);
-        }
-        *reinterpret_cast<uint32_t *>(dst + umma::sw128_offset(r, 2 * kp)) = pack_bf16x2(v0, v1);
-    }
+    return v[0];
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(UTHREADS, 1) umma_gemm_kernel(const UmmaGemm g) {
+// ------------------------------------------------------------------ packed weights
+
+// One thread per 16-byte chunk (8 k of one output unit) of the K-block images.
+__global__ void pack_weights_kernel(const float *params, uint8_t *weights, int *err) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *err = 0;
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= W_BLOCKS * T_HID * 8) return;
+    const int chunk = e & 7, n = (e >> 3) % T_HID, block = (e >> 3) / T_HID;
+    const int layer = block < W2_BLOCK ? 0 : block < W3_BLOCK ? 1 : 2;
+    const int first = layer == 0 ? 0 : layer == 1 ? W2_BLOCK : W3_BLOCK;
+    const int width = layer == 0 ? T_IN : T_HID;
+    const float *row = params + (layer == 0 ? OFF_TW1 : layer == 1 ? OFF_TW2 : OFF_TW3) + (size_t)n * width;
+    const int k = (block - first) * 64 + chunk * 8;
+    float v[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) v[q] = k + q < width ? row[k + q] : 0.f;
+    *reinterpret_cast<uint4 *>(weights + (size_t)block * W_BLOCK + umma::sw128_offset(n, chunk * 8)) = pack8(v);
+}
+
+// ------------------------------------------------------------------ forward and input gradients
+
+struct TileArgs {
+    const float *stencil, *particle, *gate, *target, *params;
+    int batch, tiles;
+    Work w;
+};
+
+constexpr int ROW_WARPS = 16, ROW_THREADS = ROW_WARPS * 32;
+constexpr int PRODUCER_WARP = ROW_WARPS, MMA_WARP = ROW_WARPS + 1, TILE_THREADS = ROW_THREADS + 64;
+constexpr int TRING = 3;
+constexpr size_t TILE_SMEM = X_IMAGE + TRING * (size_t)W_BLOCK + 1024;
+// The MMA jobs of a tile: layers 1, 2, 3 forward, then the gradients of H2 and H1.
+constexpr int JOBS = 5;
+__device__ __forceinline__ int job_blocks(int job) { return job == 0 ? X_KB : H_KB; }
+
+// Bulk copy shared -> global, and the issuing thread's wait until its copies have read their source.
+__device__ __forceinline__ void bulk_s2g(void *dst, const void *src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+                 "r"(umma::smem_u32(src)), "r"(bytes)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_wait_read() {
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
+// A tile of 128 rows per turn, 16 row warps (TMEM lane quarter w % 4, columns 64 (w / 4) ..), one
+// warp streaming weights through a ring of bulk copies, one issuing the MMAs. Operand buffer (112 KB):
+// X, then H1, H2, dZ3, dZ2, dZ1 in turn, each copied out as it stands for the weight gradients.
+// Tensor memory: columns 0-255 hold the accumulators of layers 1 and 3 and of both gradients,
+// columns 256-511 that of layer 2, replaced by GELU'(Z2). The GELU and its derivative (a precise
+// tanhf per unit and layer) bound it; the tensor cores and the weight stream work underneath.
+__global__ void __launch_bounds__(TILE_THREADS, 1) tile_kernel(const TileArgs a) {
     using namespace umma;
     extern __shared__ uint8_t dynSmem[];
     uint8_t *sA = reinterpret_cast<uint8_t *>(((uintptr_t)dynSmem + 1023) & ~(uintptr_t)1023);
-    uint8_t *sB = sA + 2 * UA_BYTES;
-    __shared__ __align__(8) uint64_t freed[2], accFull;
+    uint8_t *ring = sA + X_IMAGE;
+    __shared__ __align__(8) uint64_t full[TRING], empty[TRING], aFull, accFull;
     __shared__ uint32_t tmemSlot;
-    __shared__ int abortFlag;
+    __shared__ int abortFlag, stopFlag;
+    __shared__ float bias[3][T_HID], w4[T_OUT][T_HID], outSum[TROWS][T_OUT];
+    __shared__ float colSum[4][T_HID];  // one sum over 32 rows per lane quarter
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.y * UM, n0 = blockIdx.x * UN;
-    const int nLeft = g.N - n0;
-    const int nTile = nLeft >= UN ? UN : ((nLeft + 15) / 16) * 16;  // MMA N: multiple of 16
-    const int kBegin = blockIdx.z * g.kPerSplit;
-    const int kEnd = min(g.K, kBegin + g.kPerSplit);
-    const int nkb = kEnd > kBegin ? (kEnd - kBegin + UK - 1) / UK : 0;
     if (tid == 0) {
-        mbar_init(&freed[0], 1);
-        mbar_init(&freed[1], 1);
+        for (int s = 0; s < TRING; s++) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(&aFull, ROW_WARPS);
         mbar_init(&accFull, 1);
         abortFlag = 0;
         fence_barrier_init();
     }
-    if (warp == 0) tmem_alloc(&tmemSlot, UN);
+    for (int c = tid; c < T_HID; c += TILE_THREADS) {
+        bias[0][c] = a.params[OFF_TB1 + c];
+        bias[1][c] = a.params[OFF_TB2 + c];
+        bias[2][c] = a.params[OFF_TB3 + c];
+        for (int o = 0; o < T_OUT; o++) w4[o][c] = a.params[OFF_TW4 + (size_t)o * T_HID + c];
+    }
+    if (warp == MMA_WARP) tmem_alloc(&tmemSlot, 512);
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = tmemSlot;
-    const uint32_t idesc = idesc_bf16(UM, nTile);
-    bool ok = true;
-    for (int kb = 0; kb < nkb && ok; kb++) {
-        const int s = kb & 1;
-        // the MMAs of block kb-2 read this stage: wait for their commit
-        if (kb >= 2) ok = mbar_wait(&freed[s], (uint32_t)(((kb >> 1) + 1) & 1), &abortFlag);
+    const int mine = blockIdx.x < a.tiles ? (a.tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+
+    if (warp == PRODUCER_WARP) {
+        if (lane == 0) {
+            int issued[TRING];
+            for (int s = 0; s < TRING; s++) issued[s] = -1;
+            uint32_t g = 0;
+            bool ok = true;
+            for (int t = 0; t < mine && ok; t++)
+                for (int job = 0; job < JOBS && ok; job++)
+                    for (int kb = 0; kb < job_blocks(job) && ok; kb++, g++) {
+                        const uint32_t s = g % TRING, n = g / TRING;
+                        if (!(ok = mbar_wait(&empty[s], (n & 1) ^ 1, &abortFlag))) break;
+                        mbar_expect_tx(&full[s], W_BLOCK);
+                        uint8_t *dst = ring + s * W_BLOCK;
+                        if (job < 3) {
+                            const int block = (job == 0 ? 0 : job == 1 ? W2_BLOCK : W3_BLOCK) + kb;
+                            bulk_g2s(dst, a.w.weights + (size_t)block * W_BLOCK, W_BLOCK, &full[s]);
+                        } else {
+                            // output units 64 kb .. of every K-block: [4][64 rows][128 bytes]
+                            const int first = job == 3 ? W3_BLOCK : W2_BLOCK;
+                            for (int b = 0; b < H_KB; b++)
+                                bulk_g2s(dst + b * (W_BLOCK / 4),
+                                         a.w.weights + (size_t)(first + b) * W_BLOCK + kb * (W_BLOCK / 4),
+                                         W_BLOCK / 4, &full[s]);
+                        }
+                        issued[s] = (int)n;
+                    }
+            for (int s = 0; s < TRING; s++)  // copies still in flight land before the block exits
+                if (issued[s] >= 0) mbar_wait_bounded(&full[s], (uint32_t)issued[s] & 1);
+        }
         __syncwarp();
-        if (!ok) break;
-        const int k0 = kBegin + kb * UK;
-        stage_block(sA + s * UA_BYTES, UM, g.A, g.sam, g.sak, m0, g.M, k0, kEnd, tid);
-        stage_block(sB + s * UB_BYTES, nTile, g.B, g.sbn, g.sbk, n0, g.N, k0, kEnd, tid);
-        fence_async_shared();
-        fence_before_sync();
-        __syncthreads();
-        fence_after_sync();
-        if (abortFlag) {
-            ok = false;
-            break;
-        }
-        if (tid == 0) {
+    } else if (warp == MMA_WARP) {
+        if (lane == 0) {
+            uint32_t g = 0, jobs = 0;
+            bool ok = true;
+            for (int t = 0; t < mine && ok; t++)
+                for (int job = 0; job < JOBS && ok; job++, jobs++) {
+                    if (!(ok = mbar_wait(&aFull, jobs & 1, &abortFlag))) break;
+                    fence_after_sync();
+                    const uint32_t d = tmem + (job == 1 ? T_HID : 0);
+                    const uint32_t idesc = job < 3 ? idesc_bf16(TROWS, T_HID)
+                                                   : idesc_bf16(TROWS, T_HID) | IDESC_B_MN_MAJOR;
+                    for (int kb = 0; kb < job_blocks(job); kb++, g++) {
+                        const uint32_t s = g % TRING, n = g / TRING;
+                        if (!(ok = mbar_wait(&full[s], n & 1, &abortFlag))) break;
+                        fence_after_sync();
+                        const uint32_t A = smem_u32(sA + kb * A_BLOCK), B = smem_u32(ring + s * W_BLOCK);
 #pragma unroll
-            for (int ks = 0; ks < UK / 16; ks++)
-                mma_bf16(tmem, desc_sw128(smem_u32(sA + s * UA_BYTES + ks * 32)),
-                         desc_sw128(smem_u32(sB + s * UB_BYTES + ks * 32)), idesc, (kb | ks) != 0);
-            mma_commit(&freed[s]);
+                        for (int ks = 0; ks < 4; ks++)
+                            mma_bf16(d, desc_sw128(A + ks * 32),
+                                     job < 3 ? desc_sw128(B + ks * 32)
+                                             : desc_sw128_mn(B + ks * 2048, W_BLOCK / 4),
+                                     idesc, (kb | ks) != 0);
+                        mma_commit(&empty[s]);
+                    }
+                    if (ok) mma_commit(&accFull);
+                }
         }
+        __syncwarp();
+    } else {
+        const int quarter = warp & 3, group = warp >> 2, r = quarter * 32 + lane, c0 = group * 64;
+        const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16);
+        uint32_t jobs = 0;
+        // Waits for a job's accumulator and for the operand buffer to have been copied out (a wait
+        // that gives up raises the flag; the tile runs to its end on whatever is there).
+        auto result = [&]() {
+            mbar_wait(&accFull, jobs & 1, &abortFlag);
+            jobs++;
+            if (tid == 0) bulk_wait_read();
+            __syncwarp();
+            named_sync(1, ROW_THREADS);
+            fence_after_sync();
+        };
+        // The operand buffer is written: copies it out and hands it to the tensor cores (if wanted).
+        auto operand = [&](uint8_t *image, uint32_t bytes, bool more) {
+            fence_async_shared();
+            fence_before_sync();
+            named_sync(1, ROW_THREADS);
+            if (tid == 0) bulk_s2g(image, sA, bytes);
+            if (more && lane == 0) mbar_arrive(&aFull);
+            __syncwarp();
+        };
+        auto put8 = [&](int col, const float *v) {
+            *reinterpret_cast<uint4 *>(sA + (col / 64) * A_BLOCK + sw128_offset(r, col % 64)) = pack8(v);
+        };
+        // This quarter's column sums into `out` (the tile's sums), the quarters added in order.
+        auto column_sums = [&](float *out) {
+            named_sync(1, ROW_THREADS);
+            if (tid < T_HID)
+                out[tid] = ((colSum[0][tid] + colSum[1][tid]) + colSum[2][tid]) + colSum[3][tid];
+            named_sync(1, ROW_THREADS);
+        };
+        const bool aligned = ((reinterpret_cast<uintptr_t>(a.stencil) |
+                               reinterpret_cast<uintptr_t>(a.particle)) & 15) == 0;
+        for (int t = 0; t < mine; t++) {
+            const size_t tile = blockIdx.x + (size_t)t * gridDim.x;
+            const long long row0 = (long long)tile * TROWS;
+            float *sums = a.w.sums + tile * SUMS;
+            // ---- X: 16-byte chunks of 8 features, the particle features after the stencil's
+            if (t > 0) {
+                if (tid == 0) bulk_wait_read();
+                named_sync(1, ROW_THREADS);
+            }
+            for (int e = tid; e < TROWS * X_KB * 8; e += ROW_THREADS) {
+                const int row = e / (X_KB * 8), chunk = e % (X_KB * 8), k = chunk * 8;
+                float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                const long long n = row0 + row;
+                if (n < a.batch && k < T_IN) {
+                    const float *src = k < T_STENCIL ? a.stencil + n * T_STENCIL + k : a.particle + n * T_PARTICLE;
+                    const int count = k < T_STENCIL ? 8 : T_PARTICLE;
+                    if (aligned) {
+                        *reinterpret_cast<float4 *>(v) = __ldg(reinterpret_cast<const float4 *>(src));
+                        if (count == 8)
+                            *reinterpret_cast<float4 *>(v + 4) = __ldg(reinterpret_cast<const float4 *>(src) + 1);
+                    } else {
+                        for (int q = 0; q < 8; q++)
+                            if (q < count) v[q] = __ldg(src + q);
+                    }
+                }
+                *reinterpret_cast<uint4 *>(sA + (k / 64) * A_BLOCK + sw128_offset(row, k % 64)) = pack8(v);
+            }
+            operand(a.w.X + tile * X_IMAGE, X_IMAGE, true);
+            // ---- layer 1: H1 = GELU(Z1), its slope to global memory
+            result();
+            float4 *slope = a.w.slope1 + tile * (size_t)(T_HID / 4) * TROWS + r;
+#pragma unroll 1
+            for (int c = c0; c < c0 + 64; c += 32) {
+                float v[32];
+                tmem_ld32(acc + (uint32_t)c, v);
+#pragma unroll
+                for (int q = 0; q < 32; q += 8) {
+                    float h[8], d[8];
+#pragma unroll
+                    for (int e = 0; e < 8; e++) h[e] = gelu_exact_tanh(v[q + e] + bias[0][c + q + e], d[e]);
+                    put8(c + q, h);
+                    slope[(size_t)((c + q) / 4) * TROWS] = make_float4(d[0], d[1], d[2], d[3]);
+                    slope[(size_t)((c + q) / 4 + 1) * TROWS] = make_float4(d[4], d[5], d[6], d[7]);
+                }
+            }
+            operand(a.w.H1 + tile * H_IMAGE, H_IMAGE, true);
+            // ---- layer 2: H2 = GELU(Z2), its slope in the accumulator's place
+            result();
+#pragma unroll 1
+            for (int c = c0; c < c0 + 64; c += 32) {
+                float v[32];
+                tmem_ld32(acc + (uint32_t)(T_HID + c), v);
+#pragma unroll
+                for (int q = 0; q < 32; q += 8) {
+                    float h[8];
+#pragma unroll
+                    for (int e = 0; e < 8; e++) {
+                        float d;
+                        h[e] = gelu_exact_tanh(v[q + e] + bias[1][c + q + e], d);
+                        v[q + e] = d;
+                    }
+                    put8(c + q, h);
+                }
+                tmem_st32(acc + (uint32_t)(T_HID + c), v);
+            }
+            tmem_wait_st();
+            operand(a.w.H2 + tile * H_IMAGE, H_IMAGE, true);
+            // ---- layer 3: H3 in registers, its slope in the accumulator's place
+            result();
+            float h3[64];
+#pragma unroll
+            for (int half = 0; half < 2; half++) {
+                float v[32];
+                const int c = c0 + 32 * half;
+                tmem_ld32(acc + (uint32_t)c, v);
+#pragma unroll
+                for (int e = 0; e < 32; e++) {
+                    float d;
+                    h3[32 * half + e] = gelu_exact_tanh(v[e] + bias[2][c + e], d);
+                    v[e] = d;
+                }
+                tmem_st32(acc + (uint32_t)c, v);
+            }
+            tmem_wait_st();
+            // layer 4: each row's three sums run over the 256 units in order, so the four column
+            // groups of a row take their turns
+            float o[T_OUT];
+#pragma unroll 1
+            for (int turn = 0; turn < 4; turn++) {
+                if (turn == group) {
+#pragma unroll
+                    for (int n = 0; n < T_OUT; n++) o[n] = turn ? outSum[r][n] : 0.f;
+#pragma unroll
+                    for (int e = 0; e < 64; e++)
+#pragma unroll
+                        for (int n = 0; n < T_OUT; n++) o[n] = fmaf(h3[e], w4[n][c0 + e], o[n]);
+#pragma unroll
+                    for (int n = 0; n < T_OUT; n++) outSum[r][n] = o[n];
+                }
+                named_sync(2 + quarter, 128);
+            }
+            // Y = O g; loss = mean over batch and outputs of (Y - target)^2; dO = 2 (Y - target) g / (3 batch)
+            const float scale = 1.f / (3.f * a.batch);
+            const long long n = row0 + r;
+            float dO[T_OUT], lossSum = 0.f;
+#pragma unroll
+            for (int q = 0; q < T_OUT; q++) {
+                dO[q] = 0.f;
+                if (n < a.batch) {
+                    const float g = __ldg(a.gate + n);
+                    const float d = (outSum[r][q] + __ldg(a.params + OFF_TB4 + q)) * g - __ldg(a.target + n * T_OUT + q);
+                    lossSum += d * d;
+                    dO[q] = 2.f * d * g * scale;
+                }
+            }
+            // dW4 from BF16-rounded operands, one output at a time
+#pragma unroll 1
+            for (int q = 0; q < T_OUT; q++) {
+                const float dq = bf16_rounded(q == 0 ? dO[0] : q == 1 ? dO[1] : dO[2]);
+#pragma unroll
+                for (int half = 0; half < 2; half++) {
+                    float v[32];
+#pragma unroll
+                    for (int e = 0; e < 32; e++) v[e] = dq * bf16_rounded(h3[32 * half + e]);
+                    colSum[quarter][c0 + 32 * half + lane] = lane_sums(v, lane);
+                }
+                column_sums(sums + SUM_DW4 + q * T_HID);
+            }
+            // db4 and the loss: the first group's warps, one per lane quarter
+            if (group == 0) {
+                float s[T_OUT + 1] = {dO[0], dO[1], dO[2], lossSum};
+#pragma unroll
+                for (int q = 0; q < T_OUT + 1; q++) {
+                    for (int off = 16; off > 0; off >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], off);
+                    if (lane == 0) colSum[quarter][q] = s[q];
+                }
+            }
+            named_sync(1, ROW_THREADS);
+            if (tid < T_OUT + 1)
+                sums[SUM_DB4 + tid] = ((colSum[0][tid] + colSum[1][tid]) + colSum[2][tid]) + colSum[3][tid];
+            named_sync(1, ROW_THREADS);
+            // ---- dZ3 = (dO W4) GELU'(Z3)
+#pragma unroll
+            for (int half = 0; half < 2; half++) {
+                float v[32];
+                const int c = c0 + 32 * half;
+                tmem_ld32(acc + (uint32_t)c, v);
+#pragma unroll
+                for (int e = 0; e < 32; e++) {
+                    float d = fmaf(dO[0], w4[0][c + e], 0.f);
+                    d = fmaf(dO[1], w4[1][c + e], d);
+                    d = fmaf(dO[2], w4[2][c + e], d);
+                    v[e] = d * v[e];
+                }
+#pragma unroll
+                for (int q = 0; q < 32; q += 8) put8(c + q, v + q);
+                colSum[quarter][c + lane] = lane_sums(v, lane);
+            }
+            operand(a.w.dZ3 + tile * H_IMAGE, H_IMAGE, true);
+            column_sums(sums + SUM_DB + 2 * T_HID);
+            // ---- dZ2 = (dZ3 W3) GELU'(Z2)
+            result();
+#pragma unroll 1
+            for (int c = c0; c < c0 + 64; c += 32) {
+                float v[32], d[32];
+                tmem_ld32(acc + (uint32_t)c, v);
+                tmem_ld32(acc + (uint32_t)(T_HID + c), d);
+#pragma unroll
+                for (int e = 0; e < 32; e++) v[e] *= d[e];
+#pragma unroll
+                for (int q = 0; q < 32; q += 8) put8(c + q, v + q);
+                colSum[quarter][c + lane] = lane_sums(v, lane);
+            }
+            operand(a.w.dZ2 + tile * H_IMAGE, H_IMAGE, true);
+            column_sums(sums + SUM_DB + T_HID);
+            // ---- dZ1 = (dZ2 W2) GELU'(Z1)
+            result();
+#pragma unroll 1
+            for (int c = c0; c < c0 + 64; c += 32) {
+                float v[32];
+                tmem_ld32(acc + (uint32_t)c, v);
+#pragma unroll
+                for (int q = 0; q < 32; q += 4) {
+                    const float4 d = slope[(size_t)((c + q) / 4) * TROWS];
+                    v[q] *= d.x;
+                    v[q + 1] *= d.y;
+                    v[q + 2] *= d.z;
+                    v[q + 3] *= d.w;
+                }
+#pragma unroll
+                for (int q = 0; q < 32; q += 8) put8(c + q, v + q);
+                colSum[quarter][c + lane] = lane_sums(v, lane);
+            }
+            operand(a.w.dZ1 + tile * H_IMAGE, H_IMAGE, false);
+            column_sums(sums + SUM_DB);
+            // one thread's reading of the flag decides for all row threads, which leave together
+            if (tid == 0) stopFlag = abortFlag;
+            named_sync(1, ROW_THREADS);
+            if (stopFlag) break;
+        }
+        if (tid == 0) bulk_wait_all();
     }
-    // every MMA issued so far lands before the accumulator is read (or the block exits)
-    if (tid == 0) mma_commit(&accFull);
+    fence_before_sync();
+    __syncthreads();
+    if (warp == MMA_WARP) {
+        fence_after_sync();
+        tmem_dealloc(tmem, 512);
+    }
+    if (tid == 0 && abortFlag) atomicOr(a.w.err, 1);
+}
+
+// ------------------------------------------------------------------ weight gradients
+
+constexpr uint32_t G_A = 2 * A_BLOCK, G_B = H_KB * A_BLOCK;  // 128 hidden units of dZ; up to 256 columns
+constexpr size_t GRAD_SMEM = 2 * (size_t)(G_A + G_B) + 1024;
+constexpr int GRAD_THREADS = 128;
+
+struct GradArgs {
+    int tiles, splits;
+    Work w;
+};
+
+// Unit u over the tiles of its range: partial = sum over rows of dZ[row][m] V[row][n]. Both operands
+// are the tiles' images read along their rows (MN-major: 64 units per 128-byte row, 8 rows per 1024
+// bytes, the next 64 units one K-block further), two tiles in flight. Bound by the copies of the
+// images from L2 (96 KB for 8 MMAs).
+__global__ void __launch_bounds__(GRAD_THREADS, 1) weight_grad_kernel(const GradArgs a) {
+    using namespace umma;
+    extern __shared__ uint8_t dynSmem[];
+    uint8_t *base = reinterpret_cast<uint8_t *>(((uintptr_t)dynSmem + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) uint64_t full[2], empty[2], accFull;
+    __shared__ uint32_t tmemSlot;
+    __shared__ int abortFlag;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int unit = blockIdx.x, split = blockIdx.y, half = unit & 1;
+    const int per = (a.tiles + a.splits - 1) / a.splits;
+    const int first = split * per, last = min(a.tiles, first + per), count = max(last - first, 0);
+    const int kind = unit >> 1;  // 0: W3, 1: W2, 2: W1 columns 0-255, 3: the rest of W1
+    const uint8_t *A = (kind == 0 ? a.w.dZ3 : kind == 1 ? a.w.dZ2 : a.w.dZ1) + half * G_A;
+    const uint8_t *B = kind == 0 ? a.w.H2 : kind == 1 ? a.w.H1 : kind == 2 ? a.w.X : a.w.X + G_B;
+    const size_t strideB = kind < 2 ? H_IMAGE : X_IMAGE;
+    const uint32_t bytesB = kind < 3 ? G_B : X_IMAGE - G_B;
+    const int N = kind < 3 ? T_HID : X_TAIL_N;
+    if (tid == 0) {
+        for (int s = 0; s < 2; s++) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(&accFull, 1);
+        abortFlag = 0;
+        fence_barrier_init();
+    }
+    if (warp == 0) tmem_alloc(&tmemSlot, 256);
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    const uint32_t tmem = tmemSlot;
+    if (tid == 0) {
+        const uint32_t idesc = idesc_bf16(TROWS, N) | IDESC_A_MN_MAJOR | IDESC_B_MN_MAJOR;
+        int issued[2] = {-1, -1};
+        auto load = [&](int t) {
+            const int s = t & 1, n = t >> 1;
+            if (!mbar_wait(&empty[s], (uint32_t)(n & 1) ^ 1, &abortFlag)) return false;
+            uint8_t *dst = base + s * (G_A + G_B);
+            mbar_expect_tx(&full[s], G_A + bytesB);
+            bulk_g2s(dst, A + (size_t)(first + t) * H_IMAGE, G_A, &full[s]);
+            bulk_g2s(dst + G_A, B + (size_t)(first + t) * strideB, bytesB, &full[s]);
+            issued[s] = n;
+            return true;
+        };
+        int consumed[2] = {-1, -1};
+        bool ok = count == 0 || load(0);
+        for (int t = 0; t < count && ok; t++) {
+            if (t + 1 < count) ok = load(t + 1);
+            const int s = t & 1, n = t >> 1;
+            if (!ok || !(ok = mbar_wait(&full[s], (uint32_t)n & 1, &abortFlag))) break;
+            consumed[s] = n;
+            fence_after_sync();
+            const uint32_t sA = smem_u32(base + s * (G_A + G_B)), sB = sA + G_A;
+#pragma unroll
+            for (int ks = 0; ks < TROWS / 16; ks++)
+                mma_bf16(tmem, desc_sw128_mn(sA + ks * 2048, A_BLOCK), desc_sw128_mn(sB + ks * 2048, A_BLOCK),
+                         idesc, (t | ks) != 0);
+            mma_commit(&empty[s]);
+        }
+        mma_commit(&accFull);
+        for (int s = 0; s < 2; s++)  // copies still in flight land before the block exits
+            if (issued[s] > consumed[s]) mbar_wait_bounded(&full[s], (uint32_t)issued[s] & 1);
+    }
+    __syncwarp();
     const bool done = mbar_wait_bounded(&accFull, 0);
     __syncwarp();
     fence_after_sync();
-    const bool valid = ok && done && !abortFlag;
-    if (valid) {
-        const int quarter = warp & 3, half = warp >> 2;
-        const int m = m0 + quarter * 32 + lane;
-        for (int c0 = half * (UN / 2); c0 < (half + 1) * (UN / 2) && c0 < nTile; c0 += 32) {
-            float v[32];
-            if (nkb > 0) {
-                tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, v);
-            } else {
+    float4 *out = a.w.partial + ((size_t)unit * a.splits + split) * (T_HID / 4) * TROWS + warp * 32 + lane;
+    for (int c = 0; c < N; c += 32) {
+        float v[32];
+        tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
 #pragma unroll
-                for (int c = 0; c < 32; c++) v[c] = 0.f;
-            }
-            if (m >= g.M) continue;
-#pragma unroll
-            for (int c = 0; c < 32; c++) {
-                const int n = n0 + c0 + c;
-                if (n >= g.N) break;
-                float z = v[c];
-                if (EPI == 3) {
-                    g.partial[((size_t)blockIdx.z * g.M + m) * g.N + n] = z;
-                    continue;
-                }
-                if (EPI >= 1) z += __ldg(g.bias + n);
-                g.C[(size_t)m * g.ldc + n] = z;
-                if (EPI == 2) g.H[(size_t)m * g.ldc + n] = gelu_exact_tanh(z, nullptr);
-            }
-        }
+        for (int q = 0; q < 32; q += 4)
+            out[(size_t)((c + q) / 4) * TROWS] =
+                count ? make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    if (!valid && tid == 0) atomicOr(g.err, 1);
+    if (tid == 0 && (!done || abortFlag)) atomicOr(a.w.err, 1);
     fence_before_sync();
     __syncthreads();
     if (warp == 0) {
         fence_after_sync();
-        tmem_dealloc(tmem, UN);
+        tmem_dealloc(tmem, 256);
     }
 }
 
-// out[m][n] = sum over the splits z (in order) of partial[z][m][n].
-__global__ void split_sum_kernel(const float *partial, int splits, size_t cells, float *out) {
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < cells;
-         e += (size_t)gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int z = 0; z < splits; z++) s += partial[(size_t)z * cells + e];
-        out[e] = s;
+// ------------------------------------------------------------------ sums and Adam
+
+struct Adam {
+    float *params, *grads, *m, *v;
+    float lr, c1, c2;
+    int update;
+    // gradient of parameter e, then its Adam step (beta1 0.9, beta2 0.999, eps 1e-8, bias-corrected)
+    __device__ __forceinline__ void apply(size_t e, float gi) const {
+        grads[e] = gi;
+        if (!update) return;
+        const float mi = 0.9f * m[e] + 0.1f * gi, vi = 0.999f * v[e] + 0.001f * gi * gi;
+        m[e] = mi;
+        v[e] = vi;
+        params[e] -= lr * (mi / c1) / (sqrtf(vi / c2) + 1e-8f);
     }
+};
+
+constexpr int WEIGHT_ITEMS = UNITS * (T_HID / 4) * TROWS;  // float4s of the partial weight gradients
+constexpr int WEIGHT_BLOCKS = WEIGHT_ITEMS / 256;
+constexpr int SUM_BLOCKS = (SUMS + 31) / 32;
+
+// The first WEIGHT_BLOCKS blocks sum the splits of four weights per thread; the others sum 32 of the
+// tile sums each, 8 ranges of tiles per column added in order.
+__global__ void __launch_bounds__(256) finish_kernel(const GradArgs a, const Adam adam, float lossScale,
+                                                     float *loss) {
+    if (blockIdx.x < WEIGHT_BLOCKS) {
+        const int e = blockIdx.x * 256 + threadIdx.x;
+        const int r = e % TROWS, c = e / TROWS % (T_HID / 4) * 4, unit = e / (TROWS * (T_HID / 4));
+        const int kind = unit >> 1;
+        if (kind == 3 && c >= X_TAIL) return;
+        const float4 *p = a.w.partial + (size_t)unit * a.splits * (T_HID / 4) * TROWS + (size_t)(c / 4) * TROWS + r;
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int z = 0; z < a.splits; z++) {
+            const float4 q = p[(size_t)z * (T_HID / 4) * TROWS];
+            s.x += q.x;
+            s.y += q.y;
+            s.z += q.z;
+            s.w += q.w;
+        }
+        const int n = (unit & 1) * TROWS + r;
+        const size_t at = kind == 0   ? OFF_TW3 + (size_t)n * T_HID + c
+                          : kind == 1 ? OFF_TW2 + (size_t)n * T_HID + c
+                                      : OFF_TW1 + (size_t)n * T_IN + (kind == 3 ? T_HID : 0) + c;
+        adam.apply(at, s.x);
+        adam.apply(at + 1, s.y);
+        adam.apply(at + 2, s.z);
+        adam.apply(at + 3, s.w);
+        return;
+    }
+    __shared__ float part[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int c = (blockIdx.x - WEIGHT_BLOCKS) * 32 + lane;
+    const int per = (a.tiles + 7) / 8, first = warp * per, last = min(a.tiles, first + per);
+    float s = 0.f;
+    if (c < SUMS)
+        for (int t = first; t < last; t++) s += a.w.sums[(size_t)t * SUMS + c];
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp || c >= SUMS) return;
+    s = 0.f;
+    for (int q = 0; q < 8; q++) s += part[q][lane];
+    if (c == SUM_LOSS) *loss = s * lossScale;
+    else if (c >= SUM_DB4) adam.apply(OFF_TB4 + (c - SUM_DB4), s);
+    else if (c >= SUM_DW4) adam.apply(OFF_TW4 + (c - SUM_DW4), s);
+    else adam.apply((c < T_HID ? OFF_TB1 : c < 2 * T_HID ? OFF_TB2 : OFF_TB3) + c % T_HID, s);
 }
 
-// Floats of the weight-gradient partial sums: at most 148 / (output tiles) splits of M x N, the
-// most for a 256 x 256 weight (two tiles, 74 splits).
-constexpr size_t UMMA_PARTIAL_FLOATS = (size_t)(148 / 2) * T_HID * T_HID;
-
-cudaError_t umma_prepare() {
+// Shared-memory sizes of the tensor-core kernels, once per device.
+cudaError_t train_prepare() {
     static bool done[64] = {};
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
     if (device >= 0 && device < 64 && done[device]) return cudaSuccess;
-    for (auto fn : {umma_gemm_kernel<0>, umma_gemm_kernel<1>, umma_gemm_kernel<2>, umma_gemm_kernel<3>}) {
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)USMEM);
-        if (e != cudaSuccess) return e;
-    }
-    if (device >= 0 && device < 64) done[device] = true;
-    return cudaSuccess;
-}
-
-// C (M x N, leading dimension ldc) from a(m, k) = A[m sam + k sak] and b(n, k) = B[n sbn + k sbk]
-// on the tensor cores. EPI 3 (a reduction over a long K, the batch) splits K over about one block
-// per SM and sums the splits in order into C (ldc must be N).
-template <int EPI>
-cudaError_t umma_gemm(int M, int N, int K, const float *A, long long sam, long long sak,
-                      const float *B, long long sbn, long long sbk, const float *bias, float *C,
-                      float *H, int ldc, float *partial, int *err, cudaStream_t stream) {
-    cudaError_t e = umma_prepare();
-    if (e != cudaSuccess) return e;
-    UmmaGemm g;
-    g.M = M;
-    g.N = N;
-    g.K = K;
-    g.A = A;
-    g.sam = sam;
-    g.sak = sak;
-    g.B = B;
-    g.sbn = sbn;
-    g.sbk = sbk;
-    g.bias = bias;
-    g.C = C;
-    g.H = H;
-    g.partial = partial;
-    g.ldc = ldc;
-    g.err = err;
-    const int tilesN = (N + UN - 1) / UN, tilesM = (M + UM - 1) / UM;
-    int splits = 1;
-    g.kPerSplit = ((K + UK - 1) / UK) * UK;
-    if (EPI == 3) {
-        splits = 148 / (tilesN * tilesM);
-        if (splits < 1) splits = 1;
-        const int kBlocks = (K + UK - 1) / UK;
-        if (splits > kBlocks) splits = kBlocks > 0 ? kBlocks : 1;
-        g.kPerSplit = ((kBlocks + splits - 1) / splits) * UK;
-        splits = (K + g.kPerSplit - 1) / g.kPerSplit;
-        if (splits < 1) splits = 1;
-        if ((size_t)splits * M * N > UMMA_PARTIAL_FLOATS || ldc != N) return cudaErrorInvalidValue;
-    }
-    dim3 grid(tilesN, tilesM, splits);
-    umma_gemm_kernel<EPI><<<grid, UTHREADS, USMEM, stream>>>(g);
-    e = cudaGetLastError();
-    if (e != cudaSuccess || EPI != 3) return e;
-    const size_t cells = (size_t)M * N;
-    split_sum_kernel<<<(int)((cells + 255) / 256), 256, 0, stream>>>(partial, splits, cells, C);
-    return cudaGetLastError();
-}
-
-// C[M][N] = sum_k a(m, k) b(k, n) with a(m, k) = TA ? A[k lda + m] : A[m lda + k] and
-// b(k, n) = TB ? B[n ldb + k] : B[k ldb + n]. EPI 0: store; 1: add bias[n] and store; 2: add
-// bias[n], store Z and GELU(Z) into H; 3: add into C atomically (the K range split over
-// gridDim.z, C zeroed beforehand). 64 x 64 tiles, 256 threads of 4 x 4 outputs, K steps of 16;
-// each operand tile is read with its contiguous index fastest.
-template <bool TA, bool TB, int EPI>
-__global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, const float *A, int lda,
-                                                   const float *B, int ldb, const float *bias,
-                                                   float *C, float *H, int ldc) {
-    __shared__ float As[16][64 + 1], Bs[16][64 + 1];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    const int kPer = ((K + gridDim.z - 1) / gridDim.z + 15) / 16 * 16;
-    const int kBegin = blockIdx.z * kPer, kEnd = min(K, kBegin + kPer);
-    float acc[4][4] = {};
-    for (int k0 = kBegin; k0 < kEnd; k0 += 16) {
-        for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-            // A: m contiguous when transposed, k contiguous otherwise
-            const int kk = TA ? e / 64 : e % 16, r = TA ? e % 64 : e / 16;
-            const int m = m0 + r, k = k0 + kk;
-            As[kk][r] = (m < M && k < kEnd) ? (TA ? A[(size_t)k * lda + m] : A[(size_t)m * lda + k])
-                                            : 0.f;
-        }
-        for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-            // B: k contiguous when transposed, n contiguous otherwise
-            const int kk = TB ? e % 16 : e / 64, r = TB ? e / 16 : e % 64;
-            const int n = n0 + r, k = k0 + kk;
-            Bs[kk][r] = (n < N && k < kEnd) ? (TB ? B[(size_t)n * ldb + k] : B[(size_t)k * ldb + n])
-                                            : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; kk++) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int m = m0 + ty * 4 + i;
-        if (m >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int n = n0 + tx * 4 + j;
-            if (n >= N) continue;
-            float z = acc[i][j];
-            if (EPI == 3) {
-                atomicAdd(C + (size_t)m * ldc + n, z);
-                continue;
-            }
-            if (EPI >= 1) z += bias[n];
-            C[(size_t)m * ldc + n] = z;
-            if (EPI == 2) H[(size_t)m * ldc + n] = gelu_exact_tanh(z, nullptr);
-        }
-    }
-}
-
-template <bool TA, bool TB, int EPI>
-void gemm(int M, int N, int K, const float *A, int lda, const float *B, int ldb, const float *bias,
-          float *C, float *H, int ldc, cudaStream_t stream) {
-    // the batch reductions (EPI 3) are split so that about two blocks run per SM
-    const int tiles = ((N + 63) / 64) * ((M + 63) / 64);
-    int splits = EPI == 3 ? (296 + tiles - 1) / tiles : 1;
-    if (splits > (K + 63) / 64) splits = (K + 63) / 64 > 0 ? (K + 63) / 64 : 1;
-    dim3 grid((N + 63) / 64, (M + 63) / 64, splits);
-    gemm_kernel<TA, TB, EPI><<<grid, 256, 0, stream>>>(M, N, K, A, lda, B, ldb, bias, C, H, ldc);
-}
-
-// X = [stencil | particle], [batch][388].
-__global__ void concat_kernel(const float *stencil, const float *particle, int batch, float *X) {
-    const size_t total = (size_t)batch * T_IN;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
-         e += (size_t)gridDim.x * blockDim.x) {
-        const size_t b = e / T_IN, c = e % T_IN;
-        X[e] = c < T_STENCIL ? stencil[b * T_STENCIL + c] : particle[b * T_PARTICLE + (c - T_STENCIL)];
-    }
-}
-
-// Y = O g; loss = mean over batch and outputs of (Y - target)^2; dO = 2 (Y - target) g / (3 batch).
-__global__ void loss_kernel(const float *O, const float *gate, const float *target, int batch,
-                            float *dO, float *loss) {
-    __shared__ float partial[256];
-    float sum = 0.f;
-    const float scale = 1.f / (3.f * batch);
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < batch * T_OUT; e += gridDim.x * blockDim.x) {
-        const float g = gate[e / T_OUT];
-        const float d = O[e] * g - target[e];
-        sum += d * d;
-        dO[e] = 2.f * d * g * scale;
-    }
-    partial[threadIdx.x] = sum;
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s) partial[threadIdx.x] += partial[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) atomicAdd(loss, partial[0] * scale);
-}
-
-// dZ = dH * GELU'(Z), in place in dH.
-__global__ void gelu_backward_kernel(const float *Z, float *dH, size_t n) {
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n;
-         e += (size_t)gridDim.x * blockDim.x) {
-        float d;
-        gelu_exact_tanh(Z[e], &d);
-        dH[e] *= d;
-    }
-}
-
-// db[n] = sum over the batch of dZ[b][n], in two passes with a fixed order: block (x, y) sums the
-// 32 columns 32x.. over the rows of chunk y (warp w takes rows w, w + 8, ..., its lanes one column
-// each, so every row is read as one 128-byte line), adding its 8 warps' sums in order into
-// partial[y][n]; then the chunks are added in order.
-constexpr int COLUMN_CHUNKS = 64;
-
-__global__ void column_partial_kernel(const float *dZ, int batch, int N, float *partial) {
-    __shared__ float warpSum[8][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int n = blockIdx.x * 32 + lane;
-    const int per = (batch + COLUMN_CHUNKS - 1) / COLUMN_CHUNKS;
-    const int b0 = blockIdx.y * per, b1 = min(batch, b0 + per);
-    float sum = 0.f;
-    if (n < N)
-        for (int b = b0 + warp; b < b1; b += 8) sum += dZ[(size_t)b * N + n];
-    warpSum[warp][lane] = sum;
-    __syncthreads();
-    if (warp == 0 && n < N) {
-        float total = 0.f;
-        for (int w = 0; w < 8; w++) total += warpSum[w][lane];
-        partial[(size_t)blockIdx.y * N + n] = total;
-    }
-}
-
-__global__ void column_final_kernel(const float *partial, int N, float *db) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    float total = 0.f;
-    for (int c = 0; c < COLUMN_CHUNKS; c++) total += partial[(size_t)c * N + n];
-    db[n] = total;
-}
-
-void column_sum(const float *dZ, int batch, int N, float *partial, float *db, cudaStream_t stream) {
-    column_partial_kernel<<<dim3((N + 31) / 32, COLUMN_CHUNKS), 256, 0, stream>>>(dZ, batch, N, partial);
-    column_final_kernel<<<(N + 255) / 256, 256, 0, stream>>>(partial, N, db);
-}
-
-// Adam (beta1 0.9, beta2 0.999, eps 1e-8, bias-corrected at `step`).
-__global__ void adam_kernel(float *p, const float *g, float *m, float *v, size_t n, float lr,
-                            float c1, float c2) {
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n;
-         e += (size_t)gridDim.x * blockDim.x) {
-        const float gi = g[e];
-        const float mi = 0.9f * m[e] + 0.1f * gi, vi = 0.999f * v[e] + 0.001f * gi * gi;
-        m[e] = mi;
-        v[e] = vi;
-        p[e] -= lr * (mi / c1) / (sqrtf(vi / c2) + 1e-8f);
-    }
-}
-
-int blocks_for(size_t n) {
-    const size_t b = (n + 255) / 256;
-    return (int)(b < 148 * 8 ? (b > 0 ? b : 1) : 148 * 8);
+    e = cudaFuncSetAttribute(tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_SMEM);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(weight_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GRAD_SMEM);
+    if (e == cudaSuccess && device >= 0 && device < 64) done[device] = true;
+    return e;
 }
 
 }  // namespace
 
 size_t mlp_train_work_floats(int batch) {
-    // an error word (padded to 16 bytes), the weight-gradient partial sums, then the
-    // activations and gradients of the batch
-    return 4 + UMMA_PARTIAL_FLOATS + (size_t)batch * (T_IN + 6 * T_HID + 2 * T_OUT + 2 * T_HID);
+    // the error word and the distance to the next 1024-byte boundary, then the work areas
+    return (1024 + 16 + work_bytes(tiles_of(batch), nullptr, nullptr)) / sizeof(float);
 }
 
 cudaError_t mlp_train_step(const float *stencil, const float *particle, const float *gate,
                            const float *target, int batch, float *params, float *grads, float *m,
                            float *v, float *work, float *loss, int step, float lr, bool update,
                            cudaStream_t stream) {
-    const int B = batch;
-    int *err = reinterpret_cast<int *>(work);
-    float *partial = work + 4;
-    float *X = partial + UMMA_PARTIAL_FLOATS, *Z1 = X + (size_t)B * T_IN,
-          *H1 = Z1 + (size_t)B * T_HID, *Z2 = H1 + (size_t)B * T_HID, *H2 = Z2 + (size_t)B * T_HID,
-          *Z3 = H2 + (size_t)B * T_HID, *H3 = Z3 + (size_t)B * T_HID, *O = H3 + (size_t)B * T_HID,
-          *dO = O + (size_t)B * T_OUT, *dA = dO + (size_t)B * T_OUT, *dB = dA + (size_t)B * T_HID;
-    const float *W1 = params + OFF_TW1, *W2 = params + OFF_TW2, *W3 = params + OFF_TW3,
-                *W4 = params + OFF_TW4;
-    cudaError_t e = cudaMemsetAsync(loss, 0, sizeof(float), stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(grads, 0, T_PARAMS * sizeof(float), stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(int), stream);
+    cudaError_t e = train_prepare();
     if (e != cudaSuccess) return e;
-    concat_kernel<<<blocks_for((size_t)B * T_IN), 256, 0, stream>>>(stencil, particle, B, X);
-#define UMMA(call)                              \
-    do {                                        \
-        if ((e = (call)) != cudaSuccess) return e; \
-    } while (0)
-    // forward: layers 1-3 on the tensor cores (BF16 operands, bias and GELU in the epilogue),
-    // layer 4 (three outputs) on the CUDA cores
-    UMMA(umma_gemm<2>(B, T_HID, T_IN, X, T_IN, 1, W1, T_IN, 1, params + OFF_TB1, Z1, H1, T_HID,
-                      partial, err, stream));
-    UMMA(umma_gemm<2>(B, T_HID, T_HID, H1, T_HID, 1, W2, T_HID, 1, params + OFF_TB2, Z2, H2,
-                      T_HID, partial, err, stream));
-    UMMA(umma_gemm<2>(B, T_HID, T_HID, H2, T_HID, 1, W3, T_HID, 1, params + OFF_TB3, Z3, H3,
-                      T_HID, partial, err, stream));
-    gemm<false, true, 1>(B, T_OUT, T_HID, H3, T_HID, W4, T_HID, params + OFF_TB4, O, nullptr, T_OUT, stream);
-    loss_kernel<<<blocks_for((size_t)B * T_OUT), 256, 0, stream>>>(O, gate, target, B, dO, loss);
-    // backward, layer 4: dW4 = dO^T H3 (tensor cores, reduction over the batch), dA = dO W4
-    UMMA(umma_gemm<3>(T_OUT, T_HID, B, dO, 1, T_OUT, H3, 1, T_HID, nullptr, grads + OFF_TW4,
-                      nullptr, T_HID, partial, err, stream));
-    column_sum(dO, B, T_OUT, partial, grads + OFF_TB4, stream);
-    gemm<false, false, 0>(B, T_HID, T_OUT, dO, T_OUT, W4, T_HID, nullptr, dA, nullptr, T_HID, stream);
-    // layer 3: dZ3 = dA GELU'(Z3); dW3 = dZ3^T H2; dB = dZ3 W3
-    gelu_backward_kernel<<<blocks_for((size_t)B * T_HID), 256, 0, stream>>>(Z3, dA, (size_t)B * T_HID);
-    UMMA(umma_gemm<3>(T_HID, T_HID, B, dA, 1, T_HID, H2, 1, T_HID, nullptr, grads + OFF_TW3,
-                      nullptr, T_HID, partial, err, stream));
-    column_sum(dA, B, T_HID, partial, grads + OFF_TB3, stream);
-    UMMA(umma_gemm<0>(B, T_HID, T_HID, dA, T_HID, 1, W3, 1, T_HID, nullptr, dB, nullptr, T_HID,
-                      partial, err, stream));
-    // layer 2
-    gelu_backward_kernel<<<blocks_for((size_t)B * T_HID), 256, 0, stream>>>(Z2, dB, (size_t)B * T_HID);
-    UMMA(umma_gemm<3>(T_HID, T_HID, B, dB, 1, T_HID, H1, 1, T_HID, nullptr, grads + OFF_TW2,
-                      nullptr, T_HID, partial, err, stream));
-    column_sum(dB, B, T_HID, partial, grads + OFF_TB2, stream);
-    UMMA(umma_gemm<0>(B, T_HID, T_HID, dB, T_HID, 1, W2, 1, T_HID, nullptr, dA, nullptr, T_HID,
-                      partial, err, stream));
-    // layer 1 (no input gradient)
-    gelu_backward_kernel<<<blocks_for((size_t)B * T_HID), 256, 0, stream>>>(Z1, dA, (size_t)B * T_HID);
-    UMMA(umma_gemm<3>(T_HID, T_IN, B, dA, 1, T_HID, X, 1, T_IN, nullptr, grads + OFF_TW1,
-                      nullptr, T_IN, partial, err, stream));
-    column_sum(dA, B, T_HID, partial, grads + OFF_TB1, stream);
-#undef UMMA
-    if (update) {
-        const float c1 = 1.f - powf(0.9f, (float)step), c2 = 1.f - powf(0.999f, (float)step);
-        adam_kernel<<<blocks_for(T_PARAMS), 256, 0, stream>>>(params, grads, m, v, T_PARAMS, lr, c1, c2);
-    }
+    const int tiles = (int)tiles_of(batch);
+    Work w;
+    work_bytes((size_t)tiles, &w,
+               reinterpret_cast<uint8_t *>(((uintptr_t)(work + 4) + 1023) & ~(uintptr_t)1023));
+    w.err = reinterpret_cast<int *>(work);
+    pack_weights_kernel<<<W_BLOCKS * T_HID * 8 / 256, 256, 0, stream>>>(params, w.weights, w.err);
+    const TileArgs t{stencil, particle, gate, target, params, batch, tiles, w};
+    tile_kernel<<<tiles < 148 ? tiles : 148, TILE_THREADS, TILE_SMEM, stream>>>(t);
+    const GradArgs g{tiles, tiles < MAX_SPLITS ? tiles : MAX_SPLITS, w};
+    weight_grad_kernel<<<dim3(UNITS, g.splits), GRAD_THREADS, GRAD_SMEM, stream>>>(g);
+    const Adam adam{params, grads, m, v, lr, 1.f - powf(0.9f, (float)step),
+                    1.f - powf(0.999f, (float)step), update ? 1 : 0};
+    finish_kernel<<<WEIGHT_BLOCKS + SUM_BLOCKS, 256, 0, stream>>>(g, adam, 1.f / (3.f * batch), loss);
     return cudaGetLastError();
 }
 

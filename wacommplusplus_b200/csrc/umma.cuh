@@ -24,6 +24,9 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
+// Instruction-descriptor bits for an operand whose M (or N) index is contiguous in shared memory.
+constexpr uint32_t IDESC_A_MN_MAJOR = 1u << 15, IDESC_B_MN_MAJOR = 1u << 16;
+
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -35,6 +38,18 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {
     d |= (uint64_t)(1024 >> 4) << 32;     // stride byte offset: next 8-row group
     d |= (uint64_t)1 << 46;               // descriptor version (sm_100)
     d |= (uint64_t)2 << 61;               // 128-byte swizzle
+    return d;
+}
+
+// The same image read as an MN-major operand (its rows are the K index): 64 units of M or N per
+// 128-byte row, 8 K rows per 1024 bytes, the next 64 units `nextUnits` bytes further. A 16-deep K
+// slice is 2048 bytes of the address.
+__device__ __forceinline__ uint64_t desc_sw128_mn(uint32_t addr, uint32_t nextUnits) {
+    uint64_t d = (uint64_t)((addr & 0x3FFFF) >> 4);
+    d |= (uint64_t)(nextUnits >> 4) << 16;  // leading byte offset: next 64 units of M or N
+    d |= (uint64_t)(1024 >> 4) << 32;       // stride byte offset: next 8 K rows
+    d |= (uint64_t)1 << 46;                 // descriptor version (sm_100)
+    d |= (uint64_t)2 << 61;                 // 128-byte swizzle
     return d;
 }
 
