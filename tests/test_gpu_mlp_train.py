@@ -67,6 +67,49 @@ def test_weight_gradients_are_reproducible(cuda_device):
     assert torch.equal(first.grads, second.grads)
 
 
+# edges of the 128-row tiles, of the 18 ranges of tiles a weight gradient is split into, and of the
+# 148 tiles of one turn
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 2304, 2305, 18944, 18945])
+def test_gradients_at_tile_edges(cuda_device, n):
+    """As above; a BF16 rounding that falls to the other side changes one of n products by 2^-8, of
+    either operand, so few rows get that much more."""
+    from wacommplusplus_b200.surrogate_train import KernelTrainer
+    weights = sg.random_weights(seed=8)
+    data = _batch(n, seed=n)
+    trainer = KernelTrainer(torch, weights, batch=n)
+    loss = float(trainer.run(*_cuda(*data), update=False))
+    assert trainer.error_flag() == 0
+    want_loss, want = mo.loss_and_gradients(weights, *data, bf16_operands=True)
+    got = trainer.grads.cpu().numpy().astype(np.float64)
+    assert abs(loss - want_loss) <= (1e-4 + 2.0 ** -7 / n) * abs(want_loss), (loss, want_loss)
+    at = 0
+    for name, shape in mo.SHAPES:
+        size = int(np.prod(shape))
+        g, w = got[at:at + size], want[at:at + size]
+        rel = np.abs(g - w).max() / max(np.abs(w).max(), 1e-30)
+        assert rel < 2e-3 + 2.0 ** -7 / np.sqrt(n), (name, rel)
+        at += size
+
+
+def test_unaligned_inputs_and_work_buffer(cuda_device):
+    """Rows and the work buffer at any float boundary give the same bits."""
+    from wacommplusplus_b200.surrogate_train import KernelTrainer
+    data = _cuda(*_batch(300, seed=4))
+    trainer = KernelTrainer(torch, sg.random_weights(seed=2), batch=300)
+    trainer.run(*data, update=False)
+    want = trainer.grads.clone()
+
+    def shifted(x):
+        flat = torch.empty(x.numel() + 1, dtype=torch.float32, device="cuda")[1:]
+        flat.copy_(x.reshape(-1))
+        return flat.view(x.shape)
+    trainer.work = torch.empty(trainer.work.numel() + 3, dtype=torch.float32, device="cuda")[3:]
+    trainer.grads.zero_()
+    trainer.run(*[shifted(x) for x in data], update=False)
+    assert trainer.error_flag() == 0
+    assert torch.equal(trainer.grads, want)
+
+
 def test_adam_steps_match_the_oracle(cuda_device):
     from wacommplusplus_b200.surrogate_train import KernelTrainer
     weights = sg.random_weights(seed=6)

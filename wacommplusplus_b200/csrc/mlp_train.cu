@@ -177,8 +177,11 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 // warp streaming weights through a ring of bulk copies, one issuing the MMAs. Operand buffer (112 KB):
 // X, then H1, H2, dZ3, dZ2, dZ1 in turn, each copied out as it stands for the weight gradients.
 // Tensor memory: columns 0-255 hold the accumulators of layers 1 and 3 and of both gradients,
-// columns 256-511 that of layer 2, replaced by GELU'(Z2). The GELU and its derivative (a precise
-// tanhf per unit and layer) bound it; the tensor cores and the weight stream work underneath.
+// columns 256-511 that of layer 2, replaced by GELU'(Z2). Bound by the latency of one tile's chain of
+// five GEMMs and epilogues (a precise tanhf per unit and layer) and by issue inside them: 16,384 rows,
+// 128 tiles on 148 SMs, 71 us of a step of 0.107 ms (issue 39 %); with per-layer GEMMs that staged
+// FP32 operands through threads the step took 0.720 ms. With the GELU unrolled over 32 columns its
+// code overflowed the instruction cache: 90 us.
 __global__ void __launch_bounds__(TILE_THREADS, 1) tile_kernel(const TileArgs a) {
     using namespace umma;
     extern __shared__ uint8_t dynSmem[];
@@ -187,7 +190,8 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) tile_kernel(const TileArgs a)
     __shared__ __align__(8) uint64_t full[TRING], empty[TRING], aFull, accFull;
     __shared__ uint32_t tmemSlot;
     __shared__ int abortFlag, stopFlag;
-    __shared__ float bias[3][T_HID], w4[T_OUT][T_HID], outSum[TROWS][T_OUT];
+    __shared__ __align__(16) float bias[3][T_HID], w4[T_OUT][T_HID];
+    __shared__ float outSum[TROWS][T_OUT];
     __shared__ float colSum[4][T_HID];  // one sum over 32 rows per lane quarter
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
@@ -315,7 +319,11 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) tile_kernel(const TileArgs a)
                 if (tid == 0) bulk_wait_read();
                 named_sync(1, ROW_THREADS);
             }
-            for (int e = tid; e < TROWS * X_KB * 8; e += ROW_THREADS) {
+            // (seven chunks per thread in flight)
+            static_assert(TROWS * X_KB * 8 % (7 * ROW_THREADS) == 0, "whole groups of chunks");
+#pragma unroll 7
+            for (int turn = 0; turn < TROWS * X_KB * 8 / ROW_THREADS; turn++) {
+                const int e = turn * ROW_THREADS + tid;
                 const int row = e / (X_KB * 8), chunk = e % (X_KB * 8), k = chunk * 8;
                 float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
                 const long long n = row0 + row;
@@ -338,56 +346,49 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) tile_kernel(const TileArgs a)
             result();
             float4 *slope = a.w.slope1 + tile * (size_t)(T_HID / 4) * TROWS + r;
 #pragma unroll 1
-            for (int c = c0; c < c0 + 64; c += 32) {
-                float v[32];
-                tmem_ld32(acc + (uint32_t)c, v);
+            for (int c = c0; c < c0 + 64; c += 8) {
+                float v[8], d[8];
+                tmem_ld8(acc + (uint32_t)c, v);
 #pragma unroll
-                for (int q = 0; q < 32; q += 8) {
-                    float h[8], d[8];
-#pragma unroll
-                    for (int e = 0; e < 8; e++) h[e] = gelu_exact_tanh(v[q + e] + bias[0][c + q + e], d[e]);
-                    put8(c + q, h);
-                    slope[(size_t)((c + q) / 4) * TROWS] = make_float4(d[0], d[1], d[2], d[3]);
-                    slope[(size_t)((c + q) / 4 + 1) * TROWS] = make_float4(d[4], d[5], d[6], d[7]);
-                }
+                for (int e = 0; e < 8; e++) v[e] = gelu_exact_tanh(v[e] + bias[0][c + e], d[e]);
+                put8(c, v);
+                slope[(size_t)(c / 4) * TROWS] = make_float4(d[0], d[1], d[2], d[3]);
+                slope[(size_t)(c / 4 + 1) * TROWS] = make_float4(d[4], d[5], d[6], d[7]);
             }
             operand(a.w.H1 + tile * H_IMAGE, H_IMAGE, true);
             // ---- layer 2: H2 = GELU(Z2), its slope in the accumulator's place
             result();
 #pragma unroll 1
-            for (int c = c0; c < c0 + 64; c += 32) {
-                float v[32];
-                tmem_ld32(acc + (uint32_t)(T_HID + c), v);
+            for (int c = c0; c < c0 + 64; c += 8) {
+                float v[8], d[8];
+                tmem_ld8(acc + (uint32_t)(T_HID + c), v);
 #pragma unroll
-                for (int q = 0; q < 32; q += 8) {
-                    float h[8];
-#pragma unroll
-                    for (int e = 0; e < 8; e++) {
-                        float d;
-                        h[e] = gelu_exact_tanh(v[q + e] + bias[1][c + q + e], d);
-                        v[q + e] = d;
-                    }
-                    put8(c + q, h);
-                }
-                tmem_st32(acc + (uint32_t)(T_HID + c), v);
+                for (int e = 0; e < 8; e++) v[e] = gelu_exact_tanh(v[e] + bias[1][c + e], d[e]);
+                put8(c, v);
+                tmem_st8(acc + (uint32_t)(T_HID + c), d);
             }
             tmem_wait_st();
             operand(a.w.H2 + tile * H_IMAGE, H_IMAGE, true);
             // ---- layer 3: H3 in registers, its slope in the accumulator's place
             result();
+            // (through this thread's own slots of the free operand buffer, so that one short loop
+            // holds the GELU: unrolled over the registers its code overflows the instruction cache)
             float h3[64];
+            float *slots = reinterpret_cast<float *>(sA) + group * 32 * TROWS + r;
 #pragma unroll
             for (int half = 0; half < 2; half++) {
-                float v[32];
-                const int c = c0 + 32 * half;
-                tmem_ld32(acc + (uint32_t)c, v);
+#pragma unroll 1
+                for (int c = 0; c < 32; c += 8) {
+                    const int col = c0 + 32 * half + c;
+                    float v[8], d[8];
+                    tmem_ld8(acc + (uint32_t)col, v);
 #pragma unroll
-                for (int e = 0; e < 32; e++) {
-                    float d;
-                    h3[32 * half + e] = gelu_exact_tanh(v[e] + bias[2][c + e], d);
-                    v[e] = d;
+                    for (int e = 0; e < 8; e++)
+                        slots[(c + e) * TROWS] = gelu_exact_tanh(v[e] + bias[2][col + e], d[e]);
+                    tmem_st8(acc + (uint32_t)col, d);
                 }
-                tmem_st32(acc + (uint32_t)c, v);
+#pragma unroll
+                for (int e = 0; e < 32; e++) h3[32 * half + e] = slots[e * TROWS];
             }
             tmem_wait_st();
             // layer 4: each row's three sums run over the 256 units in order, so the four column
@@ -448,10 +449,9 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) tile_kernel(const TileArgs a)
                 sums[SUM_DB4 + tid] = ((colSum[0][tid] + colSum[1][tid]) + colSum[2][tid]) + colSum[3][tid];
             named_sync(1, ROW_THREADS);
             // ---- dZ3 = (dO W4) GELU'(Z3)
-#pragma unroll
-            for (int half = 0; half < 2; half++) {
+#pragma unroll 1
+            for (int c = c0; c < c0 + 64; c += 32) {
                 float v[32];
-                const int c = c0 + 32 * half;
                 tmem_ld32(acc + (uint32_t)c, v);
 #pragma unroll
                 for (int e = 0; e < 32; e++) {
@@ -531,7 +531,8 @@ struct GradArgs {
 // Unit u over the tiles of its range: partial = sum over rows of dZ[row][m] V[row][n]. Both operands
 // are the tiles' images read along their rows (MN-major: 64 units per 128-byte row, 8 rows per 1024
 // bytes, the next 64 units one K-block further), two tiles in flight. Bound by the copies of the
-// images from L2 (96 KB for 8 MMAs).
+// images from L2 (96 KB for 8 MMAs): 16.5 us at 16,384 rows (four GEMMs with staged operands before:
+// 169 us and their split sums 42 us).
 __global__ void __launch_bounds__(GRAD_THREADS, 1) weight_grad_kernel(const GradArgs a) {
     using namespace umma;
     extern __shared__ uint8_t dynSmem[];

@@ -165,6 +165,25 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     for (int c = 0; c < 32; c++) v[c] = __uint_as_float(r[c]);
 }
 
+// 8 consecutive FP32 columns of this thread's TMEM lane (warp-collective).
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+                   "=r"(r[7])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int c = 0; c < 8; c++) v[c] = __uint_as_float(r[c]);
+}
+
+// 8 consecutive FP32 columns of this thread's TMEM lane from registers; completes at tmem_wait_st.
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr),
+                 "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+}
+
 // 32 consecutive FP32 columns of this thread's TMEM lane from registers (warp-collective); the
 // store completes at tmem_wait_st.
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float *v) {
