@@ -126,3 +126,24 @@ def test_reference_arithmetic_on_subnormal_and_fill_values(cuda_device):
     assert np.array_equal(got["health"] > 0, want["health"] > 0)
     for name in ("k", "j", "i"):
         assert np.array_equal(got[name], want[name], equal_nan=True), name
+
+
+# one slab, five slabs and the ramp in the FP32 step; one and two slabs in the reference arithmetic
+@pytest.mark.parametrize("n,arithmetic", [(393215, "fp32"), (393216, "fp32"), (2999999, "fp32"),
+                                          (3000000, "fp32"), (393216, "reference"),
+                                          (2097152, "reference")])
+def test_host_buffer_slabs_at_the_edges_of_their_rule(cuda_device, n, arithmetic):
+    win = syn.config1_window(n_frames=2, eta=16, xi=17, s_rho=6)
+    win.times[1] = win.times[0] + 300.0
+    p = mixed_records(n, win, 3)
+    with Engine(0, arithmetic=arithmetic, rng="philox") as engine:
+        engine.load_window(win)
+        engine.set_config(default_config(random=True))
+        engine.set_particles(p)
+        engine.concentration_reset(2)
+        engine.move_interval(0)
+        resident, counts = engine.get_particles(), engine.concentration()
+        engine.concentration_reset(2)
+        engine.move_interval_host(0, p)
+        assert p.tobytes() == resident.tobytes()
+        assert np.array_equal(engine.concentration(), counts)

@@ -1334,14 +1334,26 @@ int wacomm_b200_move_interval_host(wacomm_b200_context *ctx, int time_index,
     if ((rc = grow(ctx, ctx->dAos, ctx->aosCap, n))) return rc;
     ctx->n = n;
     // Slabs: the upload of slab s+1 and the download of slab s-1 overlap the move of slab s. Only
-    // the first upload and the last download are exposed, so the end slabs are small (1/32 of the
-    // records) and the slabs double from there (1/16, 1/8) up to pieces of at most 4 M records in
-    // the middle: a slab's move (about 3 ns per record) outlasts the copy of a neighbour twice its
-    // size (about 1.2 ns per record each way over PCIe), so the compute never waits for a copy.
+    // the first upload and the last download are exposed, so the end slabs are small.
+    //  * From 3 M records on, 1/32 of the records at each end and the slabs double from there (1/16,
+    //    1/8) up to pieces of at most 4 Mi in the middle: a slab's move (about 3 ns per record)
+    //    outlasts the copy of a neighbour twice its size (about 1.2 ns per record each way over PCIe),
+    //    so the compute never waits for a copy.
+    //  * From 384 Ki on, five slabs of 1, 4, 4, 4 and 1 fourteenths: smaller end slabs or more of them
+    //    leave the chip idle in the latency of their last waves. Host interval with one slab (two
+    //    from 2 Mi) / with five: 400,000 records 2.22 / 1.89 ms (deterministic, FP16 storage) and
+    //    3.72 / 3.54 ms (random walk), 1.5 M 7.5 / 5.3 and 12.9 / 10.4 ms; 3.1 M by the ramp 12.1 /
+    //    9.9 and 23.1 / 21.3 ms. Below, the copies are shorter than what the slabs lose (262,144
+    //    records with the random walk 2.50 / 2.52 ms).
+    //  * The reference arithmetic moves a record in ten times its copies' time: one slab, two from 2 Mi
+    //    and the ramp from 4 Mi (600,000 records with five slabs: 8.9 -> 9.6 ms).
     std::vector<size_t> bounds{0};
-    if (n >= ((size_t)4 << 20)) {
+    int ordered = 1;  // slabs at the end that run one after the other on the main lane
+    const bool fp32 = ctx->opt.arithmetic == WACOMM_B200_ARITH_FP32;
+    if (n >= (fp32 ? 3000000 : (size_t)4 << 20)) {
         const size_t e = n / 32, ramp = 7 * e, rest = n - 2 * ramp;
-        const size_t pieces = (rest + ((size_t)4 << 20) - 1) / ((size_t)4 << 20);
+        const size_t pieces =
+            std::max<size_t>(2, (rest + ((size_t)4 << 20) - 1) / ((size_t)4 << 20));
         bounds.push_back(e);
         bounds.push_back(3 * e);
         bounds.push_back(ramp);
@@ -1349,11 +1361,13 @@ int wacomm_b200_move_interval_host(wacomm_b200_context *ctx, int time_index,
         bounds.push_back(n - ramp);
         bounds.push_back(n - 3 * e);
         bounds.push_back(n - e);
-        bounds.push_back(n);
-    } else {
-        const size_t pieces = n >= ((size_t)2 << 20) ? 2 : 1;
-        for (size_t q = 1; q <= pieces; q++) bounds.push_back(n * q / pieces);
+        ordered = 3;
+    } else if (!fp32) {
+        if (n >= ((size_t)2 << 20)) bounds.push_back(n / 2);
+    } else if (n >= ((size_t)384 << 10)) {
+        for (size_t q : {1, 5, 9, 13}) bounds.push_back(n * q / 14);
     }
+    bounds.push_back(n);
     const int slabs = (int)bounds.size() - 1;
     std::vector<cudaEvent_t> up(slabs), done(slabs);
     for (int s = 0; s < slabs; s++) {
@@ -1365,7 +1379,7 @@ int wacomm_b200_move_interval_host(wacomm_b200_context *ctx, int time_index,
     const bool walk = sorts && ctx->seqBounds == bounds;
     if (sorts) ctx->seqBounds.clear();
     CUDA_TRY(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
-    // Slab s runs on compute lane s % 2 (LaneSwap), the last two on the main lane: the next
+    // Slab s runs on compute lane s % 2 (LaneSwap), the last `ordered` on the main lane: the next
     // slab's conversion, sort and move fill the SMs that the previous slab's move releases in its
     // last wave. The second lane starts after the work enqueued so far on the main stream (the
     // forcing pair of the interval).
@@ -1382,13 +1396,13 @@ int wacomm_b200_move_interval_host(wacomm_b200_context *ctx, int time_index,
     for (int s = 0; s < slabs; s++) {
         size_t off = bounds[s], cnt = bounds[s + 1] - bounds[s];
         if (cnt == 0) continue;
-        // the ramp-down slabs (the last three) run on the main lane after both lanes are done,
-        // in order, so that each download overlaps the next slab's move
-        if (s == slabs - 3 && s > 0) {
+        // the ordered slabs run on the main lane after both lanes are done, so that each download
+        // overlaps the next slab's move
+        if (s == slabs - ordered && s > 0) {
             CUDA_TRY(ctx, cudaEventRecord(ctx->evLaneDone, ctx->stream2));
             CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->stream, ctx->evLaneDone, 0));
         }
-        LaneSwap lane(ctx, (s & 1) != 0 && s < slabs - 3);
+        LaneSwap lane(ctx, (s & 1) != 0 && s < slabs - ordered);
         CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->stream, up[s], 0));
         ParticleSoA S = offset_soa(ctx->S.s, off);
         CUDA_TRY(ctx, aos_to_soa(ctx->dAos + off, (int)cnt, S, ctx->stream));
