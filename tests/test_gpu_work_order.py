@@ -25,11 +25,12 @@ def mixed_records(n, win, seed):
     return p
 
 
-# 16 x 17 cells of 6 levels: 1,633 bins, told apart from 1,633 records on
-@pytest.mark.parametrize("n", [1, 31, 1632, 1633, 4099])
+# sorted from 37,889 records on; 64 x 65 cells of 10 levels: 41,601 bins, levels told apart from that
+# many records on
+@pytest.mark.parametrize("n", [1, 37888, 37889, 41600, 41601])
 @pytest.mark.parametrize("arithmetic,direction", [("fp32", 1), ("fp32", -1), ("reference", 1)])
 def test_records_do_not_depend_on_the_sort(cuda_device, n, arithmetic, direction):
-    win = syn.config1_window(n_frames=3, eta=16, xi=17, s_rho=6)
+    win = syn.config1_window(n_frames=3, eta=64, xi=65, s_rho=10)
     p = mixed_records(n, win, n)
     cfg = default_config(random=True, trackingDirection=direction, backwardDiffusion=1)
     got, counts = [], []
