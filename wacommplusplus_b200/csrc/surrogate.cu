@@ -126,8 +126,14 @@ struct CellArgs {
 };
 
 constexpr size_t CELL_SMEM = (size_t)CELL_KB * KBLOCK_A + 2 * (size_t)KBLOCK_W + 1024;
+constexpr int CELL_PARTS = 4, CELL_THREADS = CELL_PARTS * TILE;
 
-__global__ void __launch_bounds__(128, 1) surrogate_cell_kernel(const CellArgs a) {
+// Four threads per cell-level: each gathers one of the u, v blocks (64 values) of the two records and
+// half a w block, and sums its block's squared deviations for the gate from the same loads; warp w
+// then reads columns 64 (w / 4) .. of the accumulator. Bound by the gathers (the levels of a cell lie
+// in different planes). 161,290 cell-levels: 0.34 ms with one thread per cell-level and a second
+// pass of loads for the gate, 0.17 ms so (z, gates and corner records unchanged to the last bit).
+__global__ void __launch_bounds__(CELL_THREADS, 1) surrogate_cell_kernel(const CellArgs a) {
     using namespace umma;
     extern __shared__ uint8_t dynSmem[];
     uint8_t *sA = align1024(dynSmem);
@@ -136,7 +142,8 @@ __global__ void __launch_bounds__(128, 1) surrogate_cell_kernel(const CellArgs a
     __shared__ uint32_t tmemSlot;
     __shared__ int abortFlag;
     __shared__ float b1s[HID];
-    const int tid = threadIdx.x, warp = tid >> 5;
+    __shared__ float deviation[CELL_PARTS][TILE];  // squared deviations of the u, v blocks
+    const int tid = threadIdx.x, warp = tid >> 5, r = tid & (TILE - 1), part = tid / TILE;
     if (tid == 0) {
         for (int s = 0; s < 2; s++) {
             mbar_init(&full[s], 1);
@@ -147,7 +154,7 @@ __global__ void __launch_bounds__(128, 1) surrogate_cell_kernel(const CellArgs a
         fence_barrier_init();
     }
     const float *b1 = reinterpret_cast<const float *>(a.weights + OFF_B1);
-    for (int c = tid; c < HID; c += 128) b1s[c] = b1[c];
+    for (int c = tid; c < HID; c += CELL_THREADS) b1s[c] = b1[c];
     if (warp == 0) tmem_alloc(&tmemSlot, 256);
     fence_before_sync();
     __syncthreads();
@@ -160,66 +167,75 @@ __global__ void __launch_bounds__(128, 1) surrogate_cell_kernel(const CellArgs a
     int issued[2] = {-1, -1}, consumed[2] = {-1, -1};
     int it = 0;
     for (long long tile = blockIdx.x; tile < nTiles; tile += gridDim.x, it++) {
-        // ---- gather: thread = row = cell-level
-        const long long cl = tile * TILE + tid;
-        float gsum = 0.f;
-        if (cl < a.nCL) {
-            const int lev = (int)(cl % levels);
-            const long long cell = cl / levels;
-            const int j = (int)(cell / (a.xi - 1)), i = (int)(cell % (a.xi - 1));
-            const int kI = lev - (a.sW - 2);
-#pragma unroll 1
-            for (int q = 0; q < N_STENCIL / 8; q++) {
-                const int f = q * 8;
-                const int rec = f / 192, field = (f / 64) % 3, c = (f / 16) % 4, a0 = (f % 16) / 4;
-                const float *src = rec == 0 ? (field == 0 ? a.u0 : field == 1 ? a.v0 : a.w0)
-                                            : (field == 0 ? a.u1 : field == 1 ? a.v1 : a.w1);
-                const int nlev = field == 2 ? a.sW : a.sRho;
-                int L = kI - 2 + c;
-                L = L < -nlev + 1 ? -nlev + 1 : (L > 0 ? 0 : L);
-                L += nlev - 1;
-                const float scale = field == 2 ? W_FEATURE : 1.f;
-                float v[8];
+        // ---- gather
+        const long long cl = tile * TILE + r;
+        const bool live = cl < a.nCL;
+        const int lev = live ? (int)(cl % levels) : 0;
+        const long long cell = live ? cl / levels : 0;
+        const int j = (int)(cell / (a.xi - 1)), i = (int)(cell % (a.xi - 1));
+        const int kI = lev - (a.sW - 2);
+        int ii[4];
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            const int x = i - 1 + b;
+            ii[b] = x < 0 ? 0 : (x > a.xi - 1 ? a.xi - 1 : x);
+        }
+        // 8 values of a field (`levelsOf` levels): level c of the stencil, rows a0 and a0 + 1
+        auto gather8 = [&](const float *src, int levelsOf, int c, int a0, float (&v)[8]) {
+            int L = kI - 2 + c;
+            L = L < -levelsOf + 1 ? -levelsOf + 1 : (L > 0 ? 0 : L);
+            L += levelsOf - 1;
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                int jj = j - 1 + a0 + q;
+                jj = jj < 0 ? 0 : (jj > a.eta - 1 ? a.eta - 1 : jj);
+                const float *row = src + ((size_t)L * a.eta + jj) * a.xi;
+#pragma unroll
+                for (int b = 0; b < 4; b++) v[4 * q + b] = __ldg(row + ii[b]);
+            }
+        };
+        // features f .. f+7 of this row into the operand
+        auto put = [&](int f, const float (&v)[8], float scale) {
+            uint4 pk;
+            pk.x = pack_bf16(v[0] * scale, v[1] * scale);
+            pk.y = pack_bf16(v[2] * scale, v[3] * scale);
+            pk.z = pack_bf16(v[4] * scale, v[5] * scale);
+            pk.w = pack_bf16(v[6] * scale, v[7] * scale);
+            *reinterpret_cast<uint4 *>(sA + (f / 64) * KBLOCK_A + sw128_offset(r, f % 64)) = pk;
+        };
+        {
+            // block `part` of u0, v0, u1, v1 (features 0, 64, 192, 256 on), in order, its squared
+            // deviations from its node GATE_REF summed in the same order
+            const float *src = part == 0 ? a.u0 : part == 1 ? a.v0 : part == 2 ? a.u1 : a.v1;
+            const int first = part < 2 ? part * 64 : 192 + (part - 2) * 64;
+            float v[8], x0 = 0.f, sum = 0.f;
+            if (live) {
+                gather8(src, a.sRho, GATE_REF / 16, GATE_REF % 16 / 4 / 2 * 2, v);
+                x0 = v[GATE_REF % 8];
+            }
+#pragma unroll 2
+            for (int q = 0; q < 8; q++) {
+#pragma unroll
+                for (int e = 0; e < 8; e++) v[e] = 0.f;
+                if (live) gather8(src, a.sRho, q / 2, q % 2 * 2, v);
+                put(first + q * 8, v, 1.f);
 #pragma unroll
                 for (int e = 0; e < 8; e++) {
-                    int jj = j - 1 + a0 + e / 4, ii = i - 1 + e % 4;
-                    jj = jj < 0 ? 0 : (jj > a.eta - 1 ? a.eta - 1 : jj);
-                    ii = ii < 0 ? 0 : (ii > a.xi - 1 ? a.xi - 1 : ii);
-                    v[e] = __ldg(src + ((size_t)L * a.eta + jj) * a.xi + ii) * scale;
-                }
-                uint4 pk;
-                pk.x = pack_bf16(v[0], v[1]);
-                pk.y = pack_bf16(v[2], v[3]);
-                pk.z = pack_bf16(v[4], v[5]);
-                pk.w = pack_bf16(v[6], v[7]);
-                *reinterpret_cast<uint4 *>(sA + (f / 64) * KBLOCK_A + sw128_offset(tid, f % 64)) = pk;
-            }
-            // uniformity gate from the FP32 forcing: squared deviations of the u and v blocks of
-            // both records from each block's node GATE_REF
-            auto node = [&](const float *src, int n) {
-                int lv = kI - 2 + n / 16;
-                lv = lv < -a.sRho + 1 ? -a.sRho + 1 : (lv > 0 ? 0 : lv);
-                lv += a.sRho - 1;
-                int jj = j - 1 + (n % 16) / 4, ii = i - 1 + n % 4;
-                jj = jj < 0 ? 0 : (jj > a.eta - 1 ? a.eta - 1 : jj);
-                ii = ii < 0 ? 0 : (ii > a.xi - 1 ? a.xi - 1 : ii);
-                return __ldg(src + ((size_t)lv * a.eta + jj) * a.xi + ii);
-            };
-            const float *blocks[4] = {a.u0, a.v0, a.u1, a.v1};
-#pragma unroll 1
-            for (int blk = 0; blk < 4; blk++) {
-                const float x0 = node(blocks[blk], GATE_REF);
-                float sum = 0.f;
-                for (int n = 0; n < 64; n++) {
-                    const float d = node(blocks[blk], n) - x0;
+                    const float d = v[e] - x0;
                     sum = fmaf(d, d, sum);
                 }
-                gsum += sum;
             }
-        } else {
-            const uint4 zero = make_uint4(0, 0, 0, 0);
-            for (int q = 0; q < N_STENCIL / 8; q++)
-                *reinterpret_cast<uint4 *>(sA + (q * 8 / 64) * KBLOCK_A + sw128_offset(tid, (q * 8) % 64)) = zero;
+            deviation[part][r] = live ? sum : 0.f;
+            // half of w0 (features 128 on) or w1 (320 on)
+            const float *w = part < 2 ? a.w0 : a.w1;
+            const int firstW = part < 2 ? 128 : 320;
+#pragma unroll 2
+            for (int q = (part & 1) * 4; q < (part & 1) * 4 + 4; q++) {
+#pragma unroll
+                for (int e = 0; e < 8; e++) v[e] = 0.f;
+                if (live) gather8(w, a.sW, q / 2, q % 2 * 2, v);
+                put(firstW + q * 8, v, W_FEATURE);
+            }
         }
         fence_async_shared();
         fence_before_sync();
@@ -260,12 +276,12 @@ __global__ void __launch_bounds__(128, 1) surrogate_cell_kernel(const CellArgs a
         mbar_wait(&accFull, it & 1, &abortFlag);
         __syncwarp();
         fence_after_sync();
-        // ---- epilogue: z = acc + b1 (FP16), gate
-        const bool write = cl < a.nCL && !abortFlag;
+        // ---- epilogue: z = acc + b1 (FP16), this part's 64 columns of the row
+        const bool write = live && !abortFlag;
 #pragma unroll 1
-        for (int c0 = 0; c0 < HID; c0 += 32) {
+        for (int c0 = part * 64; c0 < part * 64 + 64; c0 += 32) {
             float v[32];
-            tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+            tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
             if (write) {
                 uint4 *dst = reinterpret_cast<uint4 *>(a.z + (size_t)cl * HID + c0);
 #pragma unroll
@@ -283,37 +299,44 @@ __global__ void __launch_bounds__(128, 1) surrogate_cell_kernel(const CellArgs a
                 }
             }
         }
+        // the corner record in pieces of one or two fields per part
         if (write) {
-            const int lev = (int)(cl % levels);
-            const long long cell = cl / levels;
-            const int j = (int)(cell / (a.xi - 1)), i = (int)(cell % (a.xi - 1));
-            const int kI = lev - (a.sW - 2);
             const size_t plane = (size_t)a.eta * a.xi, c00 = (size_t)j * a.xi + i;
             const size_t corner[4] = {c00, c00 + a.xi, c00 + a.xi + 1, c00 + 1};
             const size_t lr = (size_t)(kI + a.sRho - 1) * plane, lu = (size_t)(kI + a.sW - 1) * plane,
                          ll = (size_t)(kI + a.sW - 2) * plane;
-            CellCorners c;
+            CellCorners *c = a.corners + cl;
+            auto fields = [&](const float *f0, const float *f1, size_t at, float (*out)[4]) {
+                float v[2][4];
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                c.u[0][q] = a.u0[lr + corner[q]];
-                c.u[1][q] = a.u1[lr + corner[q]];
-                c.v[0][q] = a.v0[lr + corner[q]];
-                c.v[1][q] = a.v1[lr + corner[q]];
-                c.wU[0][q] = a.w0[lu + corner[q]];
-                c.wU[1][q] = a.w1[lu + corner[q]];
-                c.wL[0][q] = a.w0[ll + corner[q]];
-                c.wL[1][q] = a.w1[ll + corner[q]];
-                c.zeta[0][q] = a.z0[corner[q]];
-                c.zeta[1][q] = a.z1[corner[q]];
-                c.h[q] = (float)a.h[corner[q]];
+                for (int q = 0; q < 4; q++) {
+                    v[0][q] = __ldg(f0 + at + corner[q]);
+                    v[1][q] = __ldg(f1 + at + corner[q]);
+                }
+                float4 *dst = reinterpret_cast<float4 *>(out);
+                dst[0] = make_float4(v[0][0], v[0][1], v[0][2], v[0][3]);
+                dst[1] = make_float4(v[1][0], v[1][1], v[1][2], v[1][3]);
+            };
+            if (part == 0) {
+                fields(a.u0, a.u1, lr, c->u);
+                const CellMetric m = a.metric[c00];
+                c->invXdist = 1.0 / m.x;
+                c->invYdist = 1.0 / m.y;
+            } else if (part == 1) {
+                fields(a.v0, a.v1, lr, c->v);
+                fields(a.z0, a.z1, 0, c->zeta);
+            } else if (part == 2) {
+                fields(a.w0, a.w1, lu, c->wU);
+                *reinterpret_cast<float4 *>(c->h) =
+                    make_float4((float)a.h[corner[0]], (float)a.h[corner[1]], (float)a.h[corner[2]],
+                                (float)a.h[corner[3]]);
+            } else {
+                fields(a.w0, a.w1, ll, c->wL);
+                const float gsum = ((deviation[0][r] + deviation[1][r]) + deviation[2][r]) + deviation[3][r];
+                c->depth = a.depthIntervals[kI + a.sW - 2];
+                c->sigma = sqrtf(gsum / 256.f);
+                c->gate = fminf(sqrtf(gsum / 256.f) / GATE_SIGMA, 1.f);
             }
-            const CellMetric m = a.metric[c00];
-            c.invXdist = 1.0 / m.x;
-            c.invYdist = 1.0 / m.y;
-            c.depth = a.depthIntervals[kI + a.sW - 2];
-            c.sigma = sqrtf(gsum / 256.f);
-            c.gate = fminf(c.sigma / GATE_SIGMA, 1.f);
-            a.corners[cl] = c;
         }
         fence_before_sync();
         __syncthreads();
@@ -1407,7 +1430,7 @@ cudaError_t surrogate_cells(int eta, int xi, int sW, int sRho, const FrameDevice
     if (e != cudaSuccess) return e;
     long long tiles = (a.nCL + TILE - 1) / TILE;
     int blocks = (int)(tiles < smCount ? tiles : smCount);
-    surrogate_cell_kernel<<<blocks, 128, CELL_SMEM, stream>>>(a);
+    surrogate_cell_kernel<<<blocks, CELL_THREADS, CELL_SMEM, stream>>>(a);
     return cudaGetLastError();
 }
 
