@@ -408,7 +408,7 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
         if (diffuse) {
             const float aa = akt_at_cell(C, startColumn, alpha, kF, jF, iF);
             float sigmaDepth = (float)(cfg.sigma * (1 - p.k * P.invKLower));
-            float scale = sqrtf(dt / dtiF);
+            const float scale = dt == dtiF ? 1.f : sqrtf(dt / dtiF);
             float n0, n1, n2;
             if (drawn) {
                 n0 = normals.x;
@@ -418,9 +418,9 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
                 philox_normals3(philoxKey, P.intervalKey, (uint64_t)__double_as_longlong(elapsed),
                                 n0, n1, n2);
             } else {
-                n0 = (float)prefix_normal(stepKey, 0);
-                n1 = (float)prefix_normal(stepKey, 1);
-                n2 = (float)prefix_normal(stepKey, 2);
+                n0 = prefix_normal_f32(stepKey, 0);
+                n1 = prefix_normal_f32(stepKey, 1);
+                n2 = prefix_normal_f32(stepKey, 2);
             }
             const float2 rxy = __fmul2_rn(
                 __fmul2_rn(make_float2(sigmaDepth, sigmaDepth), make_float2(n0, n1)),

@@ -444,8 +444,8 @@ __global__ void __launch_bounds__(256) draw_normals_kernel(const uint64_t *id, u
          e += (size_t)gridDim.x * blockDim.x) {
         const unsigned s = (unsigned)(e / count), slot = (unsigned)(e - (size_t)s * count);
         const uint64_t key = key_prefix(seed, id[slot], interval, s);
-        out[e] = make_float4((float)prefix_normal(key, 0), (float)prefix_normal(key, 1),
-                             (float)prefix_normal(key, 2), 0.f);
+        out[e] = make_float4(prefix_normal_f32(key, 0), prefix_normal_f32(key, 1),
+                             prefix_normal_f32(key, 2), 0.f);
     }
 }
 
