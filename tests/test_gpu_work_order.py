@@ -16,7 +16,7 @@ def mixed_records(n, win, seed):
     rng = np.random.default_rng(seed)
     p = syn.uniform_particles(n, win.eta, win.xi, seed=seed, time=win.times[0])
     p["k"] = rng.uniform(-win.sRho + 0.5, 0.5, n)
-    p["time"] += rng.choice([0.0, 1700.0, 3600.0, 9000.0], n)
+    p["time"] += rng.choice([0.0, 130.0, 1700.0, 3600.0, 4444.4, 9000.0, 10799.9], n)
     kind = rng.integers(0, 12, n)
     p["health"][kind == 0] = -1.0
     p["health"][kind == 1] = 1e-7
@@ -26,11 +26,12 @@ def mixed_records(n, win, seed):
 
 
 # sorted from 37,889 records on; 64 x 65 cells of 10 levels: 41,601 bins, levels told apart from that
-# many records on
-@pytest.mark.parametrize("n", [1, 37888, 37889, 41600, 41601])
+# many records on, release times in up to four parts; in up to sixteen on 16 x 17 cells
+@pytest.mark.parametrize("n,eta,xi", [(1, 64, 65), (37888, 64, 65), (37889, 64, 65), (41600, 64, 65),
+                                      (41601, 64, 65), (90000, 16, 17)])
 @pytest.mark.parametrize("arithmetic,direction", [("fp32", 1), ("fp32", -1), ("reference", 1)])
-def test_records_do_not_depend_on_the_sort(cuda_device, n, arithmetic, direction):
-    win = syn.config1_window(n_frames=3, eta=64, xi=65, s_rho=10)
+def test_records_do_not_depend_on_the_sort(cuda_device, n, eta, xi, arithmetic, direction):
+    win = syn.config1_window(n_frames=4, eta=eta, xi=xi, s_rho=10)
     p = mixed_records(n, win, n)
     cfg = default_config(random=True, trackingDirection=direction, backwardDiffusion=1)
     got, counts = [], []

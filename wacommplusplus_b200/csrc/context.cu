@@ -521,7 +521,7 @@ PackedArgs packed_args(wacomm_b200_context *ctx) {
 
 // Histogram, offsets and scan scratch of the cell sort of `count` records.
 int reserve_sort(wacomm_b200_context *ctx, size_t count) {
-    size_t bins = sort_bins(ctx->eta, ctx->xi, ctx->sRho, count).count();
+    size_t bins = sort_bins(ctx->eta, ctx->xi, ctx->sRho, count, ctx->cfg.trackingDirection > 0).count();
     if (ctx->binsCap < bins + 2 || !ctx->dHist || !ctx->dOffsets) {
         cudaFree(ctx->dHist);
         cudaFree(ctx->dOffsets);
@@ -541,8 +541,11 @@ int reserve_sort(wacomm_b200_context *ctx, size_t count) {
 int sort_work(wacomm_b200_context *ctx, const IntervalParams &P, const ParticleSoA &S, size_t count,
               uint32_t *keys, uint32_t *order, const uint32_t *seqIn, uint32_t *seqOut,
               int &launches) {
-    SortBins bins = sort_bins(ctx->eta, ctx->xi, ctx->sRho, count);
-    if (P.direction > 0) bins.idleTime = P.start + P.length;  // backward tracking releases all
+    SortBins bins = sort_bins(ctx->eta, ctx->xi, ctx->sRho, count, P.direction > 0);
+    if (P.direction > 0) {  // backward tracking releases all
+        bins.start = P.start;
+        bins.end = P.start + P.length;
+    }
     int rc;
     if ((rc = reserve_sort(ctx, count))) return rc;
     CUDA_TRY(ctx, sort_by_cell(S, (int)count, bins, seqIn, keys, ctx->dHist, ctx->dOffsets,
