@@ -209,3 +209,24 @@ def test_geo_positions_match_oracle(engine):
     off = dep == 1e37
     assert 0 < off.sum() < n  # both branches exercised
     assert np.all(off[200:210])
+
+
+# the schedules of up to 256 sources are held in shared memory; spacings far below the time's last
+# place (rates of 1e9 per hour around 1.6e9 s) give runs of equal times that the rate cannot index
+@pytest.mark.parametrize("count,rate", [(255, 40.0), (256, 40.0), (257, 40.0), (3, 7.0e10)])
+def test_ranks_from_the_rate_match_the_oracle(engine, count, rate):
+    cfg = default_config()
+    engine.set_config(cfg)
+    engine.set_particles(make_particles(0))
+    rng = np.random.default_rng(count)
+    t0 = 19000.0 * DAY
+    length = 3600.0 if rate < 1e6 else 1.0e-3
+    starts = t0 + rng.choice([-7200.0, -5000.5, -100.25, 0.0], count) + rng.integers(0, 4, count) * 0.5
+    if rate > 1e6:
+        starts[:] = t0
+    src = make_sources([(-0.1, 4.5, 5.5, s / DAY, -1, rate * f, "uniform_rate")
+                        for s, f in zip(starts, rng.choice([1.0, 1.0, 0.37, 3.3], count))])
+    n = engine.emit(src, t0, t0 + length)
+    want = ob.sources_emit(cfg, src, 0.0, t0, t0 + length, 0)
+    assert n == len(want) > 0
+    assert same_records(engine.get_particles(), want, position_ulps=0)
