@@ -231,7 +231,9 @@ cudaError_t launch_move_fast(const wacomm_b200_config &cfg, const IntervalParams
     spread_launch(L.count, LaunchShape<SHAPE>::threads, M.lanes, threads);
     const long long items = (long long)(threads / 32) * M.lanes * (L.perThread > 1 ? L.perThread : 1);
     const int blocks = (int)((L.count + items - 1) / items);
-    move_fast_kernel<SEM, STORE, SHAPE, VARIANT><<<blocks, threads, 0, stream>>>(cfg, P, F, S, M);
+    FastView<STORE> G = F;
+    G.X.K = step_constants(cfg, P, F.V.g.eta, F.V.g.xi);
+    move_fast_kernel<SEM, STORE, SHAPE, VARIANT><<<blocks, threads, 0, stream>>>(cfg, P, G, S, M);
     return cudaGetLastError();
 }
 

@@ -16,7 +16,34 @@
 
 namespace wb {
 
+// Constants of a launch in the precision the step uses them in, computed on the host: read as constant
+// operands, where a conversion of the FP64 parameter would cost a register over the substep loop or,
+// repeated in it, a quarter-rate instruction (4.2 M records, lean: 9.96 -> 9.80 ms, FP16 storage 10.50 ->
+// 10.29 ms).
+struct StepConstants {
+    double jEdge, iEdge;  // last node of each axis
+    double invLength;     // 1 / length of the interval (0 for an empty one)
+    double ageSafe;       // age below which the lazy survival tests cannot change their outcome
+    float dti, sv, shore, direction, crid;
+};
+
+inline StepConstants step_constants(const wacomm_b200_config &cfg, const IntervalParams &P, int eta,
+                                    int xi) {
+    StepConstants K;
+    K.jEdge = eta - 1;
+    K.iEdge = xi - 1;
+    K.invLength = P.length == 0 ? 0.0 : 1.0 / P.length;
+    K.ageSafe = fmin(P.ageKillLo, P.ageUnder);
+    K.dti = (float)cfg.dti;
+    K.sv = (float)cfg.sv;
+    K.shore = (float)cfg.shoreLimit;
+    K.direction = (float)P.direction;
+    K.crid = (float)cfg.crid;
+    return K;
+}
+
 struct FastExtras {
+    StepConstants K;
     const float2 *invMetric;     // [eta][xi] {1/xdist, 1/ydist}
     const float *depthIntervals; // [sW-1]
     const wacomm_b200_config *cfgDevice;  // device copy of the run parameters
@@ -125,12 +152,12 @@ __device__ __forceinline__ float akt_at_cell(const CellView<STORE> &C, uint32_t 
     return fmaf(al - au, kF, au);
 }
 
-// Whether a position lies in the interpolation cells of an axis of `nodes` nodes: the cell
-// floor(x) has floor(x) >= 0 and floor(x) + 1 < nodes. Under the device rules a NaN counts as cell
+// Whether a position lies in the interpolation cells of an axis whose last node is `edge`: the cell
+// floor(x) has floor(x) >= 0 and floor(x) + 1 <= edge. Under the device rules a NaN counts as cell
 // 0 (to_index).
 template <int SEM>
-__device__ __forceinline__ bool on_axis(double x, double nodes) {
-    return SEM == SEM_HOST ? (x >= 0.0 && x < nodes - 1.0) : !(x < 0.0) && !(x >= nodes - 1.0);
+__device__ __forceinline__ bool on_axis(double x, double edge) {
+    return SEM == SEM_HOST ? (x >= 0.0 && x < edge) : !(x < 0.0) && !(x >= edge);
 }
 
 // Cell index and fraction of a position on the axis (on_axis).
@@ -266,12 +293,10 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
                                   double &elapsed, int *err) {
     const PackedView &V = F.V;
     const CellView<STORE> &C = F.C;
-    const int eta = V.g.eta, xi = V.g.xi, sW = V.g.sW;
+    const StepConstants &K = F.X.K;
+    const int xi = V.g.xi, sW = V.g.sW;
     const double kLower = P.kLower, length = P.length;
-    const double invLength = length == 0 ? 0.0 : 1.0 / length;
     const int direction = P.direction;
-    const float dirf = (float)direction, dtiF = (float)cfg.dti;
-    const float sv = (float)cfg.sv, shore = (float)cfg.shoreLimit;
     const bool midpoint = cfg.integrator == INTEGRATOR_MIDPOINT;
     constexpr bool canDiffuse = VARIANT != VAR_LEAN, full = VARIANT == VAR_FULL;
     constexpr bool canDrift = VARIANT == VAR_DRIFT || full, drawn = VARIANT == VAR_DRAWN;
@@ -285,7 +310,6 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
     // min(ageKillLo, ageUnder): neither dead nor without health), counted when the particle turns
     // lazy, two substeps short of the bound for rounding; skipped while it lasts and no closure
     // has ended the lazy tracking.
-    const double ageSafe = fmin(P.ageKillLo, P.ageUnder);
     int youngLeft = 0;
 
     if (P.firstChunk) {
@@ -330,7 +354,7 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
     while (elapsed < stop) {
         const double left = length - elapsed;
         double stepDt = cfg.dti;
-        float dt = dtiF;
+        float dt = K.dti;
         if (left < cfg.dti) {
             stepDt = left;
             dt = (float)stepDt;
@@ -351,7 +375,7 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
         const int kI = split_level<SEM>(p.k, kF);
         bool valid = !(SEM == SEM_DEVICE && (kI > 0 || kI <= -sW + 1));
         if (!haveCarried) {
-            valid = valid && on_axis<SEM>(p.j, eta) && on_axis<SEM>(p.i, xi);
+            valid = valid && on_axis<SEM>(p.j, K.jEdge) && on_axis<SEM>(p.i, K.iEdge);
             if (valid) {
                 jI = split_axis<SEM>(p.j, jF);
                 iI = split_axis<SEM>(p.i, iF);
@@ -378,9 +402,9 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
         } else if ((diffuse && !philox) || jibe) {
             stepKey = fold(prefix, (uint64_t)floor(elapsed / cfg.dti));
         }
-        const float alpha = (float)((elapsed + 0.5 * stepDt) * invLength);
+        const float alpha = (float)((elapsed + 0.5 * stepDt) * K.invLength);
         const float hc = here.height(alpha);
-        if (hc <= shore && cfg.horizontalClosure == CLOSURE_KILL) {
+        if (hc <= K.shore && cfg.horizontalClosure == CLOSURE_KILL) {
             p.health = -1;
             lazy = false;
             if (SEM == SEM_DEVICE) {
@@ -393,7 +417,7 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
         const uint32_t startColumn = startCell * (uint32_t)sW + (uint32_t)(kM + sW - 1);
         const float2 inv = metric;
         const float depthHere = __ldg(F.X.depthIntervals + (kM + sW - 2));
-        const float sa = midpoint ? (float)(elapsed * invLength) : alpha;
+        const float sa = midpoint ? (float)(elapsed * K.invLength) : alpha;
         float uu, vv, ww;
         keep_column(startColumn);
         current_at(kept, sa, kF, jF, iF, uu, vv, ww);
@@ -408,7 +432,7 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
         if (diffuse) {
             const float aa = akt_at_cell(C, startColumn, alpha, kF, jF, iF);
             float sigmaDepth = (float)(cfg.sigma * (1 - p.k * P.invKLower));
-            const float scale = dt == dtiF ? 1.f : sqrtf(dt / dtiF);
+            const float scale = dt == K.dti ? 1.f : sqrtf(dt / K.dti);
             float n0, n1, n2;
             if (drawn) {
                 n0 = normals.x;
@@ -427,18 +451,19 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
                 make_float2(scale, scale));
             rx = rxy.x;
             ry = rxy.y;
-            rz = sigmaDepth * n2 * aa * (float)cfg.crid * scale;
+            rz = sigmaDepth * n2 * aa * K.crid * scale;
         }
         const float zdist = hc * depthHere;
         const float rzdist = __frcp_rn(zdist);
         // index increments (i, j) and the vertical leap in metres
         float dI, dJ, zleap;
         if (midpoint) {
-            float kHalf = dirf * (sv + ww) * 0.5f * dt;
+            float kHalf = K.direction * (K.sv + ww) * 0.5f * dt;
             if (fabsf(kHalf) > zdist) kHalf = signf_of(zdist, kHalf);
-            // (dirf u 0.5 dt) / dx for i and j as one packed FP32x2 chain (the same roundings)
+            // (direction u 0.5 dt) / dx for i and j as one packed FP32x2 chain (the same roundings)
             const float2 half = __fmul2_rn(
-                __fmul2_rn(__fmul2_rn(make_float2(dirf * uu, dirf * vv), make_float2(0.5f, 0.5f)),
+                __fmul2_rn(__fmul2_rn(make_float2(K.direction * uu, K.direction * vv),
+                                      make_float2(0.5f, 0.5f)),
                            make_float2(dt, dt)),
                 inv);
             const double iMid = p.i + (double)half.x;
@@ -450,13 +475,13 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
             float2 im = inv;
             float um, vm, wm;
             bool moved = false;  // the lean form's lanes whose midpoint left the kept column
-            bool midValid = on_axis<SEM>(jMid, eta) && on_axis<SEM>(iMid, xi);
+            bool midValid = on_axis<SEM>(jMid, K.jEdge) && on_axis<SEM>(iMid, K.iEdge);
             if (midValid) {
                 float jf, if_;
                 const int j = split_axis<SEM>(jMid, jf), i = split_axis<SEM>(iMid, if_);
                 keep_cell((uint32_t)(j * xi + i));
                 hcMid = surface_from(surf, jf, if_).height(alpha);
-                midValid = hcMid > shore && hcMid > 0.f;
+                midValid = hcMid > K.shore && hcMid > 0.f;
                 if (midValid) {
                     jMI = j;
                     iMI = i;
@@ -485,10 +510,10 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
                 vm += dv;
             }
             const float2 d = __fmul2_rn(
-                __fmul2_rn(make_float2(dirf * um, dirf * vm), make_float2(dt, dt)), im);
+                __fmul2_rn(make_float2(K.direction * um, K.direction * vm), make_float2(dt, dt)), im);
             dI = d.x;
             dJ = d.y;
-            float detZ = dirf * (sv + wm) * dt;
+            float detZ = K.direction * (K.sv + wm) * dt;
             if (midValid) {
                 const float zdistMid =
                     hcMid * (kMI == kM ? depthHere : __ldg(F.X.depthIntervals + (kMI + sW - 2)));
@@ -498,9 +523,9 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
             dJ += ry * inv.y;
             zleap = detZ + rz;
         } else {
-            dI = (dirf * uu * dt + rx) * inv.x;
-            dJ = (dirf * vv * dt + ry) * inv.y;
-            zleap = dirf * (sv + ww) * dt + rz;
+            dI = (K.direction * uu * dt + rx) * inv.x;
+            dJ = (K.direction * vv * dt + ry) * inv.y;
+            zleap = K.direction * (K.sv + ww) * dt + rz;
         }
         if (fabsf(zleap) > zdist) zleap = signf_of(zdist, zleap);
         double jdet = p.j + (double)dJ;
@@ -510,12 +535,12 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
         if (kdet < kLower) close_lower(cfg, kLower, kdet, p.health, lazy);
 
         haveCarried = false;
-        if (on_axis<SEM>(jdet, eta) && on_axis<SEM>(idet, xi)) {
+        if (on_axis<SEM>(jdet, K.jEdge) && on_axis<SEM>(idet, K.iEdge)) {
             float jf, if_;
             const int jdetI = split_axis<SEM>(jdet, jf), idetI = split_axis<SEM>(idet, if_);
             keep_cell((uint32_t)(jdetI * xi + idetI));
             const SurfaceSums there = surface_from(surf, jf, if_);
-            if (there.height(alpha) <= shore) {
+            if (there.height(alpha) <= K.shore) {
                 if (cfg.horizontalClosure == CLOSURE_CONSTRAINT) {
                     idet = p.i;
                     jdet = p.j;
@@ -526,7 +551,7 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
                     idet = reflect_cell(p.i, iI, idet, idetI);
                     jdet = reflect_cell(p.j, jI, jdet, jdetI);
                 }
-            } else if (there.height(alpha) > shore) {
+            } else if (there.height(alpha) > K.shore) {
                 // the next step starts here
                 here = there;
                 jI = jdetI;
@@ -545,8 +570,8 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
                 p.health = -1;
                 lazy = false;
             } else if (cfg.horizontalClosure == CLOSURE_REFLECTION) {
-                p.i = reflect_domain(idet, xi - 1);
-                p.j = reflect_domain(jdet, eta - 1);
+                p.i = reflect_domain(idet, K.iEdge);
+                p.j = reflect_domain(jdet, K.jEdge);
                 p.k = kdet;
             }
         }
@@ -558,7 +583,7 @@ __device__ int move_particle_fast(const wacomm_b200_config &cfg, const IntervalP
             alive = lazy ? (p.age < P.ageUnder || exp(-p.age / cfg.tau0) > 0) : p.health > 0;
             if (alive && !lazy) {
                 // FP32 and an approximate division: the two-substep margin covers their error
-                const float n = floorf(__fdividef((float)(ageSafe - p.age), dtiF)) - 2.f;
+                const float n = floorf(__fdividef((float)(K.ageSafe - p.age), K.dti)) - 2.f;
                 youngLeft = n > 0.f ? (n < 1.0e9f ? (int)n : 1000000000) : 0;
             }
         }

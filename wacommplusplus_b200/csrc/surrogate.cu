@@ -950,6 +950,8 @@ struct WalkView {
     const CellSurface *surface;      // [cell]
     const float2 *invMetric;         // [cell] {1/xdist, 1/ydist}
     const float *depth;              // [sW-1] FP32 depthIntervals
+    StepConstants K;
+    float kLower, invKLower, sigma;
 };
 
 constexpr int WALK_BLOCKS = 5;  // resident blocks of 128 threads per SM the registers allow
@@ -1001,10 +1003,8 @@ template <int SEM, int STORE>
 __device__ int walk_particle(const wacomm_b200_config &cfg, const IntervalParams &P,
                              const WalkView<STORE> &W, const float *depthS, int eta, int xi,
                              int sW, ParticleState &p, float rateX, float rateY, float rateZ) {
-    const double length = P.length, invLength = 1.0 / length, kLower = P.kLower;
-    const float shore = (float)cfg.shoreLimit, kLowerF = (float)kLower;
-    const float invKLower = (float)P.invKLower, sigma = (float)cfg.sigma, crid = (float)cfg.crid;
-    const float dtiF = (float)cfg.dti;
+    const StepConstants &K = W.K;
+    const double length = P.length, kLower = P.kLower;
     const bool philox = P.rng == WACOMM_B200_RNG_PHILOX;
     const uint64_t prefix = fold(fold(mix64(cfg.randomSeed), p.id), (uint64_t)P.intervalKey);
     const uint64_t philoxKey = p.id ^ mix64(cfg.randomSeed);
@@ -1016,7 +1016,6 @@ __device__ int walk_particle(const wacomm_b200_config &cfg, const IntervalParams
     // ageKillLo <= ageKillHi) nor without health (age below ageUnder). Counted when the
     // particle turns lazy, two substeps short of the bound for rounding; while it lasts and no
     // closure has ended the lazy tracking, both tests are skipped.
-    const double ageSafe = fmin(P.ageKillLo, P.ageUnder);
     int youngLeft = 0;
 
     const double fj = floor(p.j), fi = floor(p.i), ck = ceil(p.k);
@@ -1056,10 +1055,10 @@ __device__ int walk_particle(const wacomm_b200_config &cfg, const IntervalParams
         load_second<STORE>(col - 1, aLo);  // akt of W level kI-1
         load_second<STORE>(col + 1, aUp);  // akt of W level kI
         const float depth = depthS[kM + sW - 2];
-        const float dt = stepDt == cfg.dti ? dtiF : (float)stepDt;
-        const float alpha = (float)((elapsed + 0.5 * stepDt) * invLength);
+        const float dt = stepDt == cfg.dti ? K.dti : (float)stepDt;
+        const float alpha = (float)((elapsed + 0.5 * stepDt) * K.invLength);
         const float hc = here.height(alpha);
-        if (hc <= shore && cfg.horizontalClosure == CLOSURE_KILL) {
+        if (hc <= K.shore && cfg.horizontalClosure == CLOSURE_KILL) {
             p.health = -1;
             lazy = false;
             if (SEM == SEM_DEVICE) break;
@@ -1078,12 +1077,12 @@ __device__ int walk_particle(const wacomm_b200_config &cfg, const IntervalParams
             n2 = (float)prefix_normal(stepKey, 2);
         }
         const float kNow = (float)kI - kF;
-        const float sigmaDepth = sigma * (1.f - kNow * invKLower);
-        const float scale = stepDt == cfg.dti ? 1.f : sqrtf(dt / dtiF);
+        const float sigmaDepth = W.sigma * (1.f - kNow * W.invKLower);
+        const float scale = stepDt == cfg.dti ? 1.f : sqrtf(dt / K.dti);
         // the two horizontal components in pairs (packed FP32x2, the same roundings)
         const float2 rxy = __fmul2_rn(__fmul2_rn(make_float2(sigmaDepth, sigmaDepth), make_float2(n0, n1)),
                                       make_float2(scale, scale));
-        const float rz = sigmaDepth * n2 * aa * crid * scale;
+        const float rz = sigmaDepth * n2 * aa * K.crid * scale;
         const float zdist = hc * depth;
         const float rzdist = __frcp_rn(zdist);
         const float2 dIJ = __fmul2_rn(__ffma2_rn(make_float2(rateX, rateY), make_float2(dt, dt), rxy), inv);
@@ -1102,8 +1101,8 @@ __device__ int walk_particle(const wacomm_b200_config &cfg, const IntervalParams
                             iD < 1.f && kD >= 0.f && kD < 1.f;
         const SurfaceSums there =
             surface_from(load_surface(W.surface, inside ? nj * xi + ni : cell), jD, iD);
-        const bool vertical = (float)kI - kN > 0.f || (float)kI - kN < kLowerF;
-        carried = inside && !vertical && there.height(alpha) > shore;
+        const bool vertical = (float)kI - kN > 0.f || (float)kI - kN < W.kLower;
+        carried = inside && !vertical && there.height(alpha) > K.shore;
         // The domain edge, under the closures that do not look at the land there: the destination
         // cell lies outside the valid cells and the level stays in range. Constraint drops the
         // horizontal move (the position and its surface sums stay); reflection mirrors each axis
@@ -1161,7 +1160,7 @@ __device__ int walk_particle(const wacomm_b200_config &cfg, const IntervalParams
                 const CellSurface at = load_surface(W.surface, jdetI * xi + idetI);
                 const float hcdet =
                     surface_from(at, (float)(jdet - fjd), (float)(idet - fid)).height(alpha);
-                if (hcdet <= shore) {
+                if (hcdet <= K.shore) {
                     if (cfg.horizontalClosure == CLOSURE_CONSTRAINT) {
                         idet = pi;
                         jdet = pj;
@@ -1207,7 +1206,7 @@ __device__ int walk_particle(const wacomm_b200_config &cfg, const IntervalParams
             if (alive) {
                 if (!lazy) {
                     // FP32 and an approximate division: the two-substep margin covers their error
-                    const float n = floorf(__fdividef((float)(ageSafe - p.age), (float)cfg.dti)) - 2.f;
+                    const float n = floorf(__fdividef((float)(K.ageSafe - p.age), K.dti)) - 2.f;
                     youngLeft = n > 0.f ? (n < 1.0e9f ? (int)n : 1000000000) : 0;
                 }
                 p.age = p.age + stepDt;
@@ -1485,6 +1484,10 @@ cudaError_t surrogate_step(const SurrogateStep &s, const ParticleSoA &S, const M
         W.surface = static_cast<const CellSurface *>(s.cellSurface);
         W.invMetric = s.invMetric;
         W.depth = s.depthF;
+        W.K = step_constants(s.cfg, *s.interval, s.eta, s.xi);
+        W.kLower = (float)s.interval->kLower;
+        W.invKLower = (float)s.interval->invKLower;
+        W.sigma = (float)s.cfg.sigma;
         MoveLaunch LW = L;
         LW.order = s.walkOrder;
         surrogate_walk_kernel<SEM, STORE><<<blocks128, 128, 0, stream>>>(a, s.cfg, *s.interval, W, S, LW);
