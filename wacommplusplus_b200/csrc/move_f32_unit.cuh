@@ -35,9 +35,9 @@ inline int fast_variant(const wacomm_b200_config &cfg, int direction) {
 }
 
 // Shapes 1, 2 and 3 carry every form; shape 0 the full one. A negative shape picks by form, the
-// register needs deciding (move kernel, shapes 1 / 2 / 3): lean, 4.2 M records 11.37 / 10.23 /
-// 9.94 ms; random walk (Philox), 1.05 M 4.09 / 3.64 / 3.77 ms; leeway drift, 400,000 2.51 / 2.27 /
-// 2.94 ms; full 5.33 / 5.97 / 7.25 ms (568 bytes of spills at shape 2, 188 at shape 1).
+// register needs deciding (move kernel, shapes 1 / 2 / 3): lean, 4.2 M records 9.81 / 9.91 / 9.80 ms
+// (FP16 storage 10.46 / 10.62 / 10.29); random walk (Philox), 1.05 M 4.08 / 3.55 / 3.61 ms; leeway
+// drift, 400,000 2.45 / 2.21 / 2.96 ms; full 5.14 / 5.74 / 6.90 ms (spills at shapes 2 and 3).
 template <int SEM, int STORE>
 cudaError_t move_f32_unit(int shape, const wacomm_b200_config &cfg, const IntervalParams &P,
                           const PackedArgs &A, const ParticleSoA &S, const MoveLaunch &L,
