@@ -423,7 +423,7 @@ int wacomm_b200_stream(const wacomm_b200_context *ctx, void **out);
  * like the reference does; wind/stokes may be NULL. Device semantics, reference arithmetic.
  * The records are moved in cell-and-level order (key, histogram, scan, scatter; the order changes
  * no result) and the bracketing forcing pair is packed once per call (grids of at most 1 Mi nodes or
- * 32 per record), with working memory taken from the device's memory pool on `stream`
+ * 32 per record, with s_w = s_rho + 1 and every field given), with working memory taken from the device's memory pool on `stream`
  * (cudaMallocAsync, about 8 B per record and per bin, 64 B per node and up to 96 B per cell,
  * released with cudaFreeAsync); when the pool has none, the records are moved in caller order and
  * the forcing is read from the caller's fields. */

@@ -230,3 +230,21 @@ def test_packed_pair_and_window_reads_agree(cuda_device, n, environment, directi
 @pytest.mark.parametrize("n", [40959, 40960])
 def test_pair_packed_by_records_on_a_large_grid(cuda_device, n):
     same_records_packed_and_read(syn.config1_window(n_frames=2, eta=512, xi=512, s_rho=4), n, False, 1)
+
+
+@pytest.mark.parametrize("form", ["more_rho_levels", "no_diffusivity"])
+def test_windows_that_are_not_packed(cuda_device, form):
+    win = syn.config1_window(n_frames=2, eta=9, xi=8, s_rho=4)
+    if form == "more_rho_levels":  # a rho level per W level: the upper ones belong to the layers
+        rng = np.random.default_rng(2)
+        win.u = rng.normal(0, 0.1, (win.T, win.sW, win.eta, win.xi)).astype(np.float32)
+        win.v = rng.normal(0, 0.1, (win.T, win.sW, win.eta, win.xi)).astype(np.float32)
+        win.sRho = win.sW
+    else:
+        win.akt = None
+    p = syn.uniform_particles(593, win.eta, win.xi, seed=3, time=win.times[0])
+    cfg = default_config(random=form == "more_rho_levels")
+    got = call_dropin(cfg, p, win, 0)
+    noalloc = call_dropin(cfg, p, win, 0, _native.lib().wacomm_b200_cuda_move_particle_noalloc)
+    assert records_equal(got, noalloc)
+    assert not np.array_equal(got["i"], p["i"])

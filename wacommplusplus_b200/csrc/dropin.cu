@@ -163,14 +163,17 @@ cudaError_t launch_dropin(const wacomm_b200_config *config, wacomm_b200_particle
 // 180,224 nodes: 1.1 ms). It bounds the scratch to 64 MB or 2 KB per record.
 constexpr size_t PACK_NODES = (size_t)1 << 20, PACK_NODES_PER_RECORD = 32;
 
-// The call's packed pair in `scratch` (null: no scratch, read the window), stream-ordered.
+// The call's packed pair in `scratch` (null: no scratch, read the window), stream-ordered. The window is
+// read, too, where a node record does not hold what the move reads: with other rho levels than one per
+// layer, or without a field (the diffusivity of a run without random walk).
 cudaError_t pack_window(const wacomm_b200_config *config, int timeIndex, int oceanTime,
                         const RawView &V, int count, PackedView &out, void **scratch,
                         cudaStream_t stream) {
     const size_t plane = (size_t)V.g.eta * V.g.xi, nodes = plane * V.g.sW;
     const bool env = V.hasWindU || V.hasWindV || V.hasStokes;
     *scratch = nullptr;
-    if (V.g.eta < 2 || V.g.xi < 2 ||
+    if (V.g.eta < 2 || V.g.xi < 2 || V.g.sW != V.g.sRho + 1 || !V.zeta || !V.u || !V.v || !V.w ||
+        !V.aktField || !V.hField || !V.lonRad || !V.latRad ||
         (nodes > PACK_NODES && nodes > PACK_NODES_PER_RECORD * (size_t)count))
         return cudaSuccess;
     const size_t bytes = nodes * sizeof(NodeRecord) +
