@@ -1380,13 +1380,24 @@ int wacomm_b200_move_interval_host(wacomm_b200_context *ctx, int time_index,
     }
     bounds.push_back(n);
     const int slabs = (int)bounds.size() - 1;
+    const bool sorts = !P.skip && sorts_work(ctx, n / slabs);
+    // The sort scratch of each lane for its largest slab, before the first one: growing it between the
+    // slabs frees it, which waits for the device and everything in flight on it.
+    size_t largest[2] = {0, 0};
+    for (int s = 0; s < slabs; s++) {
+        size_t &lane = largest[(s & 1) != 0 && s < slabs - ordered];
+        lane = std::max(lane, bounds[s + 1] - bounds[s]);
+    }
+    for (int second = 0; sorts && second < 2; second++) {
+        LaneSwap lane(ctx, second != 0);
+        if (largest[second] && (rc = reserve_sort(ctx, largest[second]))) return rc;
+    }
     std::vector<cudaEvent_t> up(slabs), done(slabs);
     for (int s = 0; s < slabs; s++) {
         cudaEventCreateWithFlags(&up[s], cudaEventDisableTiming);
         cudaEventCreateWithFlags(&done[s], cudaEventDisableTiming);
     }
     // each slab's sort walks that slab's previous order when the last call had the same slabs
-    const bool sorts = !P.skip && sorts_work(ctx, n / slabs);
     const bool walk = sorts && ctx->seqBounds == bounds;
     if (sorts) ctx->seqBounds.clear();
     CUDA_TRY(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
