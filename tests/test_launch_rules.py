@@ -1,0 +1,37 @@
+"""The host rules of the launches (csrc/launch_rules.h), compiled here with g++."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "wacommplusplus_b200", "csrc")
+
+
+def evaluate(tmp_path, body):
+    """The integers a C++ function body over the rules prints, one row per line."""
+    source, exe = tmp_path / "rules.cpp", str(tmp_path / "rules")
+    source.write_text('#include <cstdio>\n#include "launch_rules.h"\nusing namespace wb;\n'
+                      'int main() {\n' + body + '\n}\n')
+    build = subprocess.run(["g++", "-std=c++17", "-O1", "-ftrapv", str(source), "-I", CSRC, "-I",
+                            os.path.join(ROOT, "include"), "-o", exe], capture_output=True, text=True)
+    assert build.returncode == 0, build.stderr[-2000:]
+    run = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert run.returncode == 0, run.stderr[-500:]
+    return [[int(x) for x in line.split()] for line in run.stdout.splitlines()]
+
+
+# up to the largest count the entry points take: the sums stay in range and the blocks cover it
+@pytest.mark.parametrize("threads", [32, 128, 256])
+def test_launches_cover_every_count(tmp_path, threads):
+    counts = [1, 31, 592, 593, 18944, 18945, 1 << 24, (1 << 31) - 592, (1 << 31) - 591,
+              (1 << 31) - 128, (1 << 31) - 1]
+    rows = evaluate(tmp_path, "".join(
+        f"{{ int lanes, threads; spread_launch({n}, {threads}, lanes, threads);"
+        f'printf("%d %d %d\\n", lanes, threads, launch_blocks({n}, threads / 32 * lanes)); }}\n'
+        for n in counts))
+    for n, (lanes, size, blocks) in zip(counts, rows):
+        items = size // 32 * lanes
+        assert 1 <= lanes <= 32 and size % 32 == 0 and 32 <= size <= threads
+        assert (blocks - 1) * items < n <= blocks * items
+        assert lanes == 32 or n <= 18944

@@ -147,7 +147,7 @@ cudaError_t launch_dropin(const wacomm_b200_config *config, wacomm_b200_particle
     L.count = count;
     int threads;
     spread_launch(count, 128, L.lanes, threads);
-    const int items = threads / 32 * L.lanes, blocks = (count + items - 1) / items;
+    const int items = threads / 32 * L.lanes, blocks = launch_blocks(count, items);
     if (count <= KEEP_RECORDS)
         dropin_move_kernel<true><<<blocks, threads, 0, stream>>>(config, particles, order, timeIndex,
                                                                  oceanTime, times, V, L);

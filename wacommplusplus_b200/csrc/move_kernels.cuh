@@ -2,6 +2,7 @@
 #pragma once
 
 #include "engine.h"
+#include "launch_rules.h"
 #include "step.cuh"
 #include "step_fast.cuh"
 
@@ -60,22 +61,6 @@ __device__ __forceinline__ unsigned launch_item(const MoveLaunch &L, unsigned ba
     if (L.lanes >= 32) return base + threadIdx.x;
     const unsigned lane = threadIdx.x & 31;
     return lane < (unsigned)L.lanes ? base + (threadIdx.x >> 5) * L.lanes + lane : count;
-}
-
-// Lanes per warp and threads per block (at most maxThreads) of a launch over `count` items: one warp
-// per scheduler of the chip before a warp is filled, as blocks of one size on every SM. Such a launch
-// is bound by the latency of its substep chain; fewer lanes per warp meet fewer cell changes and
-// lines per load. 1,021 records (random walk) per host interval 0.473 -> 0.428 ms, 16,384 in
-// reference arithmetic 0.640 -> 0.564 ms; two warps per scheduler: 0.459 and 0.628 ms. From 18,945
-// items on the warps are full.
-inline void spread_launch(int count, int maxThreads, int &lanes, int &threads) {
-    constexpr int SMS = 148, WARPS = 4 * SMS;
-    lanes = (count + WARPS - 1) / WARPS;
-    if (lanes > 32) lanes = 32;
-    if (lanes < 1) lanes = 1;
-    const int warps = (count + lanes - 1) / lanes;
-    threads = 32 * ((warps + SMS - 1) / SMS);
-    if (threads > maxThreads) threads = maxThreads;
 }
 
 // Work items of a launch: count, or the device-side length of its list.
@@ -230,7 +215,7 @@ cudaError_t launch_move_fast(const wacomm_b200_config &cfg, const IntervalParams
     int threads;
     spread_launch(L.count, LaunchShape<SHAPE>::threads, M.lanes, threads);
     const long long items = (long long)(threads / 32) * M.lanes * (L.perThread > 1 ? L.perThread : 1);
-    const int blocks = (int)((L.count + items - 1) / items);
+    const int blocks = launch_blocks(L.count, items);
     FastView<STORE> G = F;
     G.X.K = step_constants(cfg, P, F.V.g.eta, F.V.g.xi);
     move_fast_kernel<SEM, STORE, SHAPE, VARIANT><<<blocks, threads, 0, stream>>>(cfg, P, G, S, M);
@@ -249,7 +234,7 @@ cudaError_t launch_move_soa(const wacomm_b200_config &cfg, const IntervalParams 
     int threads;
     spread_launch(L.count, blockSize, M.lanes, threads);
     const int items = threads / 32 * M.lanes;
-    const int blocks = (L.count + items - 1) / items;
+    const int blocks = launch_blocks(L.count, items);
     const bool keep = L.count <= KEEP_RECORDS;
     if (cfg.driftModel == 1) {
         if (keep) move_soa_kernel<SEM, true, true><<<blocks, threads, 0, stream>>>(cfg, P, V, S, M);
