@@ -24,6 +24,7 @@
 #include <cuda_bf16.h>
 
 #include "engine.h"
+#include "launch_rules.h"
 #include "umma.cuh"
 
 namespace wb {
@@ -54,7 +55,7 @@ constexpr int SUM_DB = 0, SUM_DW4 = 3 * T_HID, SUM_DB4 = 6 * T_HID, SUM_LOSS = S
 constexpr int UNITS = 8;
 constexpr int X_TAIL = T_IN - T_HID;           // columns of W1's second part
 constexpr int X_TAIL_N = (X_TAIL + 15) / 16 * 16;
-constexpr int MAX_SPLITS = 148 / UNITS;        // ranges of tiles: about one block per SM
+constexpr int MAX_SPLITS = B200_SMS / UNITS;   // ranges of tiles: about one block per SM
 
 // The work buffer: an error word (at its start), then, from the next 1024-byte boundary, the packed
 // weights, the images and sums per tile and the partial weight gradients.
@@ -719,7 +720,7 @@ cudaError_t mlp_train_step(const float *stencil, const float *particle, const fl
     w.err = reinterpret_cast<int *>(work);
     pack_weights_kernel<<<W_BLOCKS * T_HID * 8 / 256, 256, 0, stream>>>(params, w.weights, w.err);
     const TileArgs t{stencil, particle, gate, target, params, batch, tiles, w};
-    tile_kernel<<<tiles < 148 ? tiles : 148, TILE_THREADS, TILE_SMEM, stream>>>(t);
+    tile_kernel<<<tiles < B200_SMS ? tiles : B200_SMS, TILE_THREADS, TILE_SMEM, stream>>>(t);
     const GradArgs g{tiles, tiles < MAX_SPLITS ? tiles : MAX_SPLITS, w};
     weight_grad_kernel<<<dim3(UNITS, g.splits), GRAD_THREADS, GRAD_SMEM, stream>>>(g);
     const Adam adam{params, grads, m, v, lr, 1.f - powf(0.9f, (float)step),

@@ -50,7 +50,7 @@ cudaError_t move_f32_unit(int shape, const wacomm_b200_config &cfg, const Interv
     // records that are all resident at once at shape 1 (12 warps per SM): nothing is gained by more
     // warps, and its registers shorten the substep's chain: 600 records 0.130 ms (shape 3: 0.156),
     // 16,000 0.173 (0.196), 40,000 0.189 (0.212); random walk 0.263 (shape 2: 0.294)
-    if (shape < 0 && !L.countDevice && L.count <= 12 * 148 * 32) shape = 1;
+    if (shape < 0 && !L.countDevice && L.count <= RESIDENT_RECORDS) shape = 1;
     if (shape < 0) shape = variant == VAR_LEAN ? 3 : variant == VAR_FULL ? 1 : 2;
     switch (shape) {
         case 0: return launch_move_fast<SEM, STORE, 0, VAR_FULL>(cfg, P, F, S, L, stream);

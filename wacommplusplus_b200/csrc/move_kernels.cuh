@@ -222,8 +222,6 @@ cudaError_t launch_move_fast(const wacomm_b200_config &cfg, const IntervalParams
     return cudaGetLastError();
 }
 
-constexpr int KEEP_RECORDS = 2 * 4 * 148 * 32;  // two full warps per scheduler
-
 // Host launchers (one per template instance, defined in the instantiation units).
 template <int SEM>
 cudaError_t launch_move_soa(const wacomm_b200_config &cfg, const IntervalParams &P,
