@@ -119,26 +119,32 @@ typedef struct wacomm_b200_source {
 #define WACOMM_B200_RNG_REFERENCE 0    /* ordered-splitmix64-v2 draws, draw-for-draw with the reference */
 #define WACOMM_B200_RNG_PHILOX 1       /* Philox4x32-10 keyed on (particle id, interval, step time) */
 
-#define WACOMM_B200_LAUNCH_SHAPE_AUTO (-1) /* launch_shape by compiled form: 3 for the deterministic
-                                              form without drift (96 registers), 1 for the form
-                                              with every branch, 2 for the others; the default */
+#define WACOMM_B200_LAUNCH_SHAPE_AUTO (-1) /* launch_shape by size and compiled form: 1 up to 56,832
+                                              records, beyond 3 for the deterministic form without
+                                              drift (96 registers), 1 for the form with every
+                                              branch, 2 for the others; up to 40,000 records of a
+                                              passive random walk with RNG_REFERENCE the normals are
+                                              drawn by a kernel ahead of the step; the default */
 
 typedef struct wacomm_b200_options {
     int semantics;            /* WACOMM_B200_SEMANTICS_* */
     int arithmetic;           /* WACOMM_B200_ARITH_* */
     int storage;              /* WACOMM_B200_STORAGE_* */
     int rng;                  /* WACOMM_B200_RNG_* */
-    int block_size;           /* threads per block of the move kernel: 64..1024, multiple of 32 */
+    int block_size;           /* reference arithmetic: threads per block of the move kernel, 32..256,
+                                 multiple of 32; launches too small to fill the SMs take fewer */
     int substeps_per_launch;  /* 0: one launch per interval; else launches of this many dti */
     int sort_by_cell;         /* N >= 1: order the work by forcing cell, sorting the resident
                                  population every N-th interval (the intervals between take the
                                  last sort's order); 1 (the default): every interval; 0: never;
-                                 at most 64; wacomm_b200_autotune chooses 1, 2 or 4 */
+                                 at most 64; wacomm_b200_autotune chooses 1, 2 or 4. The plain
+                                 step sorts populations of more than 37,888 records only */
     int fuse_concentration;   /* 1: count the concentration in the move kernel's epilogue */
     int launch_shape;         /* FP32 step: 0 = 256 threads, registers unbounded; 1 = 128 threads,
                                  3 blocks/SM; 2 = 256 threads, 2 blocks/SM; 3 = 128 threads,
                                  5 blocks/SM (fewer registers, more resident warps);
-                                 WACOMM_B200_LAUNCH_SHAPE_AUTO (default): 3, 2 or 1 by form */
+                                 WACOMM_B200_LAUNCH_SHAPE_AUTO (default): by size and form.
+                                 Launches too small to fill the SMs take fewer threads per block */
     int surrogate;            /* 1: forward intervals by the learned surrogate
                                  (wacomm_b200_set_surrogate), with the plain stochastic operator
                                  per substep when the random walk is on; the rest by the FP32 step */
@@ -263,15 +269,15 @@ int wacomm_b200_graph_launch(wacomm_b200_context *ctx);
 int wacomm_b200_graph_release(wacomm_b200_context *ctx);
 
 /* Times the interval at time_index once per launch configuration of the move kernel (FP32
- * arithmetic: launch_shape 0..3; reference arithmetic: block_size 64, 128, 192, 256), each from
- * the same resident records and concentration after a warm-up pass, keeps the fastest in the
- * options and restores records and concentration: only the options change. Writes the chosen
- * value and its device ms. With FP32 arithmetic it then times the interval with 1, 2 and 4
- * work items per thread at the chosen shape and keeps the fastest in
- * options.particles_per_thread. With the cell sort on and four intervals from time_index inside
- * the forcing window, it then times those four intervals from the same snapshot sorting every
- * 1, 2 or 4 of them and keeps the fastest cadence in options.sort_by_cell. No reference
- * counterpart. */
+ * arithmetic: launch_shape 0..3, and WACOMM_B200_LAUNCH_SHAPE_AUTO where that draws the normals
+ * ahead; reference arithmetic: block_size 64, 128, 192, 256), each from the same resident records
+ * and concentration after a warm-up pass, keeps the fastest in the options and restores records
+ * and concentration: only the options change. Writes the chosen value and its device ms. With
+ * FP32 arithmetic it then times the interval with 1, 2 and 4 work items per thread at the chosen
+ * shape and keeps the fastest in options.particles_per_thread. With the population sorted
+ * (options.sort_by_cell) and four intervals from time_index inside the forcing window, it then
+ * times those four intervals from the same snapshot sorting every 1, 2 or 4 of them and keeps the
+ * fastest cadence in options.sort_by_cell. No reference counterpart. */
 int wacomm_b200_autotune(wacomm_b200_context *ctx, int time_index, int *best, float *best_ms);
 
 /* The same interval through host buffers: uploads n records from `particles` (pinned or

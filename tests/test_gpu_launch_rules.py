@@ -1,0 +1,41 @@
+"""Options of the plain step's launches: what is asked for is what is launched, with the same records."""
+import numpy as np
+import pytest
+
+from wacommplusplus_b200 import synthetic as syn
+from wacommplusplus_b200.engine import Engine
+from wacommplusplus_b200.types import default_config
+
+pytestmark = pytest.mark.gpu
+
+
+def walking_engine(n, intervals=1, **options):
+    """An engine with n records in a random walk and its forcing loaded."""
+    win = syn.config1_window(n_frames=intervals + 1, eta=16, xi=17, s_rho=6)
+    engine = Engine(0, **options)
+    engine.load_window(win)
+    engine.set_config(default_config(random=True))
+    engine.set_particles(syn.uniform_particles(n, win.eta, win.xi, seed=n, time=win.times[0]))
+    return engine
+
+
+def test_an_explicit_launch_shape_is_launched(cuda_device):
+    """The automatic shape draws a small population's normals in a launch of their own."""
+    records, launches = [], []
+    for shape in (-1, 0, 1, 2, 3):
+        with walking_engine(2000, 2, launch_shape=shape) as engine:
+            for t in range(2):
+                engine.move_interval(t)
+            records.append(engine.get_particles().tobytes())
+            launches.append(engine.stats()["launches"])
+    assert all(r == records[0] for r in records)
+    assert launches[1:] == [launches[0] - 1] * 4
+
+
+def test_autotune_of_a_population_that_is_not_sorted_keeps_its_cadence(cuda_device):
+    with walking_engine(2000, 6, sort_by_cell=3) as engine:
+        before = engine.get_particles()
+        shape, ms = engine.autotune(0)
+        assert engine.options().launch_shape == shape and ms > 0
+        assert engine.options().sort_by_cell == 3
+        assert np.array_equal(before, engine.get_particles())

@@ -35,3 +35,20 @@ def test_launches_cover_every_count(tmp_path, threads):
         assert 1 <= lanes <= 32 and size % 32 == 0 and 32 <= size <= threads
         assert (blocks - 1) * items < n <= blocks * items
         assert lanes == 32 or n <= 18944
+
+
+DRAW = """
+wacomm_b200_options o{}; wacomm_b200_config c{};
+o.arithmetic = WACOMM_B200_ARITH_FP32; o.rng = WACOMM_B200_RNG_REFERENCE;
+c.random = 1; c.trackingDirection = 1; c.dti = 30.0;
+"""
+
+
+# an explicit launch shape is the one that is launched: the draws ahead have a shape of their own
+def test_normals_are_drawn_ahead_under_the_automatic_shape_alone(tmp_path):
+    rows = evaluate(tmp_path, DRAW + """
+    for (int shape = WACOMM_B200_LAUNCH_SHAPE_AUTO; shape <= 3; shape++) {
+        o.launch_shape = shape;
+        printf("%u\\n", draw_steps(o, c, 3600.0, 1000));
+    }""")
+    assert [r[0] for r in rows] == [121, 0, 0, 0, 0]

@@ -2356,8 +2356,18 @@ int wacomm_b200_autotune(wacomm_b200_context *ctx, int time_index, int *best, fl
     if (rc) return rc;
     cudaSetDevice(ctx->device);
     const bool fp32 = ctx->opt.arithmetic == WACOMM_B200_ARITH_FP32;
-    const std::vector<int> candidates = fp32 ? std::vector<int>{0, 1, 2, 3}
-                                             : std::vector<int>{64, 128, 192, 256};
+    std::vector<int> candidates = fp32 ? std::vector<int>{0, 1, 2, 3}
+                                       : std::vector<int>{64, 128, 192, 256};
+    if (fp32 && time_index >= 0 && time_index < (int)ctx->times.size()) {
+        // where the automatic shape has the normals drawn ahead, a form that no number names
+        IntervalParams P;
+        make_interval(ctx->cfg, ctx->times.data(), (int)ctx->times.size(), time_index, ctx->sW,
+                      ctx->opt.semantics, P);
+        wacomm_b200_options automatic = ctx->opt;
+        automatic.launch_shape = WACOMM_B200_LAUNCH_SHAPE_AUTO;
+        if (draw_steps(automatic, ctx->cfg, P.length, ctx->n))
+            candidates.push_back(WACOMM_B200_LAUNCH_SHAPE_AUTO);
+    }
     // snapshot: records (AoS), concentration, then one timed interval per candidate from it
     const size_t n = ctx->n;
     if ((rc = grow(ctx, ctx->dAos, ctx->aosCap, n))) return rc;
@@ -2441,11 +2451,11 @@ int wacomm_b200_autotune(wacomm_b200_context *ctx, int time_index, int *best, fl
         ctx->opt.particles_per_thread = per;
     }
     // The sort cadence, with the chosen shape: four intervals from the snapshot sorting every
-    // 1, 2 or 4 of them; the fastest run sets options.sort_by_cell (when sorting is on and the
-    // four intervals lie inside the forcing window).
+    // 1, 2 or 4 of them; the fastest run sets options.sort_by_cell (when the population is sorted
+    // and the four intervals lie inside the forcing window).
     const int dir = ctx->cfg.trackingDirection, T = (int)ctx->times.size();
     const int runEnd = time_index + 4 * dir;
-    if (!rc && saved.sort_by_cell && runEnd >= 0 && runEnd < T) {
+    if (!rc && sorts_work(ctx, n) && runEnd >= 0 && runEnd < T) {
         int cadence = saved.sort_by_cell;
         float bestRun = INFINITY;
         for (int pass = 0; pass < 2 && !rc; pass++)

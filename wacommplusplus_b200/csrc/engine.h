@@ -99,10 +99,6 @@ cudaError_t sort_by_cell(const ParticleSoA &S, int n, const SortBins &bins, cons
                          uint32_t *keys, uint32_t *hist, uint32_t *offsets, uint32_t *temp,
                          uint32_t *order, cudaStream_t stream);
 
-// Substeps whose normals draw_normals lays out for `count` records of an interval (0: none, the step
-// draws them itself).
-unsigned draw_steps(const wacomm_b200_options &opt, const wacomm_b200_config &cfg, double length,
-                    size_t count);
 // out[s * count + slot] = the normals 0..2 of the reference keys of record `slot` in substep s.
 cudaError_t draw_normals(const uint64_t *id, int count, uint64_t seed, long long interval,
                          unsigned steps, float4 *out, cudaStream_t stream);

@@ -1,6 +1,11 @@
 // Rules of the launches that follow from sizes and options alone: plain C++, for the host.
 #pragma once
 
+#include <cmath>
+#include <cstddef>
+
+#include "wacomm_b200.h"
+
 namespace wb {
 
 constexpr int B200_SMS = 148;
@@ -28,6 +33,33 @@ inline void spread_launch(int count, int maxThreads, int &lanes, int &threads) {
 // Blocks of `items` work items each that cover `count` (1 to 2^31 - 1).
 inline int launch_blocks(int count, long long items) {
     return (int)(((long long)count + items - 1) / items);
+}
+
+// Up to here the move with the draws ahead is the faster one (whole interval of 120 substeps, with /
+// without): 1,021 records 0.26 / 0.43 ms, 20,011 0.40 / 0.51 ms, 30,000 0.45 / 0.52 ms, 45,000 0.54 /
+// 0.56 ms, 59,000 0.59 / 0.56 ms: beyond, the chip is busy with substeps and the draws cost the same
+// either way. The draws stay in L2 (77 MB at the limit).
+constexpr size_t DRAW_AHEAD_RECORDS = 40000;
+constexpr double DRAW_AHEAD_BYTES = 256.0 * (1 << 20);
+
+// Substeps whose normals are drawn ahead (draw_normals) of an interval of `length` seconds over `count`
+// records; 0: the step draws them itself. The form that reads them has one launch shape, so an explicit
+// launch_shape keeps the draws in the step.
+inline unsigned draw_steps(const wacomm_b200_options &opt, const wacomm_b200_config &cfg, double length,
+                           size_t count) {
+    const bool diffuse = cfg.random && (cfg.trackingDirection > 0 || cfg.backwardDiffusion);
+    const bool plain = cfg.driftModel != 1 && !(cfg.leewayJibeProbabilityHourly > 0);
+    if (!diffuse || !plain || opt.rng != WACOMM_B200_RNG_REFERENCE ||
+        opt.arithmetic != WACOMM_B200_ARITH_FP32 || opt.launch_shape != WACOMM_B200_LAUNCH_SHAPE_AUTO)
+        return 0;
+    // floor(elapsed / dti) of a substep that starts before the end; the quotient may round up to the
+    // next whole number there
+    const double steps = std::ceil(length / cfg.dti) + 1;
+    constexpr size_t DRAW_BYTES = 4 * sizeof(float);  // three normals and padding
+    if (!(steps >= 2 && steps <= 1e6) || count > DRAW_AHEAD_RECORDS ||
+        steps * count * DRAW_BYTES > DRAW_AHEAD_BYTES)
+        return 0;
+    return (unsigned)steps;
 }
 
 }  // namespace wb

@@ -44,7 +44,7 @@ cudaError_t move_f32_unit(int shape, const wacomm_b200_config &cfg, const Interv
                           cudaStream_t stream) {
     FastView<STORE> F = fast_view<STORE>(A);
     const int variant = fast_variant(cfg, P.direction);
-    // small launches, bound by latency: one block size serves every shape
+    // small launches under the automatic shape (draw_steps), bound by latency
     if (variant == VAR_DIFFUSE && L.draws)
         return launch_move_fast<SEM, STORE, 1, VAR_DRAWN>(cfg, P, F, S, L, stream);
     // records that are all resident at once at shape 1 (12 warps per SM): nothing is gained by more

@@ -473,28 +473,6 @@ __global__ void __launch_bounds__(256) draw_normals_kernel(const uint64_t *id, u
     }
 }
 
-// Up to here the move with the draws ahead is the faster one (whole interval of 120 substeps, with /
-// without): 1,021 records 0.26 / 0.43 ms, 20,011 0.40 / 0.51 ms, 30,000 0.45 / 0.52 ms, 45,000 0.54 /
-// 0.56 ms, 59,000 0.59 / 0.56 ms: beyond, the chip is busy with substeps and the draws cost the same
-// either way. The draws stay in L2 (77 MB at the limit).
-constexpr size_t DRAW_AHEAD_RECORDS = 40000;
-constexpr double DRAW_AHEAD_BYTES = 256.0 * (1 << 20);
-
-unsigned draw_steps(const wacomm_b200_options &opt, const wacomm_b200_config &cfg, double length,
-                    size_t count) {
-    const bool diffuse = cfg.random && (cfg.trackingDirection > 0 || cfg.backwardDiffusion);
-    const bool plain = cfg.driftModel != 1 && !(cfg.leewayJibeProbabilityHourly > 0);
-    if (!diffuse || !plain || opt.rng != WACOMM_B200_RNG_REFERENCE || opt.arithmetic != WACOMM_B200_ARITH_FP32)
-        return 0;
-    // floor(elapsed / dti) of a substep that starts before the end; the quotient may round up to the
-    // next whole number there
-    const double steps = ceil(length / cfg.dti) + 1;
-    if (!(steps >= 2 && steps <= 1e6) || count > DRAW_AHEAD_RECORDS ||
-        steps * count * sizeof(float4) > DRAW_AHEAD_BYTES)
-        return 0;
-    return (unsigned)steps;
-}
-
 cudaError_t draw_normals(const uint64_t *id, int count, uint64_t seed, long long interval,
                          unsigned steps, float4 *out, cudaStream_t stream) {
     if (count <= 0 || !steps) return cudaSuccess;

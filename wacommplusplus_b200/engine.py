@@ -36,7 +36,7 @@ class Engine:
     Options (defaults in brackets): semantics ["host"|"device"], arithmetic ["fp32"|"reference"],
     storage ["fp32"|"fp16"|"bf16"], rng ["reference"|"philox"], block_size [256],
     substeps_per_launch [0 = whole interval], sort_by_cell [True], fuse_concentration [True],
-    launch_shape [-1: 3 for the lean form, 1 for the full one, 2 for the others], surrogate [False] (needs
+    launch_shape [-1: by the number of records and the form], surrogate [False] (needs
     set_surrogate).
     """
 
@@ -230,8 +230,9 @@ class Engine:
 
     def autotune(self, time_index):
         """Times each launch configuration on interval time_index and keeps the fastest;
-        returns (chosen launch_shape or block_size, its device ms). The FP32 step's work items
-        per thread and the sort cadence it chooses next are in options()."""
+        returns (chosen launch_shape or block_size, its device ms); the launch_shape stays -1
+        where the automatic rule's small form is the fastest. The FP32 step's work items per
+        thread and the sort cadence it chooses next are in options()."""
         best, ms = ctypes.c_int(), ctypes.c_float()
         self._check(self._lib.wacomm_b200_autotune(self._ctx, time_index, ctypes.byref(best),
                                                    ctypes.byref(ms)))
