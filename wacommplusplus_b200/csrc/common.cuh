@@ -79,8 +79,9 @@ __device__ __forceinline__ double key_uniform_exact(uint64_t key) {
     return (high - 2147483648.5) + low;
 }
 
-// prefix_normal for the FP32 step: the same in FP64 up to its last bits (cos(2 pi u) by cospi, which
-// needs no argument reduction), rounded to float. 1.05 M records, 120 substeps: 6.47 -> 6.17 ms.
+// prefix_normal for the FP32 step and the learned form's walk, which draw alike: the same in FP64 up to
+// its last bits (cos(2 pi u) by cospi, which needs no argument reduction), rounded to float. 1.05 M
+// records, 120 substeps: 6.47 -> 6.17 ms.
 __device__ __forceinline__ float prefix_normal_f32(uint64_t prefix, uint64_t component) {
     const double u1 = fmax(key_uniform_exact(fold(prefix, component * 2)), DBL_MIN);
     const double u2 = key_uniform_exact(fold(prefix, component * 2 + 1));

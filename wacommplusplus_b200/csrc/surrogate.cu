@@ -1072,9 +1072,9 @@ __device__ int walk_particle(const wacomm_b200_config &cfg, const IntervalParams
                             n2);
         } else {
             const uint64_t stepKey = fold(prefix, (uint64_t)floor(elapsed / cfg.dti));
-            n0 = (float)prefix_normal(stepKey, 0);
-            n1 = (float)prefix_normal(stepKey, 1);
-            n2 = (float)prefix_normal(stepKey, 2);
+            n0 = prefix_normal_f32(stepKey, 0);
+            n1 = prefix_normal_f32(stepKey, 1);
+            n2 = prefix_normal_f32(stepKey, 2);
         }
         const float kNow = (float)kI - kF;
         const float sigmaDepth = W.sigma * (1.f - kNow * W.invKLower);
