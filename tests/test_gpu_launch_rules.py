@@ -39,3 +39,17 @@ def test_autotune_of_a_population_that_is_not_sorted_keeps_its_cadence(cuda_devi
         assert engine.options().launch_shape == shape and ms > 0
         assert engine.options().sort_by_cell == 3
         assert np.array_equal(before, engine.get_particles())
+
+
+# five slabs of which the two at the ends are too small to be sorted, all five sorted from 530,446 on
+@pytest.mark.parametrize("n", [393216, 530432, 530450])
+def test_host_buffer_intervals_walk_the_sorted_slabs_orders_alone(cuda_device, n):
+    with walking_engine(n, 3, rng="philox") as engine:
+        p = engine.get_particles()
+        for t in range(3):
+            engine.move_interval(t)
+        resident = engine.get_particles()
+    with walking_engine(1, 3, rng="philox") as engine:
+        for t in range(3):
+            engine.move_interval_host(t, p)
+    assert p.tobytes() == resident.tobytes()

@@ -80,7 +80,8 @@ struct wacomm_b200_context {
     // The last sorts' orders, the sequence the next sorts walk: for consecutive entries b, e of
     // seqBounds, dSeq[b, e) is a permutation of [0, e - b) (the work order of the records b..e-1).
     // Empty: nothing valid. {0, n}: the resident population sorted as one; the slab bounds of
-    // move_interval_host: one permutation per slab. Any permutation gives the same sort; walking
+    // move_interval_host: one permutation per slab that is sorted (sorts_work; the words of a
+    // smaller slab hold none and are not walked). Any permutation gives the same sort; walking
     // the previous one keeps the histogram atomics from piling up where particles gather.
     uint32_t *dSeq = nullptr;
     std::vector<size_t> seqBounds;
@@ -1397,7 +1398,7 @@ int wacomm_b200_move_interval_host(wacomm_b200_context *ctx, int time_index,
         cudaEventCreateWithFlags(&up[s], cudaEventDisableTiming);
         cudaEventCreateWithFlags(&done[s], cudaEventDisableTiming);
     }
-    // each slab's sort walks that slab's previous order when the last call had the same slabs
+    // each sorted slab walks its own previous order when the last call had the same slabs
     const bool walk = sorts && ctx->seqBounds == bounds;
     if (sorts) ctx->seqBounds.clear();
     CUDA_TRY(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
@@ -1430,8 +1431,9 @@ int wacomm_b200_move_interval_host(wacomm_b200_context *ctx, int time_index,
         CUDA_TRY(ctx, aos_to_soa(ctx->dAos + off, (int)cnt, S, ctx->stream));
         launches++;
         if (!P.skip) {
-            if ((rc = run_interval(ctx, P, off, cnt, ctx->dKeys + off, ctx->dOrder + off,
-                                   walk ? ctx->dSeq + off : nullptr, ctx->dSeq + off, launches)))
+            const uint32_t *seqIn = walk && sorts_work(ctx, cnt) ? ctx->dSeq + off : nullptr;
+            if ((rc = run_interval(ctx, P, off, cnt, ctx->dKeys + off, ctx->dOrder + off, seqIn,
+                                   ctx->dSeq + off, launches)))
                 return rc;
         }
         CUDA_TRY(ctx, soa_to_aos(S, (int)cnt, ctx->dAos + off, ctx->stream));
