@@ -428,11 +428,11 @@ int wacomm_b200_stream(const wacomm_b200_context *ctx, void **out);
  * the CUDA error code of the launch (0 = cudaSuccess). mask, num_thread and num_gpu are ignored
  * like the reference does; wind/stokes may be NULL. Device semantics, reference arithmetic.
  * The records are moved in cell-and-level order (key, histogram, scan, scatter; the order changes
- * no result) and the bracketing forcing pair is packed once per call (grids of at most 1 Mi nodes or
- * 32 per record, with s_w = s_rho + 1 and every field given), with working memory taken from the device's memory pool on `stream`
- * (cudaMallocAsync, about 8 B per record and per bin, 64 B per node and up to 96 B per cell,
- * released with cudaFreeAsync); when the pool has none, the records are moved in caller order and
- * the forcing is read from the caller's fields. */
+ * no result) and the bracketing forcing pair is packed once per call, with working memory taken from
+ * the device's memory pool on `stream` (cudaMallocAsync, released with cudaFreeAsync): about 8 B per
+ * record and per bin, and for the pair 64 B per node and up to 96 B per cell, where that is at most
+ * 80 MiB, or 96 B per record and 1 GiB, s_w = s_rho + 1 and every field is given. Beyond, the forcing
+ * is read from the caller's fields; when the pool has no memory, also in caller order. */
 int wacomm_b200_cuda_move_particle(const wacomm_b200_config *config_device,
                                    wacomm_b200_particle *particles_device, int time_index,
                                    int ocean_time, int s_w, int s_rho, int eta, int xi,

@@ -2,6 +2,7 @@
 import numpy as np
 import pytest
 
+from test_gpu_dropin import same_records_packed_and_read
 from wacommplusplus_b200 import synthetic as syn
 from wacommplusplus_b200.engine import Engine
 from wacommplusplus_b200.types import default_config
@@ -53,3 +54,11 @@ def test_host_buffer_intervals_walk_the_sorted_slabs_orders_alone(cuda_device, n
         for t in range(3):
             engine.move_interval_host(t, p)
     assert p.tobytes() == resident.tobytes()
+
+
+# 96 MiB of node records and tables: packed from 1,048,576 records on
+@pytest.mark.parametrize("n", [1048575, 1048576])
+def test_the_drop_in_at_the_edge_of_its_packing_rule(cuda_device, n):
+    win = syn.config1_window(n_frames=3, eta=512, xi=512, s_rho=4)
+    win.times[:] = win.times[0] + 120.0 * np.arange(3)
+    same_records_packed_and_read(win, n, False, 1)

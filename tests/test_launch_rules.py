@@ -52,3 +52,14 @@ def test_normals_are_drawn_ahead_under_the_automatic_shape_alone(tmp_path):
         printf("%u\\n", draw_steps(o, c, 3600.0, 1000));
     }""")
     assert [r[0] for r in rows] == [121, 0, 0, 0, 0]
+
+
+# the scratch the drop-in launcher asks for: 80 MiB, beyond 96 bytes per record, never above 1 GiB
+def test_the_packed_pair_of_the_drop_in_is_bounded(tmp_path):
+    mib, gib = 1 << 20, 1 << 30
+    want = {(80 * mib, 1): 1, (80 * mib + 1, 1): 0, (96 * 1000000, 1000000): 1,
+            (96 * 1000000, 999999): 0, (gib, 1 << 24): 1, (gib + 1, (1 << 31) - 1): 0,
+            (2 * 10 ** 10, 10 ** 7): 0}
+    rows = evaluate(tmp_path, "".join(f'printf("%d\\n", (int)packs_pair({b}ull, {n}ull));\n'
+                                      for b, n in want))
+    assert [r[0] for r in rows] == list(want.values())

@@ -157,15 +157,10 @@ cudaError_t launch_dropin(const wacomm_b200_config *config, wacomm_b200_particle
     return cudaGetLastError();
 }
 
-// The pair is packed up to this many nodes, and beyond while there are at most so many per record:
-// packing a node costs about 0.02 ns, reading the window and evaluating haversines instead above 10 ns
-// per record and, in the latency of its substep chain, at least 0.4 ms per call (2,000 records on
-// 180,224 nodes: 1.1 ms). It bounds the scratch to 64 MB or 2 KB per record.
-constexpr size_t PACK_NODES = (size_t)1 << 20, PACK_NODES_PER_RECORD = 32;
-
 // The call's packed pair in `scratch` (null: no scratch, read the window), stream-ordered. The window is
-// read, too, where a node record does not hold what the move reads: with other rho levels than one per
-// layer, or without a field (the diffusivity of a run without random walk).
+// read where the scratch would be too large for the records (packs_pair) or a node record does not hold
+// what the move reads: with other rho levels than one per layer, or without a field (the diffusivity of
+// a run without random walk).
 cudaError_t pack_window(const wacomm_b200_config *config, int timeIndex, int oceanTime,
                         const RawView &V, int count, PackedView &out, void **scratch,
                         cudaStream_t stream) {
@@ -173,11 +168,11 @@ cudaError_t pack_window(const wacomm_b200_config *config, int timeIndex, int oce
     const bool env = V.hasWindU || V.hasWindV || V.hasStokes;
     *scratch = nullptr;
     if (V.g.eta < 2 || V.g.xi < 2 || V.g.sW != V.g.sRho + 1 || !V.zeta || !V.u || !V.v || !V.w ||
-        !V.aktField || !V.hField || !V.lonRad || !V.latRad ||
-        (nodes > PACK_NODES && nodes > PACK_NODES_PER_RECORD * (size_t)count))
+        !V.aktField || !V.hField || !V.lonRad || !V.latRad)
         return cudaSuccess;
     const size_t bytes = nodes * sizeof(NodeRecord) +
                          plane * (sizeof(SurfRecord) + sizeof(CellMetric) + (env ? sizeof(EnvPair) : 0));
+    if (!packs_pair(bytes, (size_t)count)) return cudaSuccess;
     if (cudaMallocAsync(scratch, bytes, stream) != cudaSuccess) {
         *scratch = nullptr;
         (void)cudaGetLastError();  // no pool memory: read the window

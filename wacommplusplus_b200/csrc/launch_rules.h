@@ -62,4 +62,22 @@ inline unsigned draw_steps(const wacomm_b200_options &opt, const wacomm_b200_con
     return (unsigned)steps;
 }
 
+// Whether the drop-in launcher packs the forcing pair of `count` records into `bytes` of scratch from
+// the caller's memory pool. Packing saves 10 ns and more per record and hour of 120 substeps (at least
+// 0.4 ms per call) and costs 4 us per MB, and 9 us more per MB in a program that synchronizes after the
+// call, when the pool gives its memory back and maps it anew. Up to 80 MiB it is worth it for any
+// count: 1,000 records on 990,000 nodes 1.00 -> 0.84 ms per queued call, 1.45 -> 1.77 ms per
+// synchronized one; on 840,000 nodes 0.99 -> 0.59 and 1.43 -> 1.31 ms (intervals of a few substeps pay the
+// pack without the gain: four on 990,000 nodes 0.2 -> 0.4 and 0.6 -> 1.3 ms). Beyond, from a node record and
+// its tables per record on, where synchronized calls of four substeps lose little, too (records, nodes,
+// synchronized / queued read from the window -> packed): 4 M on 5.5 M 82 / 83 -> 48 / 44 ms, four substeps
+// 4.4 / 3.6 -> 8.3 / 3.6; 200,000 on 1.94 M 5.0 / 4.6 -> 6.0 / 3.8 ms, four substeps 0.7 / 0.3 -> 2.4 /
+// 0.7; 500,000 on 12.3 M 11.7 / 11.1 -> 18.5 / 10.8 ms, four substeps 1.0 / 0.6 -> 11 / 3.3. At most 1 GiB
+// is asked for.
+constexpr size_t PACK_BYTES = (size_t)80 << 20, PACK_BYTES_PER_RECORD = 96, PACK_BYTES_MOST = (size_t)1 << 30;
+
+inline bool packs_pair(size_t bytes, size_t count) {
+    return bytes <= PACK_BYTES || (bytes <= PACK_BYTES_MOST && bytes / PACK_BYTES_PER_RECORD <= count);
+}
+
 }  // namespace wb
