@@ -62,3 +62,20 @@ def test_the_drop_in_at_the_edge_of_its_packing_rule(cuda_device, n):
     win = syn.config1_window(n_frames=3, eta=512, xi=512, s_rho=4)
     win.times[:] = win.times[0] + 120.0 * np.arange(3)
     same_records_packed_and_read(win, n, False, 1)
+
+
+# 27,915 records of 601 substeps fit the draws' buffer and 27,916 do not; 40,000 are drawn ahead and
+# 40,001 are not. An engine's first interval draws in the step whatever the size.
+@pytest.mark.parametrize("n,dti,ahead", [(1, 30.0, 1), (27915, 6.0, 1), (27916, 6.0, 0),
+                                         (40000, 60.0, 1), (40001, 60.0, 0)])
+def test_normals_are_drawn_ahead_from_the_second_interval_on(cuda_device, n, dti, ahead):
+    got, launches = [], []
+    for shape in (-1, 2):
+        with walking_engine(n, 2, sort_by_cell=0, launch_shape=shape) as engine:
+            engine.set_config(default_config(random=True, dti=dti))
+            for t in range(2):
+                engine.move_interval(t)
+                launches.append(engine.stats()["launches"])
+            got.append(engine.get_particles())
+    assert got[0].tobytes() == got[1].tobytes()
+    assert launches == [launches[0], launches[0] + ahead, launches[0], launches[0]]
