@@ -3,6 +3,7 @@ import numpy as np
 import pytest
 
 from test_gpu_dropin import same_records_packed_and_read
+from test_gpu_work_order import mixed_records
 from wacommplusplus_b200 import synthetic as syn
 from wacommplusplus_b200.engine import Engine
 from wacommplusplus_b200.types import default_config
@@ -65,14 +66,23 @@ def test_the_drop_in_at_the_edge_of_its_packing_rule(cuda_device, n):
 
 
 # 27,915 records of 601 substeps fit the draws' buffer and 27,916 do not; 40,000 are drawn ahead and
-# 40,001 are not. An engine's first interval draws in the step whatever the size.
+# 40,001 are not; 0.1 and 7.3 do not sum to whole substeps. An engine's first interval draws in the step
+# whatever the size.
 @pytest.mark.parametrize("n,dti,ahead", [(1, 30.0, 1), (27915, 6.0, 1), (27916, 6.0, 0),
-                                         (40000, 60.0, 1), (40001, 60.0, 0)])
-def test_normals_are_drawn_ahead_from_the_second_interval_on(cuda_device, n, dti, ahead):
+                                         (40000, 60.0, 1), (40001, 60.0, 0), (777, 0.1, 1),
+                                         (3001, 7.3, 1)])
+@pytest.mark.parametrize("chunk", [0, 7])
+def test_normals_are_drawn_ahead_from_the_second_interval_on(cuda_device, n, dti, ahead, chunk):
+    win = syn.config1_window(n_frames=3, eta=16, xi=17, s_rho=6)
+    if dti < 1:
+        win.times[:] = win.times[0] + 60.0 * np.arange(3)
+    p = mixed_records(n, win, 9)
     got, launches = [], []
     for shape in (-1, 2):
-        with walking_engine(n, 2, sort_by_cell=0, launch_shape=shape) as engine:
+        with Engine(0, sort_by_cell=0, launch_shape=shape, substeps_per_launch=chunk) as engine:
+            engine.load_window(win)
             engine.set_config(default_config(random=True, dti=dti))
+            engine.set_particles(p)
             for t in range(2):
                 engine.move_interval(t)
                 launches.append(engine.stats()["launches"])
