@@ -91,7 +91,11 @@ __device__ __forceinline__ const PackedView &at_interval(const PackedView &V, co
 // kernel, each thread derives the interval from the device copies of config and times
 // (kernel.cu:158-171); the particle is read from and written back to the caller's AoS array.
 // 524,287 records on 128 x 128 x 10, 120 substeps: 13.7 ms with the window read and two haversines
-// per substep (244 registers), 3.9 ms with the packed pair (3.4 times faster per call); bound as move_soa_kernel is.
+// per substep (244 registers), 3.9 ms with the packed pair (3.4 times faster per call). Bound by L1 (87 %
+// of its throughput: two stencil reads per substep, and spills, because the config is on the device and
+// the drift form is in the same kernel). Whole calls at 244 registers without spills / now: with leeway
+// drift 524,287 records 21.7 / 9.7 ms packed; read from a window of 12.3 M nodes 50,000 records 3.3 / 2.0
+// ms, 500,000 15.3 / 11.0 ms, with leeway drift 25.4 / 20.2 ms.
 template <bool KEEP, class View>
 __global__ void __launch_bounds__(128, KEEP ? 1 : 4) dropin_move_kernel(
     const wacomm_b200_config *__restrict__ config, wacomm_b200_particle *particles,

@@ -210,9 +210,9 @@ __global__ void offsets_kernel(const unsigned long long *counts, int n, unsigned
 constexpr int EMIT_HELD = 256;
 
 // One thread per release, bound by issue in the ranks: 2 M releases of 64 sources 2.2 ms with each
-// rank by bisection from global memory, 1.05 ms from the rates and shared memory. Its merged rank is its index within its source plus the releases of
-// earlier sources at or before its time and of later sources strictly before it: the position
-// std::stable_sort by time gives it in the source-major list.
+// rank by bisection from global memory, 1.05 ms from the rates and shared memory. Its merged rank is
+// its index within its source plus the releases of earlier sources at or before its time and of later
+// sources strictly before it: the position std::stable_sort by time gives it in the source-major list.
 __global__ void emit_kernel(const wacomm_b200_source *sources, const Schedule *schedules,
                             int nSources, const unsigned long long *offsets,
                             unsigned long long total, const wacomm_b200_config *cfgp,

@@ -103,7 +103,9 @@ __device__ __forceinline__ void warp_sum_steps(unsigned long long *counter, int 
 // KEEP / not: 16,384 records 0.366 / 0.449 ms, 65,536 0.751 / 0.802 ms, 131,072 1.37 / 1.36 ms,
 // 500,009 4.73 / 3.71 ms (with the random walk 0.609 / 0.687, 1.28 / 1.15, 2.44 / 1.96, 8.14 / 6.30);
 // 242 registers and float operands before: 500,009 with the random walk 10.2 ms, XU pipe 54 -> 22 %,
-// FP64 24 -> 44 %, issue 36 -> 57 %.
+// FP64 24 -> 44 %, issue 36 -> 57 %. The drift form spills 622 bytes at 128 registers and takes what it
+// took at 242 without spills (whole interval, before / now: 50,000 records 2.21 / 2.15 ms, 131,072 4.18 /
+// 4.12 ms, 500,009 13.4 / 13.3 ms, with the random walk 15.3 / 15.2 ms).
 template <int SEM, bool DRIFT, bool KEEP>
 __global__ void __launch_bounds__(256, KEEP ? 1 : 2) move_soa_kernel(const wacomm_b200_config cfg,
                                                           const IntervalParams P,

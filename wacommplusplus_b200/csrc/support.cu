@@ -119,7 +119,8 @@ constexpr int PACK_ROW = 36, PACK_LEVEL = 2 * PACK_ROW, PACK_FIELD = PACK_LEVELS
 // rows come through shared memory in the fields' own order, the records leave in theirs (each eight
 // quads per level, the levels of a cell consecutive), so that both sides of the transposition move
 // whole lines. Cells on the last row or column (never valid) are zero. Bound by the record writes:
-// 491,520 cells of 25 levels 0.73 ms with one thread per (level, cell) and 128 bytes each, 0.48 ms so (4.0 TB/s).
+// 491,520 cells of 25 levels 0.73 ms with one thread per (level, cell) and 128 bytes each, 0.48 ms so
+// (4.0 TB/s).
 template <int STORE>
 __global__ void __launch_bounds__(256) pack_cells_kernel(int eta, int xi, int sW, FrameDevice f0,
                                                          FrameDevice f1, CellQuad<STORE> *cells) {
