@@ -89,3 +89,31 @@ def test_normals_are_drawn_ahead_from_the_second_interval_on(cuda_device, n, dti
             got.append(engine.get_particles())
     assert got[0].tobytes() == got[1].tobytes()
     assert launches == [launches[0], launches[0] + ahead, launches[0], launches[0]]
+
+
+# 65 x 64 x 10: the stencil is kept up to 41,600 records
+@pytest.mark.parametrize("drift", [0, 1])
+def test_reference_arithmetic_at_the_edge_of_the_kept_stencil(cuda_device, drift):
+    win = syn.RealisticForcing(eta=65, xi=64, s_rho=10, n_frames=2, seed=4, dlon=0.002, dlat=0.002,
+                               land_fraction=0.1, water_border=2).window()
+    win.windU10, win.windV10 = syn.vector_series((65, 64), 2, 8.0, 3, 8.0)
+    p = mixed_records(41601, win, 12)
+    p["driftObjectType"], p["driftSide"] = np.arange(len(p)) % 23, 1
+    got = []
+    for n in (41600, 41601):
+        with Engine(0, arithmetic="reference") as engine:
+            engine.load_window(win)
+            engine.set_config(default_config(random=True, driftModel=drift, hasWind=bool(drift)))
+            engine.set_particles(p[:n])
+            engine.move_interval(0)
+            got.append(engine.get_particles()[:41600])
+    assert got[0].tobytes() == got[1].tobytes()
+
+
+# 65 x 64 x 10: the drop-in keeps the stencil up to 41,600 records too
+@pytest.mark.parametrize("n", [41600, 41601])
+@pytest.mark.parametrize("environment", [False, True])
+def test_the_drop_in_at_the_edge_of_the_kept_stencil(cuda_device, n, environment):
+    win = syn.RealisticForcing(eta=65, xi=64, s_rho=10, n_frames=3, seed=8, land_fraction=0.1,
+                               water_border=1).window()
+    same_records_packed_and_read(win, n, environment, 1)

@@ -63,3 +63,13 @@ def test_the_packed_pair_of_the_drop_in_is_bounded(tmp_path):
     rows = evaluate(tmp_path, "".join(f'printf("%d\\n", (int)packs_pair({b}ull, {n}ull));\n'
                                       for b, n in want))
     assert [r[0] for r in rows] == list(want.values())
+
+
+# two warps per scheduler, and beyond a record per cell and level
+@pytest.mark.parametrize("grid,limit", [((16, 17, 6), 37888), ((128, 128, 10), 163840),
+                                        ((1 << 15, 1 << 15, 4), (1 << 31) - 1)])
+def test_the_stencil_is_kept_by_thinly_spread_records(tmp_path, grid, limit):
+    rows = evaluate(tmp_path, "".join(
+        f'printf("%d\\n", (int)keeps_stencil({n}, {grid[0]}, {grid[1]}, {grid[2]}));\n'
+        for n in (1, limit, min(limit + 1, (1 << 31) - 1))))
+    assert [r[0] for r in rows] == [1, 1, int(limit == (1 << 31) - 1)]

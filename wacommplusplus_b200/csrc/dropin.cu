@@ -93,9 +93,10 @@ __device__ __forceinline__ const PackedView &at_interval(const PackedView &V, co
 // 524,287 records on 128 x 128 x 10, 120 substeps: 13.7 ms with the window read and two haversines
 // per substep (244 registers), 3.9 ms with the packed pair (3.4 times faster per call). Bound by L1 (87 %
 // of its throughput: two stencil reads per substep, and spills, because the config is on the device and
-// the drift form is in the same kernel). Whole calls at 244 registers without spills / now: with leeway
-// drift 524,287 records 21.7 / 9.7 ms packed; read from a window of 12.3 M nodes 50,000 records 3.3 / 2.0
-// ms, 500,000 15.3 / 11.0 ms, with leeway drift 25.4 / 20.2 ms.
+// the drift form is in the same kernel); up to a record per cell and level the packed form keeps its
+// stencil (keeps_stencil: 100,000 records on 200 x 200 x 20 1.95 -> 1.22 ms). Whole calls at 244 registers
+// without spills / now: with leeway drift 500,000 records 20.2 / 8.9 ms packed; read from a window of 12.3 M
+// nodes 50,000 records 3.1 / 1.9 ms, 500,000 15.3 / 10.9 ms, with leeway drift 24.1 / 19.2 ms.
 template <bool KEEP, class View>
 __global__ void __launch_bounds__(128, KEEP ? 1 : 4) dropin_move_kernel(
     const wacomm_b200_config *__restrict__ config, wacomm_b200_particle *particles,
@@ -146,13 +147,13 @@ __global__ void __launch_bounds__(128, KEEP ? 1 : 4) dropin_move_kernel(
 template <class View>
 cudaError_t launch_dropin(const wacomm_b200_config *config, wacomm_b200_particle *particles,
                           const uint32_t *order, int timeIndex, int oceanTime, const double *times,
-                          const View &V, int count, cudaStream_t stream) {
+                          const View &V, bool keep, int count, cudaStream_t stream) {
     MoveLaunch L{};
     L.count = count;
     int threads;
     spread_launch(count, 128, L.lanes, threads);
     const int items = threads / 32 * L.lanes, blocks = launch_blocks(count, items);
-    if (count <= KEEP_RECORDS)
+    if (keep)
         dropin_move_kernel<true><<<blocks, threads, 0, stream>>>(config, particles, order, timeIndex,
                                                                  oceanTime, times, V, L);
     else
@@ -261,11 +262,13 @@ int dropin_move(const wacomm_b200_config *config, wacomm_b200_particle *particle
     PackedView packed;
     void *pair = nullptr;
     cudaError_t e = pack_window(config, timeIndex, oceanTime, V, count, packed, &pair, stream);
+    // Read from the window, 16 warps per SM hide the haversines of thinly spread records, too: 500,000
+    // on 12.3 M nodes 10.9 ms, 13.2 ms with the stencil kept at 8 (100,000: 3.7 and 3.2, 50,000: 1.9 and 2.1).
     if (e == cudaSuccess)
-        e = pair ? launch_dropin(config, particles, order, timeIndex, oceanTime, times, packed, count,
-                                 stream)
-                 : launch_dropin(config, particles, order, timeIndex, oceanTime, times, V, count,
-                                 stream);
+        e = pair ? launch_dropin(config, particles, order, timeIndex, oceanTime, times, packed,
+                                 keeps_stencil(count, eta, xi, sRho), count, stream)
+                 : launch_dropin(config, particles, order, timeIndex, oceanTime, times, V,
+                                 count <= KEEP_RECORDS, count, stream);
     for (void *held : {pair, (void *)scratch})
         if (held) {
             cudaError_t f = cudaFreeAsync(held, stream);

@@ -11,7 +11,7 @@ namespace wb {
 constexpr int B200_SMS = 148;
 
 // Two full warps per scheduler: up to here the plain step's records are not sorted, and the reference
-// arithmetic keeps its velocity stencil in registers.
+// arithmetic keeps its velocity stencil in registers (keeps_stencil).
 constexpr int KEEP_RECORDS = 2 * 4 * B200_SMS * 32;
 // All resident at once at launch shape 1 of the FP32 step (12 warps per SM).
 constexpr int RESIDENT_RECORDS = 12 * B200_SMS * 32;
@@ -28,6 +28,16 @@ inline void spread_launch(int count, int maxThreads, int &lanes, int &threads) {
     lanes = (int)(per < 1 ? 1 : per > 32 ? 32 : per);
     const long long warps = ((long long)count + lanes - 1) / lanes, even = 32 * ((warps + SMS - 1) / SMS);
     threads = even < maxThreads ? (int)even : maxThreads;
+}
+
+// Whether the reference arithmetic keeps the velocity stencil of `count` records in registers (8 warps per
+// SM) instead of reading it twice per substep (16 warps per SM): where one or two warps per scheduler hold
+// all records, and up to a record per cell and level. With fewer, the lanes of a warp share no lines, and
+// the stencils of 512 threads (384 bytes of lines each) do not fit L1. Whole interval read / kept, 200 x
+// 200 x 20: 100,000 records 1.98 / 1.24 ms, 500,000 5.55 / 5.09, 1.5 M 12.5 / 14.3; 300 x 300 x 20: 100,000
+// 2.37 / 1.35, 1.5 M 15.6 / 14.5; 128 x 128 x 10: 100,000 1.30 / 1.17, 200,000 2.06 / 2.21 ms.
+inline bool keeps_stencil(int count, int eta, int xi, int sRho) {
+    return count <= KEEP_RECORDS || count <= (long long)eta * xi * sRho;
 }
 
 // Blocks of `items` work items each that cover `count` (1 to 2^31 - 1).

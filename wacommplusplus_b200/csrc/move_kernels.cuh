@@ -98,14 +98,14 @@ __device__ __forceinline__ void warp_sum_steps(unsigned long long *counter, int 
 }
 
 // Reference arithmetic. The latency of FP64 chains and the conversions to float and back bound it;
-// 128 registers allow 16 warps per SM. Where one or two warps per scheduler hold all records (KEEP)
-// the registers go to the velocity stencil instead, out of the substep's chain of loads. Move kernel,
-// KEEP / not: 16,384 records 0.366 / 0.449 ms, 65,536 0.751 / 0.802 ms, 131,072 1.37 / 1.36 ms,
+// 128 registers allow 16 warps per SM. Where one or two warps per scheduler hold all records, or they are
+// spread thinly over the grid (keeps_stencil), the registers go to the velocity stencil instead (KEEP), out
+// of the substep's chain of loads. Move kernel on 128 x 128 x 10, KEEP / not: 16,384 records 0.366 / 0.449 ms, 65,536 0.751 / 0.802 ms, 131,072 1.37 / 1.36 ms,
 // 500,009 4.73 / 3.71 ms (with the random walk 0.609 / 0.687, 1.28 / 1.15, 2.44 / 1.96, 8.14 / 6.30);
 // 242 registers and float operands before: 500,009 with the random walk 10.2 ms, XU pipe 54 -> 22 %,
-// FP64 24 -> 44 %, issue 36 -> 57 %. The drift form spills 622 bytes at 128 registers and takes what it
-// took at 242 without spills (whole interval, before / now: 50,000 records 2.21 / 2.15 ms, 131,072 4.18 /
-// 4.12 ms, 500,009 13.4 / 13.3 ms, with the random walk 15.3 / 15.2 ms).
+// FP64 24 -> 44 %, issue 36 -> 57 %. The drift form spills 622 bytes at 128 registers, which cost it what the
+// warps brought in (whole interval, at 242 without spills / now): 500,009 records 13.3 / 12.8 ms, with the
+// random walk 15.2 / 14.6 ms; 100,000, with the stencil kept, 3.35 / 2.78 ms (4.0 at 128 registers).
 template <int SEM, bool DRIFT, bool KEEP>
 __global__ void __launch_bounds__(256, KEEP ? 1 : 2) move_soa_kernel(const wacomm_b200_config cfg,
                                                           const IntervalParams P,
@@ -235,7 +235,7 @@ cudaError_t launch_move_soa(const wacomm_b200_config &cfg, const IntervalParams 
     spread_launch(L.count, blockSize, M.lanes, threads);
     const int items = threads / 32 * M.lanes;
     const int blocks = launch_blocks(L.count, items);
-    const bool keep = L.count <= KEEP_RECORDS;
+    const bool keep = keeps_stencil(L.count, V.g.eta, V.g.xi, V.g.sRho);
     if (cfg.driftModel == 1) {
         if (keep) move_soa_kernel<SEM, true, true><<<blocks, threads, 0, stream>>>(cfg, P, V, S, M);
         else move_soa_kernel<SEM, true, false><<<blocks, threads, 0, stream>>>(cfg, P, V, S, M);
