@@ -33,28 +33,31 @@ __global__ void dropin_key_kernel(const wacomm_b200_particle *particles, int n, 
 
 // The call's forcing pair and cell metric in the engine's layout. Like the move, each thread reads
 // the tracking direction from the device copy of the config; one thread per (level, node).
-__global__ void dropin_pack_kernel(const wacomm_b200_config *__restrict__ config, int timeIndex,
-                                   int oceanTime, RawView V, NodeRecord *nodes, SurfRecord *surf,
-                                   CellMetric *metric, EnvPair *env) {
+__global__ void __launch_bounds__(256) dropin_pack_kernel(
+    const wacomm_b200_config *__restrict__ config, int timeIndex, int oceanTime, RawView V,
+    NodeRecord *nodes, SurfRecord *surf, CellMetric *metric, EnvPair *env) {
+    __shared__ NodeStage stage;
     const int next = timeIndex + config->trackingDirection;
     V.t0 = timeIndex;
     V.t1 = next >= 0 && next < oceanTime ? next : timeIndex;
     const int eta = V.g.eta, xi = V.g.xi;
     const size_t plane = (size_t)eta * xi, total = plane * V.g.sW;
-    for (size_t n = blockIdx.x * (size_t)blockDim.x + threadIdx.x; n < total;
-         n += (size_t)gridDim.x * blockDim.x) {
+    for (size_t base = blockIdx.x * (size_t)256; base < total; base += gridDim.x * (size_t)256) {
+        const size_t n = base + threadIdx.x;
         const int L = (int)(n / plane);
         const size_t c = n - (size_t)L * plane;
         const int j = (int)(c / xi), i = (int)(c - (size_t)j * xi);
         NodeRecord r;
-        r.w = V.pair(V.w, L, V.g.sW, j, i);
-        r.akt = V.pair(V.aktField, L, V.g.sW, j, i);
-        r.u = r.v = make_double2(0.0, 0.0);
-        if (L > 0) {
-            r.u = V.pair(V.u, L - 1, V.g.sRho, j, i);
-            r.v = V.pair(V.v, L - 1, V.g.sRho, j, i);
+        r.w = r.akt = r.u = r.v = make_double2(0.0, 0.0);
+        if (n < total) {
+            r.w = V.pair(V.w, L, V.g.sW, j, i);
+            r.akt = V.pair(V.aktField, L, V.g.sW, j, i);
+            if (L > 0) {
+                r.u = V.pair(V.u, L - 1, V.g.sRho, j, i);
+                r.v = V.pair(V.v, L - 1, V.g.sRho, j, i);
+            }
         }
-        nodes[n] = r;
+        store_nodes(stage, r, base, total, nodes);
         if (L == 0) {
             const SurfPair<float> s = V.surface(j, i);
             surf[c] = SurfRecord{s.h, s.z0, s.z1, 0.0};

@@ -17,20 +17,23 @@ size_t surf_record_bytes() { return sizeof(SurfRecord); }
 // ------------------------------------------------------------------ forcing pair packing
 
 // Interleaves records t0 and t1 into the node records of the reference arithmetic.
-__global__ void pack_nodes_kernel(int eta, int xi, int sW, FrameDevice f0, FrameDevice f1,
-                                  NodeRecord *nodes) {
-    size_t plane = (size_t)eta * xi, total = plane * sW;
-    for (size_t n = blockIdx.x * (size_t)blockDim.x + threadIdx.x; n < total;
-         n += (size_t)gridDim.x * blockDim.x) {
+__global__ void __launch_bounds__(256) pack_nodes_kernel(int eta, int xi, int sW, FrameDevice f0,
+                                                         FrameDevice f1, NodeRecord *nodes) {
+    __shared__ NodeStage stage;
+    const size_t plane = (size_t)eta * xi, total = plane * sW;
+    for (size_t base = blockIdx.x * (size_t)256; base < total; base += gridDim.x * (size_t)256) {
+        const size_t n = base + threadIdx.x;
         NodeRecord r;
-        r.w = make_double2(f0.w[n], f1.w[n]);
-        r.akt = make_double2(f0.akt[n], f1.akt[n]);
-        r.u = r.v = make_double2(0.0, 0.0);
-        if (n >= plane) {  // W level 0 has no rho level below it
-            r.u = make_double2(f0.u[n - plane], f1.u[n - plane]);
-            r.v = make_double2(f0.v[n - plane], f1.v[n - plane]);
+        r.w = r.akt = r.u = r.v = make_double2(0.0, 0.0);
+        if (n < total) {
+            r.w = make_double2(f0.w[n], f1.w[n]);
+            r.akt = make_double2(f0.akt[n], f1.akt[n]);
+            if (n >= plane) {  // W level 0 has no rho level below it
+                r.u = make_double2(f0.u[n - plane], f1.u[n - plane]);
+                r.v = make_double2(f0.v[n - plane], f1.v[n - plane]);
+            }
         }
-        nodes[n] = r;
+        store_nodes(stage, r, base, total, nodes);
     }
 }
 
