@@ -117,3 +117,33 @@ def test_the_drop_in_at_the_edge_of_the_kept_stencil(cuda_device, n, environment
     win = syn.RealisticForcing(eta=65, xi=64, s_rho=10, n_frames=3, seed=8, land_fraction=0.1,
                                water_border=1).window()
     same_records_packed_and_read(win, n, environment, 1)
+
+
+# intervals of three and four substeps, and launches of one
+@pytest.mark.parametrize("seconds,chunk", [(90.0, 0), (120.0, 0), (120.0, 1)])
+def test_records_of_short_launches_do_not_depend_on_the_sort(cuda_device, seconds, chunk):
+    win = syn.config1_window(n_frames=3, eta=16, xi=17, s_rho=6)
+    win.times[:] = win.times[0] + seconds * np.arange(3)
+    p = mixed_records(40000, win, 4)
+    p["time"] = win.times[0] + np.random.default_rng(4).choice([0.0, 31.0, 100.0, 150.0, 500.0], 40000)
+    got = []
+    for sort in (0, 1):
+        with Engine(0, sort_by_cell=sort, substeps_per_launch=chunk) as engine:
+            engine.load_window(win)
+            engine.set_config(default_config(random=True))
+            engine.set_particles(p)
+            for t in range(2):
+                engine.move_interval(t)
+            got.append(engine.get_particles())
+    assert got[0].tobytes() == got[1].tobytes()
+
+
+# 255, 256 and 260 nodes: the records of a block of 256 leave it together
+@pytest.mark.parametrize("eta,xi,s_rho", [(5, 17, 2), (8, 8, 3), (4, 13, 4)])
+def test_node_records_at_the_edges_of_a_block(cuda_device, eta, xi, s_rho):
+    win = syn.config1_window(n_frames=3, eta=eta, xi=xi, s_rho=s_rho)
+    rng = np.random.default_rng(1)
+    for name in ("u", "v", "w", "akt"):
+        field = getattr(win, name)
+        field[:] = rng.normal(0, 0.1, field.shape).astype(np.float32)
+    same_records_packed_and_read(win, 600, False, 1)

@@ -73,3 +73,15 @@ def test_the_stencil_is_kept_by_thinly_spread_records(tmp_path, grid, limit):
         f'printf("%d\\n", (int)keeps_stencil({n}, {grid[0]}, {grid[1]}, {grid[2]}));\n'
         for n in (1, limit, min(limit + 1, (1 << 31) - 1))))
     assert [r[0] for r in rows] == [1, 1, int(limit == (1 << 31) - 1)]
+
+
+# 16 x 17 x 6: 1,632 cells and levels; a bin more for the records that take no step
+@pytest.mark.parametrize("count,forward,substeps,levels,late", [
+    (1632, 0, 120, 1, 1), (1633, 0, 120, 6, 1), (1633, 1, 120, 6, 4), (400, 1, 120, 1, 4),
+    (40000, 1, 120, 6, 16), (40000, 1, 4, 6, 16), (40000, 1, 3, 1, 1), (40000, 0, 1, 1, 1)])
+def test_the_bins_of_the_sort(tmp_path, count, forward, substeps, levels, late):
+    rows = evaluate(tmp_path, f"""
+    const SortBins b = sort_bins(16, 17, 6, {count}, {forward}, {substeps});
+    const SortBins most = sort_bins(16, 17, 6, {count}, {forward}, INFINITY);
+    printf("%d %d %d\\n", b.levels, b.late, (int)(b.count() <= most.count()));""")
+    assert rows == [[levels, late, 1]]

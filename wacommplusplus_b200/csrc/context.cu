@@ -521,9 +521,10 @@ PackedArgs packed_args(wacomm_b200_context *ctx) {
     return A;
 }
 
-// Histogram, offsets and scan scratch of the cell sort of `count` records.
+// Histogram, offsets and scan scratch of the cell sort of `count` records (for intervals of any length).
 int reserve_sort(wacomm_b200_context *ctx, size_t count) {
-    size_t bins = sort_bins(ctx->eta, ctx->xi, ctx->sRho, count, ctx->cfg.trackingDirection > 0).count();
+    size_t bins = sort_bins(ctx->eta, ctx->xi, ctx->sRho, count, ctx->cfg.trackingDirection > 0,
+                            INFINITY).count();
     if (ctx->binsCap < bins + 2 || !ctx->dHist) {
         cudaFree(ctx->dHist);
         ctx->dHist = ctx->dOffsets = nullptr;
@@ -538,14 +539,15 @@ int reserve_sort(wacomm_b200_context *ctx, size_t count) {
     return reserve_scan(ctx, std::max(bins, count));
 }
 
-// Cell sort of `count` records for interval P: walks them in seqIn (a permutation of [0, count),
+// Cell sort of `count` records for `seconds` of interval P: walks them in seqIn (a permutation of [0, count),
 // or null: slot order) and copies the resulting order to seqOut (or not, if null). A sort of the
 // whole resident set walks the previous full sort's order (when that is still a permutation of
 // the slots); a sort of a slab walks its own previous one or its slots.
-int sort_work(wacomm_b200_context *ctx, const IntervalParams &P, const ParticleSoA &S, size_t count,
-              uint32_t *keys, uint32_t *order, const uint32_t *seqIn, uint32_t *seqOut,
+int sort_work(wacomm_b200_context *ctx, const IntervalParams &P, double seconds, const ParticleSoA &S,
+              size_t count, uint32_t *keys, uint32_t *order, const uint32_t *seqIn, uint32_t *seqOut,
               int &launches) {
-    SortBins bins = sort_bins(ctx->eta, ctx->xi, ctx->sRho, count, P.direction > 0);
+    SortBins bins = sort_bins(ctx->eta, ctx->xi, ctx->sRho, count, P.direction > 0,
+                              seconds / ctx->cfg.dti);
     if (P.direction > 0) {  // backward tracking releases all
         bins.start = P.start;
         bins.end = P.start + P.length;
@@ -623,8 +625,8 @@ int run_interval(wacomm_b200_context *ctx, const IntervalParams &base, size_t of
             L.order = seqIn;
             ctx->sortedAgo++;
         } else if (sorts_work(ctx, count)) {
-            int rc = sort_work(ctx, P, S, count, keys, order, c == 0 ? seqIn : seqOut, seqOut,
-                               launches);
+            int rc = sort_work(ctx, P, nChunks > 1 ? chunk : base.length, S, count, keys, order,
+                               c == 0 ? seqIn : seqOut, seqOut, launches);
             if (rc) return rc;
             L.order = order;
             if (c == 0) ctx->sortedAgo = 0;
@@ -813,8 +815,8 @@ int run_surrogate(wacomm_b200_context *ctx, const IntervalParams &P, int &launch
             st.walkOrder = seqIn;
         } else {
             ctx->seqBounds.clear();
-            if ((rc = sort_work(ctx, P, ctx->S.s, count, ctx->dKeys, ctx->dOrder, seqIn, ctx->dSeq,
-                                launches)))
+            if ((rc = sort_work(ctx, P, P.length, ctx->S.s, count, ctx->dKeys, ctx->dOrder, seqIn,
+                                ctx->dSeq, launches)))
                 return rc;
             ctx->seqBounds = whole;
             ctx->sortedAgo = 0;

@@ -236,7 +236,7 @@ int dropin_move(const wacomm_b200_config *config, wacomm_b200_particle *particle
     uint32_t *order = nullptr, *scratch = nullptr;
     if (eta >= 2 && xi >= 2) {
         // keys[count] | order[count] | histogram[bins] | offsets[bins + 1] | scan partials
-        const int levels = sort_bins(eta, xi, sRho, (size_t)count, false).levels;
+        const int levels = sort_bins(eta, xi, sRho, (size_t)count, false, INFINITY).levels;
         size_t bins = (size_t)eta * xi * levels + 1;
         size_t words = 2 * (size_t)count + 2 * bins + 1 + scan_temp_words(bins);
         if (cudaMallocAsync((void **)&scratch, words * sizeof(uint32_t), stream) == cudaSuccess) {

@@ -9,6 +9,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include "launch_rules.h"
 #include "wacomm_b200.h"
 
 namespace wb {
@@ -78,19 +79,6 @@ cudaError_t build_metric(int semantics, int eta, int xi, const double *lonRad,
 size_t scan_temp_words(size_t n);
 cudaError_t exclusive_scan(const uint32_t *in, uint32_t *out, size_t n, uint32_t *total,
                            uint32_t *temp, cudaStream_t stream);
-
-// Bins of the counting sort by forcing cell: one per cell or, with levels > 1, per vertical level
-// of a cell; each split by release time into `late` parts (the first: released by the interval's
-// start, the others: equal parts of the interval), then one last bin for the records that take no
-// step in the interval (off the grid, or released at or after its end).
-struct SortBins {
-    int eta, xi, levels, late;
-    double start, end;  // of a forward interval; infinite: no release test
-    size_t count() const { return (size_t)eta * xi * levels * late + 1; }
-};
-// The bins `count` records are sorted into on a grid of sRho levels; `forward`: records are released
-// in the interval's direction.
-SortBins sort_bins(int eta, int xi, int sRho, size_t count, bool forward);
 
 // Counting sort of particles by forcing cell: order[] receives particle slots grouped by bin.
 // The records are visited in the sequence seq[n] (a permutation of the slots; null: slot order).

@@ -30,6 +30,47 @@ inline void spread_launch(int count, int maxThreads, int &lanes, int &threads) {
     threads = even < maxThreads ? (int)even : maxThreads;
 }
 
+// Bins of the counting sort by forcing cell: one per cell or, with levels > 1, per vertical level
+// of a cell; each split by release time into `late` parts (the first: released by the interval's
+// start, the others: equal parts of the interval), then one last bin for the records that take no
+// step in the interval (off the grid, or released at or after its end).
+struct SortBins {
+    int eta, xi, levels, late;
+    double start, end;  // of a forward interval; infinite: no release test
+    size_t count() const { return (size_t)eta * xi * levels * late + 1; }
+};
+
+// The bins `count` records are sorted into on a grid of sRho levels for a launch of `substeps`;
+// `forward`: records are released in the interval's direction.
+//
+// Levels are told apart from one record per bin on: the forcing records of a cell's levels lie apart
+// in memory, so a warp of one cell on several levels reads several lines per load, and the FP32 step
+// over FP32 storage is bound by its L1 wavefronts (83 % of the L1 throughput with four levels mixed).
+// 16.8 M records on 128 x 128 x 10 with the upper four levels in use: 46.9 ms per host interval
+// against 53.6 ms by cell alone; 1.05 M with the random walk: 10.0 against 11.1 ms. With fewer
+// records than bins a warp meets as many lines either way and the larger scan costs: 2 M records on
+// 640 x 768 x 24, 11.8 M bins: 0.6 % slower with levels.
+//
+// Records released during the interval take fewer substeps the later they come; the lanes of a warp run
+// as long as its longest. Parts of the interval are told apart while the bins stay below four per
+// record (their scan is cheap): 2 M records released in the first of two hours on 640 x 768 x 24, 8
+// parts: 31.1 -> 27.4 ms; 400,000 drift records of 32 scenarios over six hours 11.6 -> 11.4 ms; no
+// change where all are released.
+//
+// A launch of one to three substeps does not bring in the larger scan: 4 M records on 128 x 128 x 10, one
+// substep 0.94 ms by cell and 1.03 split, four 1.28 and 1.24 ms.
+inline SortBins sort_bins(int eta, int xi, int sRho, size_t count, bool forward, double substeps) {
+    const size_t split = (size_t)eta * xi * sRho + 1;
+    SortBins B{eta, xi, 1, 1, -INFINITY, INFINITY};
+    if (substeps < 4) return B;
+    if (split <= count && split < ((size_t)1 << 31)) B.levels = sRho;
+    const size_t cells = (size_t)eta * xi * B.levels;
+    while (forward && B.late < 16 && cells * 2 * B.late <= 4 * count &&
+           cells * 2 * B.late < ((size_t)1 << 31))
+        B.late *= 2;
+    return B;
+}
+
 // Whether the reference arithmetic keeps the velocity stencil of `count` records in registers (8 warps per
 // SM) instead of reading it twice per substep (16 warps per SM): where one or two warps per scheduler hold
 // all records, and up to a record per cell and level. With fewer, the lanes of a warp share no lines, and

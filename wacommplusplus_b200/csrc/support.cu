@@ -419,30 +419,6 @@ __global__ void key_scatter_kernel(const uint32_t *keys, int n, const uint32_t *
     }
 }
 
-// Levels are told apart from one record per bin on: the forcing records of a cell's levels lie apart
-// in memory, so a warp of one cell on several levels reads several lines per load, and the FP32 step
-// over FP32 storage is bound by its L1 wavefronts (83 % of the L1 throughput with four levels mixed).
-// 16.8 M records on 128 x 128 x 10 with the upper four levels in use: 46.9 ms per host interval
-// against 53.6 ms by cell alone; 1.05 M with the random walk: 10.0 against 11.1 ms. With fewer
-// records than bins a warp meets as many lines either way and the larger scan costs: 2 M records on
-// 640 x 768 x 24, 11.8 M bins: 0.6 % slower with levels.
-//
-// Records released during the interval take fewer substeps the later they come; the lanes of a warp run
-// as long as its longest. Parts of the interval are told apart while the bins stay below four per
-// record (their scan is cheap): 2 M records released in the first of two hours on 640 x 768 x 24, 8
-// parts: 31.1 -> 27.4 ms; 400,000 drift records of 32 scenarios over six hours 11.6 -> 11.4 ms; no
-// change where all are released.
-SortBins sort_bins(int eta, int xi, int sRho, size_t count, bool forward) {
-    const size_t split = (size_t)eta * xi * sRho + 1;
-    SortBins B{eta, xi, 1, 1, -INFINITY, INFINITY};
-    if (split <= count && split < ((size_t)1 << 31)) B.levels = sRho;
-    const size_t cells = (size_t)eta * xi * B.levels;
-    while (forward && B.late < 16 && cells * 2 * B.late <= 4 * count &&
-           cells * 2 * B.late < ((size_t)1 << 31))
-        B.late *= 2;
-    return B;
-}
-
 cudaError_t sort_by_cell(const ParticleSoA &S, int n, const SortBins &bins, const uint32_t *seq,
                          uint32_t *keys, uint32_t *hist, uint32_t *offsets, uint32_t *temp,
                          uint32_t *order, cudaStream_t stream) {
