@@ -277,7 +277,9 @@ int wacomm_b200_graph_release(wacomm_b200_context *ctx);
  * shape and keeps the fastest in options.particles_per_thread. With the population sorted
  * (options.sort_by_cell) and four intervals from time_index inside the forcing window, it then
  * times those four intervals from the same snapshot sorting every 1, 2 or 4 of them and keeps the
- * fastest cadence in options.sort_by_cell. No reference counterpart. */
+ * fastest cadence in options.sort_by_cell. The choice holds for the population it was made with: a
+ * launch_shape it sets stays until it is set again, however the population grows. No reference
+ * counterpart. */
 int wacomm_b200_autotune(wacomm_b200_context *ctx, int time_index, int *best, float *best_ms);
 
 /* The same interval through host buffers: uploads n records from `particles` (pinned or
